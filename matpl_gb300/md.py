@@ -30,7 +30,7 @@ from typing import Dict, Optional, Sequence
 import numpy as np
 import torch
 
-from . import _lib, dp as _dp
+from . import _lib, dp as _dp, ops
 from ._lib import check, ptr
 from .params import DPConfig
 from .structures import Structure, maxwell_boltzmann
@@ -167,6 +167,7 @@ class ReplicaMD:
         with torch.cuda.graph(self.graph, stream=side):
             for _ in range(self.steps_per_graph):
                 self._step()
+        self._graph_keep = ops.stream_workspaces(side.cuda_stream)   # read by address
         for k, t in keep.items():
             getattr(self, k).copy_(t)
         for k, t in keep_out.items():

@@ -270,6 +270,11 @@ def _image_index(counts, dev):
     return t
 
 
+def cached_image_index(counts, dev):
+    """The cached image index of ``counts`` (None before its first use)."""
+    return _img_cache.get((counts, dev))
+
+
 class _NepForceVirial(torch.autograd.Function):
     """Forces [N, 3] and per-image virial [B, 9] of one list (``matpl_nep_force_virial``);
     linear in dE, its backward (``matpl_nep_force_virial_grad``) is the transpose map."""

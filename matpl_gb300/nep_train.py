@@ -228,14 +228,18 @@ class GraphedNepTrainer:
             loss = self.loss(static, tindex)
             loss.backward()
             self.opt.step()
-        return g, static, loss
+        # the graph reads the one-hot type index and the module caches' tensors (image index,
+        # row of ones) by address, so they live as long as the graph does
+        counts = tuple(int(c) for c in static["num_atom"].tolist())
+        keep = (tindex, nep_ops.cached_image_index(counts, tindex.device), splitk.cached_ones())
+        return g, static, loss, keep
 
     def step(self, batch) -> torch.Tensor:
         key = tuple(tuple(batch[k].shape) for k in self.KEYS) + \
             (tuple(batch["num_atom"].reshape(-1).tolist()),)
         if key not in self.graphs:
             self.graphs[key] = self._capture(batch)
-        g, static, loss = self.graphs[key]
+        g, static, loss, _ = self.graphs[key]
         for k in self.KEYS:
             if batch[k].data_ptr() != static[k].data_ptr():
                 static[k].copy_(batch[k], non_blocking=True)

@@ -200,6 +200,12 @@ def workspace(device: torch.device, nbytes: int, tag: str) -> torch.Tensor:
     return buf
 
 
+def stream_workspaces(stream: int):
+    """The scratch buffers held now for one stream, for a graph captured on it to keep alive
+    (streams come from a pool, so a later capture on the same one may replace them)."""
+    return tuple(buf for (_, st, _), buf in _ws_cache.items() if st == stream)
+
+
 @_lib.on_device
 def find_neighbore(type_maps: torch.Tensor, frac_position: torch.Tensor, lattice: torch.Tensor,
                    ntypes: int, m_neigh: int, Rc_M: float, Rc_type: Union[float, Sequence[float]],

@@ -54,6 +54,11 @@ def _ones_row(n, dev, dt):
     return t
 
 
+def cached_ones():
+    """The rows of ones held now, for a captured graph to keep alive."""
+    return tuple(_ones_rows.values())
+
+
 class _AddRow(torch.autograd.Function):
     """z [N, F] + b [F]; the gradient of b, a sum over the N rows, as ones[1, N] @ g through
     ``_MM`` (differentiable again)."""

@@ -640,14 +640,17 @@ class GraphedTrainer:
         with torch.cuda.graph(g, stream=side):   # the warm-up's workspaces are reused
             loss, le, lf = self.tr._loss_and_backward(static, self.w_f, self.w_e)
             self.opt.step()
-        return g, static, loss
+        # the graph reads the trainer's type-grouped rows and this stream's workspaces by
+        # address: a later batch shape replaces them, so they live as long as the graph does
+        keep = (self.tr._rows, ops.stream_workspaces(side.cuda_stream))
+        return g, static, loss, keep
 
     def step(self, batch):
         keys = self._keys(batch)
         key = tuple(tuple(batch[k].shape) for k in keys) + (tuple(batch["atom_type"]),)
         if key not in self.graphs:
             self.graphs[key] = self._capture(batch)
-        g, static, loss = self.graphs[key]
+        g, static, loss, _ = self.graphs[key]
         for k in keys:
             if batch[k].data_ptr() != static[k].data_ptr():
                 static[k].copy_(batch[k], non_blocking=True)

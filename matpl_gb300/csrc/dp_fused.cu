@@ -9,7 +9,7 @@
 //                n_empty * R_pad^T G(s_pad), evaluated once per type pair.
 //   dp_embed_fwd warp per centre atom, lane per occupied slot: environment row -> embedding
 //                MLP -> A[4][25] += R^T G (smem-staged, lanes own A entries) -> A / (m T).
-//   dp_fit       CTA per tile of atoms: D = A^T A[:, :16], fitting net forward (Ei) and its
+//   dp_fit       CTA per tile of 1 to 16 atoms: D = A^T A[:, :16], fitting net forward (Ei) and its
 //                adjoint down to dE/dA, with tanh outputs kept in shared memory.
 //   dp_embed_bwd warp per centre atom: recomputes the environment row and the embedding
 //                activations (never stored), back-propagates dE/dA to dE/dR_k, contracts with
@@ -228,9 +228,10 @@ dp_embed_fwd(const int32_t *__restrict__ list_neigh, const T *__restrict__ idr,
     const int nnet = P.ntypes * P.ntypes;
     T *wsm = reinterpret_cast<T *>(smem_raw);
     const int wcount = WS ? nnet * EmbOff::SIZE : 0;
-    T *Gs_all = wsm + wcount;                                  // [kWarps][32][E+1]
-    T *Rs_all = Gs_all + kWarps * 32 * (E + 1);                // [kWarps][32][4]
-    int *list_all = reinterpret_cast<int *>(Rs_all + kWarps * 32 * 4);
+    T *Gs_all = wsm + wcount;                                  // [nwarps][32][E+1]
+    const int nwarps = blockDim.x >> 5;                        // 1 or kWarps
+    T *Rs_all = Gs_all + nwarps * 32 * (E + 1);                // [nwarps][32][4]
+    int *list_all = reinterpret_cast<int *>(Rs_all + nwarps * 32 * 4);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     T *Gs = Gs_all + warp * 32 * (E + 1);
     T *Rs = Rs_all + warp * 32 * 4;
@@ -238,8 +239,8 @@ dp_embed_fwd(const int32_t *__restrict__ list_neigh, const T *__restrict__ idr,
     if (WS) stage_weights(params, wsm, wcount);
     const int S = P.nslots;
     const long long total = (long long)P.batch * P.natoms;
-    for (long long t = (long long)blockIdx.x * kWarps + warp; t < total;
-         t += (long long)gridDim.x * kWarps) {
+    for (long long t = (long long)blockIdx.x * nwarps + warp; t < total;
+         t += (long long)gridDim.x * nwarps) {
         const int i = (int)(t % P.natoms);
         const int ti = type_map[i];
         T *Arow = Aout + t * NA;
@@ -311,51 +312,101 @@ dp_embed_fwd(const int32_t *__restrict__ list_neigh, const T *__restrict__ idr,
 }
 
 // --------------------------------------------------------------------------- dp_fit
-// Row-tiled GEMM helper: out[r][col] (+)= sum_k X[r][k] * W[k][col] for this warp's rows.
-template <typename T, int RW, int NC>
-__device__ __forceinline__ void warp_gemm(const T *X, int ldx, int K, const T *__restrict__ W,
-                                          int ldw, int ncols, int lane, T acc[RW][NC]) {
-    for (int k = 0; k < K; ++k) {
-        T w[NC];
+// Two consecutive activations of one row (rows are even-strided and 16-byte aligned).
+__device__ __forceinline__ void lds2(const float *p, float v[2]) {
+    const float2 q = *reinterpret_cast<const float2 *>(p);
+    v[0] = q.x; v[1] = q.y;
+}
+__device__ __forceinline__ void lds2(const double *p, double v[2]) {
+    const double2 q = *reinterpret_cast<const double2 *>(p);
+    v[0] = q.x; v[1] = q.y;
+}
+
+// acc[r][q] = sum_k X[r][k] W[k][lane + 32 q] over R rows, K = 50 in order, and the 50 columns
+// from W (lane + 32 < 50 for the second half).
+template <typename T, int R>
+__device__ __forceinline__ void fit_gemm50(const T *X, const T *__restrict__ W, int ldw, int lane,
+                                           T acc[R][2]) {
+    const bool hi = lane + 32 < F;
+#pragma unroll 5
+    for (int k = 0; k < F; k += 2) {
+        const T *w = W + k * ldw + lane;
+        const T a0 = w[0], a1 = w[ldw];
+        const T b0 = hi ? w[32] : T(0), b1 = hi ? w[ldw + 32] : T(0);
 #pragma unroll
-        for (int q = 0; q < NC; ++q) {
-            const int col = lane + 32 * q;
-            w[q] = col < ncols ? W[(long long)k * ldw + col] : T(0);
-        }
-#pragma unroll
-        for (int r = 0; r < RW; ++r) {
-            const T xv = X[r * ldx + k];
-#pragma unroll
-            for (int q = 0; q < NC; ++q) acc[r][q] += xv * w[q];
+        for (int r = 0; r < R; ++r) {
+            T x[2];
+            lds2(X + r * F + k, x);
+            acc[r][0] += x[0] * a0;
+            acc[r][1] += x[0] * b0;
+            acc[r][0] += x[1] * a1;
+            acc[r][1] += x[1] * b1;
         }
     }
 }
 
-template <typename T, int TILE>
+// out(o, q, sum) for every output q = r * 50 + o of X [R][K] * W [K][50] (K even).  A thread
+// takes one column of RG rows, so a weight load serves RG FMAs and the whole CTA reads each
+// weight matrix R / RG times from L1; every sum runs over k in order.
+template <typename T, int R, typename OUT>
+__device__ __forceinline__ void fit_layer(const T *X, int ldx, int K, const T *__restrict__ W,
+                                          OUT out) {
+    constexpr int RG = R >= 4 ? R / 4 : 1;
+    const int g = threadIdx.x / F, o = threadIdx.x - g * F;
+    T acc[RG];
+#pragma unroll
+    for (int r = 0; r < RG; ++r) acc[r] = T(0);
+    if (g < R / RG) {
+        const T *x0 = X + g * RG * ldx;
+#pragma unroll 5
+        for (int k = 0; k < K; k += 2) {
+            const T w0 = W[k * F + o], w1 = W[(k + 1) * F + o];
+#pragma unroll
+            for (int r = 0; r < RG; ++r) {
+                T x[2];
+                lds2(x0 + r * ldx + k, x);
+                acc[r] += x[0] * w0;
+                acc[r] += x[1] * w1;
+            }
+        }
+    }
+    __syncthreads();                                     // X read by every thread
+    if (g < R / RG)
+#pragma unroll
+        for (int r = 0; r < RG; ++r) out(o, (g * RG + r) * F + o, acc[r]);
+    __syncthreads();
+}
+
+// One CTA of eight warps per tile of R atoms: the hidden layers give each thread a column of
+// RG rows, dE/dD (400 columns) gives each warp 50 columns of all rows.  Bound: shared loads and
+// the latency of the weight loads (80 KB per net, from L2).  A tile of 64 atoms whose eight warps
+// each read every weight ran 108 CTAs on 152 SMs at 6,913 atoms: 197 us; 16-atom tiles with a
+// weight load shared by four rows (eight in dE/dD's halves) take 74 us there.
+template <typename T, int R>
 __global__ void __launch_bounds__(256)
 dp_fit(const T *__restrict__ Ain, const int32_t *__restrict__ type_map,
        const T *__restrict__ params, T *__restrict__ Ei, T *__restrict__ dAout, EvalParams P) {
-    constexpr int RW = TILE / 8;                 // rows per warp
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    T *As = reinterpret_cast<T *>(smem_raw);     // [TILE][NA]
-    T *Ds = As + TILE * NA;                      // [TILE][DIN]  (D, later dE/dD)
-    T *T1 = Ds + TILE * DIN;                     // [TILE][F]
-    T *T2 = T1 + TILE * F;
-    T *T3 = T2 + TILE * F;
-    T *X = T3 + TILE * F;                        // [TILE][F] running activation / adjoint
-    __shared__ int rtype[TILE];
+    T *Ds = reinterpret_cast<T *>(smem_raw);     // [R][DIN] D, later dE/dD
+    T *As = Ds + R * DIN;                        // [R][NA]
+    T *T1 = As + R * NA;                         // [R][F] each
+    T *T2 = T1 + R * F;
+    T *T3 = T2 + R * F;
+    T *X = T3 + R * F;                           // running activation / adjoint
+    static_assert(8 * F == DIN, "eight warps of 50 columns cover dE/dD");
+    __shared__ int rtype[R];
     __shared__ int tflag[16];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long long total = (long long)P.batch * P.natoms;
-    const long long ntiles = (total + TILE - 1) / TILE;
+    const long long ntiles = (total + R - 1) / R;
     const long long woff = (long long)P.ntypes * P.ntypes * EmbOff::SIZE;
 
     for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const long long t0 = tile * TILE;
+        const long long t0 = tile * R;
         __syncthreads();
         for (int q = threadIdx.x; q < 16; q += blockDim.x) tflag[q] = 0;
         __syncthreads();
-        for (int r = threadIdx.x; r < TILE; r += blockDim.x) {
+        for (int r = threadIdx.x; r < R; r += blockDim.x) {
             const long long t = t0 + r;
             int ty = -1;
             if (t < total) {
@@ -365,7 +416,7 @@ dp_fit(const T *__restrict__ Ain, const int32_t *__restrict__ type_map,
             rtype[r] = ty;
             if (ty >= 0) tflag[ty] = 1;
         }
-        for (int q = threadIdx.x; q < TILE * NA; q += blockDim.x) {
+        for (int q = threadIdx.x; q < R * NA; q += blockDim.x) {
             const long long t = t0 + q / NA;
             As[q] = t < total ? Ain[t0 * NA + q] : T(0);
         }
@@ -374,7 +425,7 @@ dp_fit(const T *__restrict__ Ain, const int32_t *__restrict__ type_map,
             if (!tflag[tt]) continue;
             const T *fw = params + woff + (long long)tt * FitOff::SIZE;
             // D[r][p*M2+q] = sum_c A[r][c][p] A[r][c][q]
-            for (int q = threadIdx.x; q < TILE * DIN; q += blockDim.x) {
+            for (int q = threadIdx.x; q < R * DIN; q += blockDim.x) {
                 const int r = q / DIN, e = q - r * DIN;
                 const int p = e / M2, qq = e - p * M2;
                 const T *a = As + r * NA;
@@ -382,140 +433,68 @@ dp_fit(const T *__restrict__ Ain, const int32_t *__restrict__ type_map,
                         a[3 * E + p] * a[3 * E + qq];
             }
             __syncthreads();
-            const int r0 = warp * RW;
-            {   // layer 0: T1 = tanh(D W0 + b0), X = T1
-                T acc[RW][2];
-#pragma unroll
-                for (int r = 0; r < RW; ++r) { acc[r][0] = T(0); acc[r][1] = T(0); }
-                warp_gemm<T, RW, 2>(Ds + r0 * DIN, DIN, DIN, fw + FitOff::W0, F, F, lane, acc);
-#pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                    const int o = lane + 32 * q;
-                    if (o < F) {
-                        const T b = fw[FitOff::B0 + o];
-#pragma unroll
-                        for (int r = 0; r < RW; ++r) {
-                            const T tv = dev_tanh(acc[r][q] + b);
-                            T1[(r0 + r) * F + o] = tv;
-                            X[(r0 + r) * F + o] = tv;
-                        }
-                    }
-                }
-            }
-            __syncwarp();
+            // layer 0: T1 = tanh(D W0 + b0), X = T1
+            fit_layer<T, R>(Ds, DIN, DIN, fw + FitOff::W0, [&](int o, int q, T v) {
+                const T tv = dev_tanh(v + fw[FitOff::B0 + o]);
+                T1[q] = tv;
+                X[q] = tv;
+            });
             // layers 1, 2: X = tanh(X W + b) * dt + X
-#pragma unroll
-            for (int l = 1; l <= 2; ++l) {
-                const int OW = l == 1 ? FitOff::W1 : FitOff::W2;
-                const int OB = l == 1 ? FitOff::B1 : FitOff::B2;
-                const int OD = l == 1 ? FitOff::DT1 : FitOff::DT2;
-                T *Tl = l == 1 ? T2 : T3;
-                T acc[RW][2];
-#pragma unroll
-                for (int r = 0; r < RW; ++r) { acc[r][0] = T(0); acc[r][1] = T(0); }
-                warp_gemm<T, RW, 2>(X + r0 * F, F, F, fw + OW, F, F, lane, acc);
-                __syncwarp();
-#pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                    const int o = lane + 32 * q;
-                    if (o < F) {
-                        const T b = fw[OB + o], dt = fw[OD + o];
-#pragma unroll
-                        for (int r = 0; r < RW; ++r) {
-                            const T tv = dev_tanh(acc[r][q] + b);
-                            Tl[(r0 + r) * F + o] = tv;
-                            X[(r0 + r) * F + o] = tv * dt + X[(r0 + r) * F + o];
-                        }
-                    }
-                }
-                __syncwarp();
-            }
-            // Ei = X W3 + b3 ; backward seed dX = W3
-#pragma unroll
-            for (int r = 0; r < RW; ++r) {
+            fit_layer<T, R>(X, F, F, fw + FitOff::W1, [&](int o, int q, T v) {
+                const T tv = dev_tanh(v + fw[FitOff::B1 + o]);
+                T2[q] = tv;
+                X[q] = tv * fw[FitOff::DT1 + o] + X[q];
+            });
+            fit_layer<T, R>(X, F, F, fw + FitOff::W2, [&](int o, int q, T v) {
+                const T tv = dev_tanh(v + fw[FitOff::B2 + o]);
+                T3[q] = tv;
+                X[q] = tv * fw[FitOff::DT2 + o] + X[q];
+            });
+            // Ei = X W3 + b3
+            for (int r = warp; r < R; r += 8) {
                 T part = T(0);
 #pragma unroll
                 for (int q = 0; q < 2; ++q) {
                     const int o = lane + 32 * q;
-                    if (o < F) part += X[(r0 + r) * F + o] * fw[FitOff::W3 + o];
+                    if (o < F) part += X[r * F + o] * fw[FitOff::W3 + o];
                 }
                 part = warp_sum(part);
-                const long long t = t0 + r0 + r;
-                if (lane == 0 && t < total && rtype[r0 + r] == tt) Ei[t] = part + fw[FitOff::B3];
+                const long long t = t0 + r;
+                if (lane == 0 && t < total && rtype[r] == tt) Ei[t] = part + fw[FitOff::B3];
             }
-            __syncwarp();
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                const int o = lane + 32 * q;
-                if (o < F)
-#pragma unroll
-                    for (int r = 0; r < RW; ++r) X[(r0 + r) * F + o] = fw[FitOff::W3 + o];
+            __syncthreads();
+            // back through layers 2, 1 from dX = W3: g = dX * dt * (1 - t^2);  dX += g W^T
+            for (int q = threadIdx.x; q < R * F; q += blockDim.x) {
+                const int o = q % F;
+                const T dx = fw[FitOff::W3 + o], tv = T3[q];
+                X[q] = dx;
+                T3[q] = dx * fw[FitOff::DT2 + o] * (T(1) - tv * tv);
             }
-            __syncwarp();
-            // back through layers 2, 1: g = dX * dt * (1 - t^2);  dX += g W^T
-#pragma unroll
-            for (int l = 2; l >= 1; --l) {
-                const int OWT = l == 1 ? FitOff::W1T : FitOff::W2T;
-                const int OD = l == 1 ? FitOff::DT1 : FitOff::DT2;
-                T *Tl = l == 1 ? T2 : T3;
-                // g into Tl (tanh values no longer needed afterwards)
-#pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                    const int o = lane + 32 * q;
-                    if (o < F) {
-                        const T dt = fw[OD + o];
-#pragma unroll
-                        for (int r = 0; r < RW; ++r) {
-                            const T tv = Tl[(r0 + r) * F + o];
-                            Tl[(r0 + r) * F + o] = X[(r0 + r) * F + o] * dt * (T(1) - tv * tv);
-                        }
-                    }
-                }
-                __syncwarp();
-                T acc[RW][2];
-#pragma unroll
-                for (int r = 0; r < RW; ++r) { acc[r][0] = T(0); acc[r][1] = T(0); }
-                warp_gemm<T, RW, 2>(Tl + r0 * F, F, F, fw + OWT, F, F, lane, acc);
-#pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                    const int o = lane + 32 * q;
-                    if (o < F)
-#pragma unroll
-                        for (int r = 0; r < RW; ++r) X[(r0 + r) * F + o] += acc[r][q];
-                }
-                __syncwarp();
-            }
+            __syncthreads();
+            fit_layer<T, R>(T3, F, F, fw + FitOff::W2T, [&](int o, int q, T v) {
+                const T dx = X[q] + v, tv = T2[q];
+                X[q] = dx;
+                T2[q] = dx * fw[FitOff::DT1 + o] * (T(1) - tv * tv);
+            });
             // layer 0: g1 = dX * (1 - T1^2);  dD = g1 W0^T  (into Ds)
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                const int o = lane + 32 * q;
-                if (o < F)
-#pragma unroll
-                    for (int r = 0; r < RW; ++r) {
-                        const T tv = T1[(r0 + r) * F + o];
-                        T1[(r0 + r) * F + o] = X[(r0 + r) * F + o] * (T(1) - tv * tv);
-                    }
-            }
-            __syncwarp();
+            fit_layer<T, R>(T2, F, F, fw + FitOff::W1T, [&](int, int q, T v) {
+                const T tv = T1[q];
+                T1[q] = (X[q] + v) * (T(1) - tv * tv);
+            });
             {
-                constexpr int NC = (DIN + 31) / 32;   // 13
-                T acc[RW][NC];
+                T acc[R][2];
 #pragma unroll
-                for (int r = 0; r < RW; ++r)
+                for (int r = 0; r < R; ++r) acc[r][0] = acc[r][1] = T(0);
+                fit_gemm50<T, R>(T1, fw + FitOff::W0T + warp * F, DIN, lane, acc);
 #pragma unroll
-                    for (int q = 0; q < NC; ++q) acc[r][q] = T(0);
-                warp_gemm<T, RW, NC>(T1 + r0 * F, F, F, fw + FitOff::W0T, DIN, DIN, lane, acc);
-#pragma unroll
-                for (int q = 0; q < NC; ++q) {
-                    const int col = lane + 32 * q;
-                    if (col < DIN)
-#pragma unroll
-                        for (int r = 0; r < RW; ++r) Ds[(r0 + r) * DIN + col] = acc[r][q];
+                for (int r = 0; r < R; ++r) {
+                    Ds[r * DIN + warp * F + lane] = acc[r][0];
+                    if (lane + 32 < F) Ds[r * DIN + warp * F + lane + 32] = acc[r][1];
                 }
             }
             __syncthreads();
             // dA[r][c][p] = sum_q dD[p][q] A[c][q] + (p < M2 ? sum_p' dD[p'][p] A[c][p'] : 0)
-            for (int q = threadIdx.x; q < TILE * NA; q += blockDim.x) {
+            for (int q = threadIdx.x; q < R * NA; q += blockDim.x) {
                 const int r = q / NA, e = q - r * NA;
                 const long long t = t0 + r;
                 if (t >= total || rtype[r] != tt) continue;
@@ -534,16 +513,30 @@ dp_fit(const T *__restrict__ Ain, const int32_t *__restrict__ type_map,
             __syncthreads();
         }
         // rows without a present type
-        for (int q = threadIdx.x; q < TILE * NA; q += blockDim.x) {
+        for (int q = threadIdx.x; q < R * NA; q += blockDim.x) {
             const int r = q / NA;
             const long long t = t0 + r;
             if (t < total && rtype[r] < 0) dAout[t * NA + (q - r * NA)] = T(0);
         }
-        for (int r = threadIdx.x; r < TILE; r += blockDim.x) {
+        for (int r = threadIdx.x; r < R; r += blockDim.x) {
             const long long t = t0 + r;
             if (t < total && rtype[r] < 0) Ei[t] = T(0);
         }
     }
+}
+
+template <typename T, int R>
+int launch_fit(const T *A, const int32_t *type_map, const T *params, T *Ei, T *dA,
+               const EvalParams &P, cudaStream_t s) {
+    const size_t smem = sizeof(T) * (size_t)R * (NA + DIN + 4 * F);
+    if (cudaFuncSetAttribute(dp_fit<T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)smem) != cudaSuccess)
+        return check_launch("cudaFuncSetAttribute(dp_fit)");
+    const long long ntiles = ((long long)P.batch * P.natoms + R - 1) / R;
+    const int grid = (int)std::min<long long>(ntiles, (long long)device_sms() * 16);
+    ProfScope ps("dp_fit", s);
+    dp_fit<T, R><<<grid, 256, smem, s>>>(A, type_map, params, Ei, dA, P);
+    return check_launch("dp_fit");
 }
 
 // --------------------------------------------------------------------------- dp_embed_bwd
@@ -557,9 +550,10 @@ dp_embed_bwd(const int32_t *__restrict__ list_neigh, const T *__restrict__ idr,
     const int nnet = P.ntypes * P.ntypes;
     T *wsm = reinterpret_cast<T *>(smem_raw);
     const int wcount = WS ? nnet * EmbOff::SIZE : 0;
-    T *act_all = wsm + wcount;                                 // [kWarps][2][E][32]
-    T *dA_all = act_all + kWarps * 2 * E * 32;                 // [kWarps][NA]
-    int *list_all = reinterpret_cast<int *>(dA_all + kWarps * NA);
+    const int nwarps = blockDim.x >> 5;                        // 1 or kWarps
+    T *act_all = wsm + wcount;                                 // [nwarps][2][E][32]
+    T *dA_all = act_all + nwarps * 2 * E * 32;                 // [nwarps][NA]
+    int *list_all = reinterpret_cast<int *>(dA_all + nwarps * NA);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     T *t1s = act_all + warp * 2 * E * 32 + lane;
     T *t2s = t1s + E * 32;
@@ -569,8 +563,8 @@ dp_embed_bwd(const int32_t *__restrict__ list_neigh, const T *__restrict__ idr,
     const int S = P.nslots;
     const int nall = P.natoms + P.nghost;
     const long long total = (long long)P.batch * P.natoms;
-    for (long long t = (long long)blockIdx.x * kWarps + warp; t < total;
-         t += (long long)gridDim.x * kWarps) {
+    for (long long t = (long long)blockIdx.x * nwarps + warp; t < total;
+         t += (long long)gridDim.x * nwarps) {
         const int b = (int)(t / P.natoms);
         const int i = (int)(t - (long long)b * P.natoms);
         const int ti = type_map[i];
@@ -806,15 +800,21 @@ int launch_eval(int mode, const matpl_dp_model *M, const EvalParams &P,
         dp_pad<T><<<(nnet + 3) / 4, 128, 0, s>>>(params, davg, dstd, pad, P.ntypes, P);
     }
 
-    const long long nwarp_blocks = (total + kWarps - 1) / kWarps;
-    const int gridw = (int)(nwarp_blocks < (long long)device_sms() * 8 ? (nwarp_blocks < 1 ? 1 : nwarp_blocks) : (long long)device_sms() * 8);
+    // A small batch runs one-warp blocks, so that its atoms reach every SM before any SM takes a
+    // second: FP64 issues two lanes a clock per SM, and 108 atoms in four-warp blocks kept 27 SMs
+    // busy (forward + backward 1.5 ms, 0.97 ms in one-warp blocks).  Above 16 atoms per SM both
+    // shapes fill the chip and the four-warp block stages the nets a quarter as often.
+    const int nwarps = total < 16LL * device_sms() ? 1 : kWarps;
+    const long long nwarp_blocks = (total + nwarps - 1) / nwarps;
+    const int gridw = (int)std::max<long long>(
+        1, std::min<long long>(nwarp_blocks, (long long)device_sms() * 8 * (kWarps / nwarps)));
     const size_t wbytes = sizeof(T) * (size_t)nnet * EmbOff::SIZE;
     const bool ws_ok = wbytes <= 128 * 1024 && P.ctab == nullptr;   // tables: no net weights
     const size_t wpart = ws_ok ? wbytes : 0;
-    const size_t smem_f = wpart + sizeof(T) * kWarps * 32 * (E + 1 + 4) +
-                          sizeof(int) * kWarps * P.nslots;
-    const size_t smem_b = wpart + sizeof(T) * kWarps * (2 * E * 32 + NA) +
-                          sizeof(int) * kWarps * P.nslots;
+    const size_t smem_f = wpart + sizeof(T) * nwarps * 32 * (E + 1 + 4) +
+                          sizeof(int) * nwarps * P.nslots;
+    const size_t smem_b = wpart + sizeof(T) * nwarps * (2 * E * 32 + NA) +
+                          sizeof(int) * nwarps * P.nslots;
     auto kf = P.ctab ? dp_embed_fwd<T, false, true>
                      : (ws_ok ? dp_embed_fwd<T, true, false> : dp_embed_fwd<T, false, false>);
     auto kb = P.ctab ? dp_embed_bwd<T, false, true>
@@ -827,7 +827,7 @@ int launch_eval(int mode, const matpl_dp_model *M, const EvalParams &P,
         cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_f);
         cudaFuncSetAttribute(kb, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b);
         ProfScope ps("dp_embed_fwd", s);
-        kf<<<gridw, kWarps * 32, smem_f, s>>>(list_neigh, idr, type_map, params, davg, dstd, pad, A, P);
+        kf<<<gridw, nwarps * 32, smem_f, s>>>(list_neigh, idr, type_map, params, davg, dstd, pad, A, P);
     } else {
         st = prep_mixed_tiles((const float *)params, wt, P.ntypes, s);
         if (st) return st;
@@ -835,14 +835,15 @@ int launch_eval(int mode, const matpl_dp_model *M, const EvalParams &P,
                        nullptr, M->err_dev, s);
         if (st) return st;
     }
-    constexpr int TILE = sizeof(T) == 8 ? 32 : 64;
-    const size_t smem_fit = sizeof(T) * (size_t)TILE * (NA + DIN + 4 * F);
-    cudaFuncSetAttribute(dp_fit<T, TILE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_fit);
-    const long long ntiles = (total + TILE - 1) / TILE;
-    const int gridf = (int)(ntiles < (long long)device_sms() * 4 ? ntiles : (long long)device_sms() * 4);
     if (mode == MATPL_F32 || mode == MATPL_F64) {
-        ProfScope ps("dp_fit", s);
-        dp_fit<T, TILE><<<gridf, 256, smem_fit, s>>>(A, type_map, params, Ei, dA, P);
+        // the widest tile that still gives every SM one: at 108 atoms (FP64) one-atom tiles
+        // take 48 us where four 32-atom tiles took over 300
+        constexpr int RB = sizeof(T) == 8 ? 8 : 16;
+        const long long sms = device_sms();
+        if (total >= RB * sms) st = launch_fit<T, RB>(A, type_map, params, Ei, dA, P, s);
+        else if (total >= 4 * sms) st = launch_fit<T, 4>(A, type_map, params, Ei, dA, P, s);
+        else st = launch_fit<T, 1>(A, type_map, params, Ei, dA, P, s);
+        if (st) return st;
     } else {
         st = launch_fit_tc(mode != MATPL_MIXED_TANHF, (const float *)A, type_map, (const float *)params,
                            (unsigned char *)(ws + lay.ftiles), (float *)Ei, (float *)dA,
@@ -851,7 +852,7 @@ int launch_eval(int mode, const matpl_dp_model *M, const EvalParams &P,
     }
     if (simt_embed) {
         ProfScope ps("dp_embed_bwd", s);
-        kb<<<gridw, kWarps * 32, smem_b, s>>>(list_neigh, idr, type_map, params, davg, dstd, dA,
+        kb<<<gridw, nwarps * 32, smem_b, s>>>(list_neigh, idr, type_map, params, davg, dstd, dA,
                                               force, avir, P);
     } else {
         st = run_mixed(mode, true, P, list_neigh, idr, type_map, params, wt, davg, dstd, dA,

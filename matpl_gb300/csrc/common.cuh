@@ -166,6 +166,15 @@ template <> __device__ __forceinline__ float pair_r<float>(double dd) {
     return sqrt_to_f32(sqrtf(to_f32(dd)), dd);
 }
 
+// four consecutive values at a 16-byte aligned address
+__device__ __forceinline__ void store4(float *p, float a, float b, float c, float d) {
+    *reinterpret_cast<float4 *>(p) = make_float4(a, b, c, d);
+}
+__device__ __forceinline__ void store4(double *p, double a, double b, double c, double d) {
+    reinterpret_cast<double2 *>(p)[0] = make_double2(a, b);
+    reinterpret_cast<double2 *>(p)[1] = make_double2(c, d);
+}
+
 // bit pattern of a non-negative double: orders like the value (NaN above +inf)
 __device__ __forceinline__ unsigned long long ubits(double v) {
     return (unsigned long long)__double_as_longlong(v);

@@ -32,6 +32,8 @@ struct NbImage {
     int nb[3];       // cell bins per fractional axis (minimum-image branch)
     int ncells;
     int ortho;       // off-diagonal lattice entries all (signed) zero
+    float Lf[9];     // L and the squared pre-filter radius in FP32 (see maybe_within)
+    float thr2;
 };
 
 struct NbParams {
@@ -96,57 +98,54 @@ __device__ __forceinline__ bool lt_bits(double a, double b) {
     return __double_as_longlong(a) < __double_as_longlong(b);
 }
 
-__device__ __forceinline__ void store4(float *p, float a, float b, float c, float d) {
-    *reinterpret_cast<float4 *>(p) = make_float4(a, b, c, d);
-}
-__device__ __forceinline__ void store4(double *p, double a, double b, double c, double d) {
-    reinterpret_cast<double2 *>(p)[0] = make_double2(a, b);
-    reinterpret_cast<double2 *>(p)[1] = make_double2(c, d);
-}
-
+// One warp per image, lane k < 3 on cell vector k: the FP64 square roots and divisions of the
+// three directions run side by side (one thread doing all of them took 8 us per call).
 __global__ void nb_setup(const double *__restrict__ lattice, NbImage *__restrict__ img,
                          int batch, double Rc, int cell_cap) {
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < batch; b += gridDim.x * blockDim.x) {
-        NbImage im;
-        const double *L = lattice + 9 * b;
-        for (int q = 0; q < 9; ++q) im.L[q] = L[q];
-        im.iflag = 0;
-        for (int v = 0; v < 3; ++v) {
-            double d = sqrt(da(da(dm(L[3 * v], L[3 * v]), dm(L[3 * v + 1], L[3 * v + 1])),
-                               dm(L[3 * v + 2], L[3 * v + 2])));
-            im.nper[v] = (int)(Rc / d) + 1;
-            if (d < 2 * Rc) im.iflag = 1;
-        }
-        // thickness h_k = V / |a_i x a_j|
-        const double *a = L, *bb = L + 3, *c = L + 6;
-        double cr[3][3];
-        const double *vv[3][2] = {{bb, c}, {c, a}, {a, bb}};
-        for (int k = 0; k < 3; ++k) {
-            const double *p = vv[k][0], *q = vv[k][1];
-            cr[k][0] = p[1] * q[2] - p[2] * q[1];
-            cr[k][1] = p[2] * q[0] - p[0] * q[2];
-            cr[k][2] = p[0] * q[1] - p[1] * q[0];
-        }
-        const double V = fabs(a[0] * cr[0][0] + a[1] * cr[0][1] + a[2] * cr[0][2]);
-        long long prod = 1;
-        for (int k = 0; k < 3; ++k) {
-            double area = sqrt(cr[k][0] * cr[k][0] + cr[k][1] * cr[k][1] + cr[k][2] * cr[k][2]);
-            double h = V / area;
-            int n = (int)floor(h / (Rc * 1.0000001));
-            im.nb[k] = n < 1 ? 1 : (n > 1024 ? 1024 : n);
-        }
-        for (;;) {
-            prod = (long long)im.nb[0] * im.nb[1] * im.nb[2];
-            if (prod <= cell_cap) break;
-            int kmax = 0;
-            for (int k = 1; k < 3; ++k)
-                if (im.nb[k] > im.nb[kmax]) kmax = k;
-            im.nb[kmax] = (im.nb[kmax] + 1) / 2;
-        }
+    const int lane = threadIdx.x & 31;
+    const int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (b >= batch) return;                      // whole warps
+    const double *L = lattice + 9 * b;
+    const int k = lane < 3 ? lane : 0;
+    const double *a = L + 3 * k, *p = L + 3 * ((k + 1) % 3), *q = L + 3 * ((k + 2) % 3);
+    const double d = sqrt(da(da(dm(a[0], a[0]), dm(a[1], a[1])), dm(a[2], a[2])));
+    // thickness h_k = V / |a_i x a_j|
+    const double c0 = p[1] * q[2] - p[2] * q[1], c1 = p[2] * q[0] - p[0] * q[2],
+                 c2 = p[0] * q[1] - p[1] * q[0];
+    const double V = __shfl_sync(0xffffffffu, fabs(a[0] * c0 + a[1] * c1 + a[2] * c2), 0);
+    const double h = V / sqrt(c0 * c0 + c1 * c1 + c2 * c2);
+    int nb = (int)floor(h / (Rc * 1.0000001));
+    nb = nb < 1 ? 1 : (nb > 1024 ? 1024 : nb);
+    const int nper = (int)(Rc / d) + 1;
+    const unsigned small = __ballot_sync(0xffffffffu, lane < 3 && d < 2 * Rc);
+    int nbk[3];
+    for (int v = 0; v < 3; ++v) nbk[v] = __shfl_sync(0xffffffffu, nb, v);
+    long long prod = 1;
+    for (;;) {
+        prod = (long long)nbk[0] * nbk[1] * nbk[2];
+        if (prod <= cell_cap) break;
+        int kmax = 0;
+        for (int v = 1; v < 3; ++v)
+            if (nbk[v] > nbk[kmax]) kmax = v;
+        nbk[kmax] = (nbk[kmax] + 1) / 2;
+    }
+    NbImage &im = img[b];
+    if (lane < 3) im.nper[lane] = nper;
+    float lsum = 0.f;
+#pragma unroll
+    for (int e = 0; e < 9; ++e) lsum += fabsf((float)L[e]);
+    if (lane < 9) {
+        im.L[lane] = L[lane];
+        im.Lf[lane] = (float)L[lane];
+    }
+    if (lane == 0) {
+        for (int v = 0; v < 3; ++v) im.nb[v] = nbk[v];
+        im.iflag = small != 0u;
         im.ncells = im.iflag ? 0 : (int)prod;
         im.ortho = L[1] == 0.0 && L[2] == 0.0 && L[3] == 0.0 && L[5] == 0.0 && L[6] == 0.0 &&
                    L[7] == 0.0;
-        img[b] = im;
+        const float rc2f = (float)(Rc * Rc);
+        im.thr2 = rc2f + 0.01f + 1e-5f * lsum * sqrtf(rc2f);
     }
 }
 
@@ -251,26 +250,35 @@ __device__ __forceinline__ float mic_f(float d, bool &tie) {
     return d;
 }
 
+// ints of shared memory per warp: S sort keys and up to four closing ones (16-byte rows), then
+// 2 S candidates
+__host__ __device__ inline int nb_ints(int S) { return (S + 7) / 4 * 4 + (2 * S + 3) / 4 * 4; }
+
+// Bound: the FP64 pipe (two lanes a clock per SM) and the latency of the candidate gathers.  What
+// is uniform per image or atom (FP32 lattice, bin) is read instead of converted per atom, and the
+// rank sort reads four one-word keys a load: 32,000 atoms, 44 pairs each, 270 -> 238 us; 16 cells
+// of 96 atoms (27 images each) 51 -> 36 us.
 template <typename TO>
 __global__ void __launch_bounds__(kWarps * 32)
 nb_search(const NbImage *__restrict__ img, const double *__restrict__ wpos,
           const float4 *__restrict__ wpos32, const int32_t *__restrict__ type_map,
-          const int *__restrict__ cell_start, const int *__restrict__ cell_atoms,
+          const int *__restrict__ cell_of, const int *__restrict__ cell_start, const int *__restrict__ cell_atoms,
           int32_t *__restrict__ list_neigh, TO *__restrict__ image_dr,
           int32_t *__restrict__ num_neigh, int32_t *__restrict__ err, NbParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int S = P.ntypes * P.m;
     const int CAP = 2 * S;                         // pre-filtered candidates per atom
+    const int ISTR = nb_ints(S);                   // ints per warp: candidates, then sort keys
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // accepted pairs: the output row (r, x, y, z) in the output dtype (the f64 values are the
     // exact ones; the f32 ones their rounding, formed here once)
     constexpr int KV = sizeof(TO) * 4;              // bytes per accepted pair
     TO *kvec = reinterpret_cast<TO *>(smem_raw) + 4 * warp * S;
-    int *cand = reinterpret_cast<int *>(smem_raw + (size_t)KV * kWarps * S) + warp * (CAP + S);
-    int *keys = cand + CAP;
+    int *keys = reinterpret_cast<int *>(smem_raw + (size_t)KV * kWarps * S) + warp * ISTR;
+    int *cand = keys + (S + 7) / 4 * 4;
     unsigned char *ktype = reinterpret_cast<unsigned char *>(
                                reinterpret_cast<int *>(smem_raw + (size_t)KV * kWarps * S) +
-                               kWarps * (CAP + S)) + warp * S;
+                               kWarps * ISTR) + warp * S;
     const long long total = (long long)P.batch * P.natoms;
     for (long long t = (long long)blockIdx.x * kWarps + warp; t < total;
          t += (long long)gridDim.x * kWarps) {
@@ -286,14 +294,12 @@ nb_search(const NbImage *__restrict__ img, const double *__restrict__ wpos,
             if (lane == 0) atomicMax(err, MATPL_KERR_BAD_TYPE);
             continue;
         }
-        float Lf[9], lsum = 0.f;
+        // the FP32 lattice comes from nb_setup: converting it here, a warp-wide FP64
+        // instruction per entry and atom, was a third of the FP64 pipe's work
+        float Lf[9];
 #pragma unroll
-        for (int q = 0; q < 9; ++q) {
-            Lf[q] = (float)im.L[q];
-            lsum += fabsf(Lf[q]);
-        }
-        const float rc2f = (float)P.rc2;
-        const float thr2 = rc2f + 0.01f + 1e-5f * lsum * sqrtf(rc2f);
+        for (int q = 0; q < 9; ++q) Lf[q] = im.Lf[q];
+        const float thr2 = im.thr2;
         const int nimg1 = 2 * im.nper[2] + 1, nimg2 = 2 * im.nper[1] + 1;
         const int nimg = im.iflag ? (2 * im.nper[0] + 1) * nimg2 * nimg1 : 1;
 
@@ -306,19 +312,28 @@ nb_search(const NbImage *__restrict__ img, const double *__restrict__ wpos,
                 if (lane == 0) atomicMax(err, MATPL_KERR_BAD_BOX);
                 T = 0;
             }
+            // candidate c = (j, i1, i2, i3) in mixed radix, advanced by 32 per pass without
+            // divisions
+            const int n3 = nimg1, n2 = nimg2, n1 = 2 * im.nper[0] + 1;
+            const int s3 = 32 % n3, s2 = 32 / n3 % n2, s1 = 32 / n3 / n2 % n1, sj = 32 / n3 / n2 / n1;
+            int i3 = lane % n3, i2 = lane / n3 % n2, i1 = lane / n3 / n2 % n1, j = lane / n3 / n2 / n1;
             for (long long c0 = 0; c0 < T; c0 += 32) {
-                const long long c = c0 + lane;
                 bool keep = false;
                 int key = 0;
-                if (c < T) {
-                    const int j = (int)(c / nimg), idx = (int)(c - (long long)j * nimg);
-                    const int i3 = idx % nimg1 - im.nper[2];
-                    const int i2 = (idx / nimg1) % nimg2 - im.nper[1];
-                    const int i1 = idx / (nimg1 * nimg2) - im.nper[0];
+                if (j < P.natoms) {
                     const float4 fj = pos32[j];
-                    keep = maybe_within(Lf, fj.x - fi.x + i1, fj.y - fi.y + i2, fj.z - fi.z + i3, thr2);
-                    key = j * nimg + idx;
+                    keep = maybe_within(Lf, fj.x - fi.x + (i1 - im.nper[0]),
+                                        fj.y - fi.y + (i2 - im.nper[1]),
+                                        fj.z - fi.z + (i3 - im.nper[2]), thr2);
+                    key = ((j * n1 + i1) * n2 + i2) * n3 + i3;
                 }
+                i3 += s3;
+                if (i3 >= n3) { i3 -= n3; ++i2; }
+                i2 += s2;
+                if (i2 >= n2) { i2 -= n2; ++i1; }
+                i1 += s1;
+                if (i1 >= n1) { i1 -= n1; ++j; }
+                j += sj;
                 const unsigned mk = __ballot_sync(0xffffffffu, keep);
                 const int at = ncand + __popc(mk & ((1u << lane) - 1u));
                 if (keep && at < CAP) cand[at] = key;
@@ -326,17 +341,12 @@ nb_search(const NbImage *__restrict__ img, const double *__restrict__ wpos,
             }
         } else {
             // up to 9 (x, y) columns x 2 z-ranges; lane q < nr holds range q
-            int ci[3];
-            ci[0] = min((int)(fi.x * im.nb[0]), im.nb[0] - 1);
-            ci[1] = min((int)(fi.y * im.nb[1]), im.nb[1] - 1);
-            ci[2] = min((int)(fi.z * im.nb[2]), im.nb[2] - 1);
-            // the FP32 bin may differ from the FP64 bin at a bin edge: use the FP64 one
+            int ci[3];                          // the atom's bin, as nb_bin placed it
             {
-                const double f[3] = {pi0, pi1, pi2};
-                for (int k = 0; k < 3; ++k) {
-                    int q = (int)(f[k] * im.nb[k]);
-                    ci[k] = q >= im.nb[k] ? im.nb[k] - 1 : (q < 0 ? 0 : q);
-                }
+                const int cell = cell_of[t];
+                ci[2] = cell % im.nb[2];
+                ci[1] = cell / im.nb[2] % im.nb[1];
+                ci[0] = cell / im.nb[2] / im.nb[1];
             }
             const int *cs = cell_start + (long long)b * (P.cell_cap + 1);
             const int *ca = cell_atoms + (long long)b * P.natoms;
@@ -416,6 +426,11 @@ nb_search(const NbImage *__restrict__ img, const double *__restrict__ wpos,
 #pragma unroll
         for (int q = 0; q < kMaxTypes; ++q) cntM[q] = 0;
         int n_acc = 0;
+        int ncount[kMaxTypes];                  // stored pairs per neighbor type
+#pragma unroll
+        for (int q = 0; q < kMaxTypes; ++q) ncount[q] = 0;
+        // sort keys (type, j, image) in one word where j * images + image fits 27 bits
+        const bool one_word = (long long)P.natoms * nimg <= (1 << 27);
         const double rct2 = P.rct2[ti];
         for (int c0 = 0; c0 < ncand; c0 += 32) {
             // every lane evaluates a candidate (lanes past the end repeat the last one and are
@@ -453,8 +468,12 @@ nb_search(const NbImage *__restrict__ img, const double *__restrict__ wpos,
                 if (q < P.ntypes) cntM[q] += __popc(__ballot_sync(0xffffffffu, inM && tj == q));
             const unsigned ma = __ballot_sync(0xffffffffu, inT);
             const int at = n_acc + __popc(ma & ((1u << lane) - 1u));
-            if (inT && at < S) {
-                keys[at] = key;
+            const bool put = inT && at < S;
+#pragma unroll
+            for (int q = 0; q < kMaxTypes; ++q)
+                if (q < P.ntypes) ncount[q] += __popc(__ballot_sync(0xffffffffu, put && tj == q));
+            if (put) {
+                keys[at] = one_word ? (int)((unsigned)tj << 27 | (unsigned)key) : key;
                 ktype[at] = (unsigned char)tj;
                 store4(kvec + 4 * at, pair_r<TO>(pdd), conv<TO>(px), conv<TO>(py), conv<TO>(pz));
             }
@@ -465,24 +484,28 @@ nb_search(const NbImage *__restrict__ img, const double *__restrict__ wpos,
         for (int q = 0; q < kMaxTypes; ++q) overflow |= (q < P.ntypes) && cntM[q] > P.m;
         if (overflow && lane == 0) atomicMax(err, MATPL_KERR_NEIGHBOR_OVERFLOW);
         const int nst = n_acc < S ? n_acc : S;
+        if (lane < 4 && nst + lane < (S + 7) / 4 * 4) keys[nst + lane] = -1;   // above every key
         __syncwarp();
-        int ncount[kMaxTypes];
-#pragma unroll
-        for (int q = 0; q < kMaxTypes; ++q) {
-            int c = 0;
-            if (q < P.ntypes) {
-                for (int e = lane; e < nst; e += 32) c += ktype[e] == q;
-                c = warp_sum(c);
-            }
-            ncount[q] = c < P.m ? c : P.m;
-        }
         const long long row = t * (long long)S;
-        // ---- phase C: rank sort by (j, image) inside each type block, write occupied slots
+        // ---- phase C: rank sort by (j, image) inside each type block, write occupied slots.
+        // One-word keys: the rank in the block is the number of smaller keys minus the pairs of
+        // the lower types, four keys per 16-byte broadcast.
         for (int e = lane; e < nst; e += 32) {
-            const int key = keys[e];
             const int ty = ktype[e];
-            int rank = 0;
-            for (int f = 0; f < nst; ++f) rank += (ktype[f] == ty) & (keys[f] < key);
+            int key = keys[e], rank = 0;
+            if (one_word) {
+                const unsigned mine = (unsigned)key;
+                for (int f = 0; f < nst; f += 4) {
+                    const uint4 k4 = *reinterpret_cast<const uint4 *>(keys + f);
+                    rank += (k4.x < mine) + (k4.y < mine) + (k4.z < mine) + (k4.w < mine);
+                }
+#pragma unroll
+                for (int q = 0; q < kMaxTypes; ++q)
+                    if (q < ty) rank -= ncount[q];
+                key &= (1 << 27) - 1;
+            } else {
+                for (int f = 0; f < nst; ++f) rank += (ktype[f] == ty) & (keys[f] < key);
+            }
             if (rank >= P.m) continue;
             const int j = key / nimg;
             const TO *kv = kvec + 4 * e;
@@ -490,6 +513,8 @@ nb_search(const NbImage *__restrict__ img, const double *__restrict__ wpos,
             list_neigh[slot] = j + 1;
             store4(image_dr + 4 * slot, kv[0], kv[1], kv[2], kv[3]);
         }
+#pragma unroll
+        for (int q = 0; q < kMaxTypes; ++q) ncount[q] = min(ncount[q], P.m);
         // ---- phase D: clear the empty slots (the occupied-slot form leaves them untouched:
         // its readers take the block lengths from num_neigh)
         for (int s = lane; s < S && !P.occupied_only; s += 32) {
@@ -646,25 +671,25 @@ static int neighbor_build(int batch, int natoms, int ntypes, int m_neigh, double
     const long long na = (long long)batch * natoms;
     {
         ProfScope ps("nb_cells", s);
-        nb_setup<<<(batch + 127) / 128, 128, 0, s>>>(lattice, img, batch, Rc_M, P.cell_cap);
+        nb_setup<<<(batch + 3) / 4, 128, 0, s>>>(lattice, img, batch, Rc_M, P.cell_cap);
         nb_bin<<<grid_for(na, 256), 256, 0, s>>>(frac_pos, img, wpos, wpos32, cell_of, cell_count, P);
         nb_scan<<<batch, 1024, 0, s>>>(img, cell_count, cell_start, P);
         nb_fill<<<grid_for(na, 256), 256, 0, s>>>(cell_of, cell_start, cell_fill, cell_atoms, P);
     }
     ProfScope ps("nb_search", s);
     const int S = ntypes * m_neigh;
-    const size_t smem = (size_t)kWarps * (S * 4 * (out_dtype == MATPL_F64 ? 8 : 4) + 3 * S * 4 + S);
+    const size_t smem = (size_t)kWarps * (S * 4 * (out_dtype == MATPL_F64 ? 8 : 4) + nb_ints(S) * 4 + S);
     if (out_dtype == MATPL_F64) {
         cudaFuncSetAttribute(nb_search<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem);
         nb_search<double><<<grid_for(na, kWarps), kWarps * 32, smem, s>>>(
-            img, wpos, wpos32, type_map, cell_start, cell_atoms, list_neigh, (double *)image_dr,
+            img, wpos, wpos32, type_map, cell_of, cell_start, cell_atoms, list_neigh, (double *)image_dr,
             num_neigh, err_dev, P);
     } else {
         cudaFuncSetAttribute(nb_search<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem);
         nb_search<float><<<grid_for(na, kWarps), kWarps * 32, smem, s>>>(
-            img, wpos, wpos32, type_map, cell_start, cell_atoms, list_neigh, (float *)image_dr,
+            img, wpos, wpos32, type_map, cell_of, cell_start, cell_atoms, list_neigh, (float *)image_dr,
             num_neigh, err_dev, P);
     }
     return check_launch("matpl_neighbor_build");

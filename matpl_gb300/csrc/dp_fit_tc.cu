@@ -2,9 +2,14 @@
 //
 // Same math as dp_fused.cu's dp_fit (src/model/dp_embedding.py:140-163 and dp_dp.py:304-342 plus
 // the autograd adjoint down to dE/dA): per atom D = A^T A[:, :16] (400), Ei = fit(D), dE/dA.
-// Atoms are first sorted by element (fit_order, a stable counting sort), so that a CTA of 128
-// threads owns a tile of 128 atoms of one element (thread r = atom r, MMA M = 128) and runs
-// that element's net only:
+// Atoms are first sorted by element (fit_order, a stable counting sort), so that a CTA owns a
+// tile of 128 atoms of one element (MMA M = 128) and runs that element's net only.  Two threads
+// share an atom: thread (r, half) forms one of the two D columns of a chunk, holds 32 of the 64
+// (padded) hidden columns and two of the four rows of dE/dA.  A tile is one chain of 24 dependent
+// steps, so its length is what the kernel takes at any batch up to two tiles per SM.  One thread
+// per atom, weights copied in front of each step and dE/dA added up in global memory took 84 us
+// per tile and 122 us for 250 tiles (32,000 atoms); two threads, weights copied behind the step
+// before and dE/dA kept on chip take 37 and 53 us.
 //
 //   layer 1  h1 = D W0: 13 K-chunks of 32; each chunk of D is built on the SIMT cores from the
 //            atom's A (kept in shared memory) and double-buffered into the MMA (N = 64, the 50
@@ -24,7 +29,9 @@ namespace matpl {
 namespace {
 
 using namespace dp;
-constexpr int FM = 128;                   // atoms per tile = threads
+constexpr int FM = 128;                   // atoms per tile
+constexpr int FT = 2 * FM;                // threads
+constexpr int HC = 32;                    // hidden columns per thread
 constexpr int FN = 64;                    // padded fitting width
 constexpr int K1C = 13;                   // K chunks of layer 1 (32 each; 400 padded to 416)
 constexpr int NDC = 7;                    // N chunks of dE/dD (64 each; 400 padded to 448)
@@ -111,16 +118,9 @@ __device__ __forceinline__ void cp_async_wait_all() {
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-__device__ __forceinline__ void copy_tiles(const unsigned char *__restrict__ src, unsigned char *dst,
-                                           int bytes) {
-    const uint4 *s4 = reinterpret_cast<const uint4 *>(src);
-    uint4 *d4 = reinterpret_cast<uint4 *>(dst);
-    for (int q = threadIdx.x; q < bytes / 16; q += blockDim.x) d4[q] = __ldg(s4 + q);
-}
-
-// Row r of a 128-row K-major tile: NK values as BF16 hi and lo halves.
+// Row r of a 128-row K-major tile: NK values from column 8 c0 as BF16 hi and lo halves.
 template <int NK>
-__device__ __forceinline__ void store_row_hilo(unsigned char *hi, unsigned char *lo, int r,
+__device__ __forceinline__ void store_row_hilo(unsigned char *hi, unsigned char *lo, int r, int c0,
                                                const float *v) {
 #pragma unroll
     for (int c = 0; c < NK / 8; ++c) {
@@ -130,8 +130,8 @@ __device__ __forceinline__ void store_row_hilo(unsigned char *hi, unsigned char 
             h[q] = v[8 * c + q];
             l[q] = v[8 * c + q] - __bfloat162float(__float2bfloat16_rn(v[8 * c + q]));
         }
-        tc::store_row8(hi, r, c, XKS, h);
-        tc::store_row8(lo, r, c, XKS, l);
+        tc::store_row8(hi, r, c0 + c, XKS, h);
+        tc::store_row8(lo, r, c0 + c, XKS, l);
     }
 }
 
@@ -163,12 +163,6 @@ __device__ __forceinline__ void issue_split3(uint32_t tmem, const unsigned char 
             acc = 1u;
         }
     }
-}
-
-__device__ __forceinline__ void ld64(uint32_t tmem, float v[64]) {
-    const uint32_t base = tmem + ((uint32_t)((threadIdx.x >> 5) * 32) << 16);
-    tc::tmem_ld32(base, v);
-    tc::tmem_ld32(base + 32, v + 32);
 }
 
 template <bool FAST>
@@ -254,13 +248,15 @@ __global__ void fit_order_scatter(const int32_t *__restrict__ type_map, int nato
     }
 }
 
-__device__ __forceinline__ void st64(uint32_t taddr, const float v[64]) {
-    tc::tmem_st32(taddr, v);
-    tc::tmem_st32(taddr + 32, v + 32);
+// 4-byte asynchronous copy, or a zero where !ok
+__device__ __forceinline__ void copy4_async(const float *src, float *dst, bool ok) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(tc::smem_u32(dst)), "l"(src),
+                 "r"(ok ? 4 : 0)
+                 : "memory");
 }
 
 template <bool FAST>
-__global__ void __launch_bounds__(FM, 2)
+__global__ void __launch_bounds__(FT, 2)
 dp_fit_tc(const float *__restrict__ Ain, const int *__restrict__ order,
           const int *__restrict__ type_start, const float *__restrict__ params,
           const unsigned char *__restrict__ ftiles, float *__restrict__ Ei,
@@ -271,11 +267,13 @@ dp_fit_tc(const float *__restrict__ Ain, const int *__restrict__ order,
     __shared__ uint32_t tmem_base;
     __shared__ long long ratom[FM];
     __shared__ float vec[6 * FN + 4];
+    __shared__ float esum[FM];
     float *As = reinterpret_cast<float *>(smem_raw);
     unsigned char *XB = reinterpret_cast<unsigned char *>(As + FM * ASTR);
     unsigned char *WB = XB + 2 * X64;
-    const int r = threadIdx.x, warp = r >> 5;
-    if (r == 0) {
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const int r = tid & (FM - 1), half = tid >> 7, col0 = HC * half;
+    if (tid == 0) {
         tc::mbar_init(&mbar[0], 1);
         tc::mbar_init(&mbar[1], 1);
     }
@@ -284,7 +282,9 @@ dp_fit_tc(const float *__restrict__ Ain, const int *__restrict__ order,
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = tmem_base;
-    const uint32_t lane_q = (uint32_t)(warp * 32) << 16;
+    // this thread's row and columns of the accumulator and of the stashes (warp w reaches the
+    // TMEM lanes of quarter w % 4)
+    const uint32_t tmine = tmem + ((uint32_t)((warp & 3) * 32) << 16) + col0;
     uint32_t ph[2] = {0u, 0u};
     bool ok = true;
     const long long woff = (long long)ntypes * ntypes * EmbOff::SIZE;
@@ -308,58 +308,53 @@ dp_fit_tc(const float *__restrict__ Ain, const int *__restrict__ order,
         const int idx = type_start[tt] + chunk * FM + r;
         const bool valid = idx < type_start[tt + 1];
         const long long t = valid ? b * natoms + order[idx] : -1;
-        __syncthreads();
-        ratom[r] = t;
-        __syncthreads();
-        for (int q = r; q < FM * NA; q += FM) {
-            const int row = q / NA, e = q - row * NA;
-            const long long tr = ratom[row];
-            As[row * ASTR + e] = tr >= 0 ? Ain[tr * NA + e] : 0.f;
-        }
-        __syncthreads();
-        const float *a = As + r * ASTR;
+        const unsigned char *tw = ftiles + (size_t)tt * FIT_TILE_BYTES;
+        __syncthreads();                           // the previous tile's buffers are free
+        copy_tiles_async(tw + OFF_F0, WB, 2 * W32);
+        if (half == 0) ratom[r] = t;
         {
             const float *fw = params + woff + (long long)tt * FitOff::SIZE;
-            const unsigned char *tw = ftiles + (size_t)tt * FIT_TILE_BYTES;
-            __syncthreads();
-            for (int q = r; q < 6 * FN; q += FM) {
+            for (int q = tid; q < 6 * FN; q += FT) {
                 const int part = q / FN, o = q - part * FN;
                 vec[q] = o < F ? fw[vsrc[part] + o] : 0.f;
             }
-            if (r == 0) vec[6 * FN] = fw[FitOff::B3];
-            __syncthreads();
-            const bool mine = valid;
-            // ---- layer 1: 13 double-buffered K chunks of D W0.  The weights of chunk c + 1
-            // are copied asynchronously while chunk c is formed and multiplied; buffer b of
-            // chunk c is free once the MMA of chunk c - 2 is done (waited at the end of the
-            // previous chunk, before that chunk's prefetch).
+            if (tid == 0) vec[6 * FN] = fw[FitOff::B3];
+        }
+        __syncthreads();
+        for (int q = tid; q < FM * NA; q += FT) {
+            const int row = q / NA, e = q - row * NA;
+            const long long tr = ratom[row];
+            copy4_async(Ain + (tr >= 0 ? tr * NA + e : 0), As + row * ASTR + e, tr >= 0);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        cp_async_wait_all();
+        __syncthreads();
+        float *a = As + r * ASTR;
+        // ---- layer 1: 13 double-buffered K chunks of D W0.  The weights of chunk c + 1
+        // are copied asynchronously while chunk c is formed and multiplied; buffer b of
+        // chunk c is free once the MMA of chunk c - 2 is done (waited at the end of the
+        // previous chunk, before that chunk's prefetch).
+        {
             float aq[4][M2];                      // A[c][q], q < M2: every chunk's right factor
 #pragma unroll
             for (int c4 = 0; c4 < 4; ++c4)
 #pragma unroll
                 for (int q = 0; q < M2; ++q) aq[c4][q] = a[c4 * E + q];
-            copy_tiles_async(tw + OFF_F0, WB, 2 * W32);
             for (int c = 0; c < K1C; ++c) {
                 const int b = c & 1;
-                float d[32];
+                const int p = 2 * c + half;
+                float d[16];
+                const float ap0 = p < E ? a[p] : 0.f, ap1 = p < E ? a[E + p] : 0.f,
+                            ap2 = p < E ? a[2 * E + p] : 0.f, ap3 = p < E ? a[3 * E + p] : 0.f;
 #pragma unroll
-                for (int h2 = 0; h2 < 2; ++h2) {
-                    const int p = 2 * c + h2;
-                    const float ap0 = p < E ? a[p] : 0.f, ap1 = p < E ? a[E + p] : 0.f,
-                                ap2 = p < E ? a[2 * E + p] : 0.f, ap3 = p < E ? a[3 * E + p] : 0.f;
-#pragma unroll
-                    for (int q = 0; q < 16; ++q) {
-                        const int k = 32 * c + 16 * h2 + q;
-                        d[16 * h2 + q] = k < DIN ? ap0 * aq[0][q] + ap1 * aq[1][q] +
-                                                       ap2 * aq[2][q] + ap3 * aq[3][q]
-                                                 : 0.f;
-                    }
-                }
+                for (int q = 0; q < 16; ++q)
+                    d[q] = p < E ? ap0 * aq[0][q] + ap1 * aq[1][q] + ap2 * aq[2][q] + ap3 * aq[3][q]
+                                 : 0.f;
                 unsigned char *xh = XB + b * 2 * X32;
-                store_row_hilo<32>(xh, xh + X32, r, d);
+                store_row_hilo<16>(xh, xh + X32, r, 2 * half, d);
                 cp_async_wait_all();
                 mma_sync_point();
-                if (r == 0) {
+                if (tid == 0) {
                     issue_split3<2>(tmem, xh, xh + X32, WB + b * 2 * W32, WB + b * 2 * W32 + W32, c > 0);
                     tc::commit(&mbar[b]);
                 }
@@ -372,122 +367,139 @@ dp_fit_tc(const float *__restrict__ Ain, const int *__restrict__ order,
                                      WB + (b ^ 1) * 2 * W32, 2 * W32);
                 }
             }
-            ok &= tc::mbar_wait(&mbar[1], ph[1], kWait);
-            ph[1] ^= 1u;
+        }
+        ok &= tc::mbar_wait(&mbar[1], ph[1], kWait);
+        ph[1] ^= 1u;
+        ok &= tc::mbar_wait(&mbar[0], ph[0], kWait);
+        ph[0] ^= 1u;
+        tc::fence_after_sync();
+        // from here on every step's weights are copied while the step before it is finished on
+        // the SIMT cores (the MMA that read the buffer is done).  real(o): hidden column, not
+        // padding (those stay zero whatever an overflown row holds).
+        auto real = [&](int o) { return o < F - HC || half == 0; };
+        copy_tiles_async(tw + OFF_F1, WB, 2 * W64);
+        float h[HC], x[HC];
+        tc::tmem_ld32(tmine, h);
+#pragma unroll
+        for (int o = 0; o < HC; ++o) x[o] = real(o) ? fit_act<FAST>(h[o] + vec[col0 + o]) : 0.f;
+        tc::tmem_st32(tmine + 64, x);
+        auto run_mma64 = [&]() {                      // accumulator = X W of the staged tiles
+            cp_async_wait_all();
+            mma_sync_point();
+            if (tid == 0) {
+                issue_split3<4>(tmem, XB, XB + X64, WB, WB + W64, false);
+                tc::commit(&mbar[0]);
+            }
             ok &= tc::mbar_wait(&mbar[0], ph[0], kWait);
             ph[0] ^= 1u;
             tc::fence_after_sync();
-            float h[64], x[64];
-            ld64(tmem, h);
-#pragma unroll
-            for (int o = 0; o < 64; ++o) x[o] = o < F ? fit_act<FAST>(h[o] + vec[o]) : 0.f;
-            st64(tmem + 64 + lane_q, x);
-            // ---- layers 2, 3
+        };
+        // ---- layers 2, 3
 #pragma unroll 1
-            for (int l = 1; l <= 2; ++l) {
-                store_row_hilo<64>(XB, XB + X64, r, x);
-                copy_tiles(tw + (l == 1 ? OFF_F1 : OFF_F2), WB, 2 * W64);
-                mma_sync_point();
-                if (r == 0) {
-                    issue_split3<4>(tmem, XB, XB + X64, WB, WB + W64, false);
-                    tc::commit(&mbar[0]);
-                }
-                ok &= tc::mbar_wait(&mbar[0], ph[0], kWait);
-                ph[0] ^= 1u;
-                tc::fence_after_sync();
-                ld64(tmem, h);
-                const float *bias = vec + (l == 1 ? FN : 3 * FN);
-                const float *dt = vec + (l == 1 ? 2 * FN : 4 * FN);
+        for (int l = 1; l <= 2; ++l) {
+            store_row_hilo<HC>(XB, XB + X64, r, 4 * half, x);
+            run_mma64();
+            copy_tiles_async(tw + (l == 1 ? OFF_F2 : OFF_B2), WB, 2 * W64);
+            tc::tmem_ld32(tmine, h);
+            const float *bias = vec + (l == 1 ? FN : 3 * FN) + col0;
+            const float *dt = vec + (l == 1 ? 2 * FN : 4 * FN) + col0;
 #pragma unroll
-                for (int o = 0; o < 64; ++o) {
-                    h[o] = o < F ? fit_act<FAST>(h[o] + bias[o]) : 0.f;
-                    if (o < F) x[o] = h[o] * dt[o] + x[o];
-                }
-                st64(tmem + 64 + 64 * l + lane_q, h);
+            for (int o = 0; o < HC; ++o) {
+                h[o] = real(o) ? fit_act<FAST>(h[o] + bias[o]) : 0.f;
+                x[o] = fmaf(h[o], dt[o], x[o]);
             }
+            tc::tmem_st32(tmine + 64 + 64 * l, h);
+        }
+        // Ei in column order: the first half's sum, then the second half's terms
+        if (half == 0) {
             float e = vec[6 * FN];
 #pragma unroll
-            for (int o = 0; o < F; ++o) e += x[o] * vec[5 * FN + o];
-            if (mine) Ei[t] = e;
-            // ---- adjoint: dx3 = W3; through layers 3 and 2
+            for (int o = 0; o < HC; ++o) e += x[o] * vec[5 * FN + o];
+            esum[r] = e;
+        }
+        __syncthreads();
+        if (half == 1 && valid) {
+            float e = esum[r];
 #pragma unroll
-            for (int o = 0; o < F; ++o) x[o] = vec[5 * FN + o];
+            for (int o = 0; o < F - HC; ++o) e += x[o] * vec[5 * FN + HC + o];
+            Ei[t] = e;
+        }
+        // ---- adjoint: dx3 = W3; through layers 3 and 2
+#pragma unroll
+        for (int o = 0; o < HC; ++o) x[o] = vec[5 * FN + col0 + o];
 #pragma unroll 1
-            for (int l = 2; l >= 1; --l) {
-                const float *dt = vec + (l == 2 ? 4 * FN : 2 * FN);
-                ld64(tmem + 64 + 64 * l, h);          // tanh outputs of layer l
+        for (int l = 2; l >= 1; --l) {
+            const float *dt = vec + (l == 2 ? 4 * FN : 2 * FN) + col0;
+            tc::tmem_ld32(tmine + 64 + 64 * l, h);    // tanh outputs of layer l
 #pragma unroll
-                for (int o = 0; o < 64; ++o) h[o] = o < F ? x[o] * dt[o] * (1.f - h[o] * h[o]) : 0.f;
-                store_row_hilo<64>(XB, XB + X64, r, h);
-                copy_tiles(tw + (l == 2 ? OFF_B2 : OFF_B1), WB, 2 * W64);
-                mma_sync_point();
-                if (r == 0) {
-                    issue_split3<4>(tmem, XB, XB + X64, WB, WB + W64, false);
-                    tc::commit(&mbar[0]);
-                }
-                ok &= tc::mbar_wait(&mbar[0], ph[0], kWait);
-                ph[0] ^= 1u;
-                tc::fence_after_sync();
-                ld64(tmem, h);
+            for (int o = 0; o < HC; ++o) h[o] = real(o) ? x[o] * dt[o] * (1.f - h[o] * h[o]) : 0.f;
+            store_row_hilo<HC>(XB, XB + X64, r, 4 * half, h);
+            run_mma64();
+            copy_tiles_async(tw + (l == 2 ? OFF_B1 : OFF_B0), WB, 2 * W64);
+            tc::tmem_ld32(tmine, h);
 #pragma unroll
-                for (int o = 0; o < F; ++o) x[o] += h[o];
-            }
-            ld64(tmem + 64, h);                       // tanh outputs of layer 1
+            for (int o = 0; o < HC; ++o) x[o] += h[o];     // padding: masked when it is used
+        }
+        tc::tmem_ld32(tmine + 64, h);                 // tanh outputs of layer 1
 #pragma unroll
-            for (int o = 0; o < 64; ++o) h[o] = o < F ? x[o] * (1.f - h[o] * h[o]) : 0.f;
-            store_row_hilo<64>(XB, XB + X64, r, h);
-            // ---- dE/dD = g1 W0^T in 7 chunks of 64 D entries, folded into dE/dA
-            float acc2[4][16];
+        for (int o = 0; o < HC; ++o) h[o] = real(o) ? x[o] * (1.f - h[o] * h[o]) : 0.f;
+        store_row_hilo<HC>(XB, XB + X64, r, 4 * half, h);
+        // ---- dE/dD = g1 W0^T in 7 chunks of 64 D entries (columns p = 4c + j, q), folded into
+        // rows 2 half and 2 half + 1 of dE/dA:
+        //   dA[c4][p] = sum_q dD[p][q] A[c4][q] (+ sum_p' dD[p'][p] A[c4][p'] for p < 16).
+        // Column p of A is used by chunk c only when p >= 16, so dA[p] replaces it in shared
+        // memory; the first 16 columns wait in registers for their second sum.
+        float acc2[2][16], first[2][16];
 #pragma unroll
-            for (int c4 = 0; c4 < 4; ++c4)
+        for (int k = 0; k < 2; ++k)
 #pragma unroll
-                for (int q = 0; q < 16; ++q) acc2[c4][q] = 0.f;
-#pragma unroll 1
-            for (int c = 0; c < NDC; ++c) {
-                copy_tiles(tw + OFF_B0 + (size_t)c * 2 * W64, WB, 2 * W64);
-                mma_sync_point();
-                if (r == 0) {
-                    issue_split3<4>(tmem, XB, XB + X64, WB, WB + W64, false);
-                    tc::commit(&mbar[0]);
-                }
-                ok &= tc::mbar_wait(&mbar[0], ph[0], kWait);
-                ph[0] ^= 1u;
-                tc::fence_after_sync();
-                ld64(tmem, h);                        // h[n] = dE/dD[64c + n]
+            for (int q = 0; q < 16; ++q) acc2[k][q] = 0.f;
+        float *ah = a + 2 * half * E;
 #pragma unroll
-                for (int c4 = 0; c4 < 4; ++c4) {
-                    float ap[4], sj[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int c = 0; c < NDC; ++c) {
+            run_mma64();
+            if (c + 1 < NDC) copy_tiles_async(tw + OFF_B0 + (size_t)(c + 1) * 2 * W64, WB, 2 * W64);
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) ap[j] = 4 * c + j < E ? a[c4 * E + 4 * c + j] : 0.f;
+            for (int jp = 0; jp < 4; jp += 2) {       // two D columns at a time
+                if (4 * c + jp >= E) break;
+                tc::tmem_ld32(tmine - col0 + 16 * jp, h);
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    float sj[2] = {0.f, 0.f};
 #pragma unroll
                     for (int q = 0; q < M2; ++q) {
-                        const float aqv = a[c4 * E + q];
-                        float acc = acc2[c4][q];
+                        const float aqv = ah[k * E + q];
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            if (4 * c + j >= E) break;
+                        for (int j = 0; j < 2; ++j) {
+                            if (4 * c + jp + j >= E) break;
                             sj[j] += h[16 * j + q] * aqv;
-                            acc += h[16 * j + q] * ap[j];
+                            acc2[k][q] += h[16 * j + q] * ah[k * E + 4 * c + jp + j];
                         }
-                        acc2[c4][q] = acc;
                     }
 #pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        if (mine && 4 * c + j < E) dAout[t * NA + c4 * E + 4 * c + j] = sj[j];
+                    for (int j = 0; j < 2; ++j) {
+                        if (4 * c + jp + j >= E) break;
+                        if (4 * c + jp + j < 16) first[k][(4 * c + jp + j) & 15] = sj[j];
+                        else ah[k * E + 4 * c + jp + j] = sj[j];
+                    }
                 }
             }
-            if (mine) {
+        }
 #pragma unroll
-                for (int c4 = 0; c4 < 4; ++c4)
+        for (int k = 0; k < 2; ++k)
 #pragma unroll
-                    for (int q = 0; q < M2; ++q) dAout[t * NA + c4 * E + q] += acc2[c4][q];
-            }
+            for (int q = 0; q < 16; ++q) ah[k * E + q] = first[k][q] + acc2[k][q];
+        __syncthreads();
+        for (int q = tid; q < FM * NA; q += FT) {
+            const int row = q / NA, e = q - row * NA;
+            const long long tr = ratom[row];
+            if (tr >= 0) dAout[tr * NA + e] = As[row * ASTR + e];
         }
     }
     // atoms whose element is not evaluated: Ei = 0, dE/dA = 0
     const int nskip = type_start[ntypes + 1] - type_start[ntypes];
-    for (long long q = (long long)blockIdx.x * FM + r; q < (long long)batch * nskip;
-         q += (long long)gridDim.x * FM) {
+    for (long long q = (long long)blockIdx.x * FT + tid; q < (long long)batch * nskip;
+         q += (long long)gridDim.x * FT) {
         const long long b = q / nskip;
         const long long t = b * natoms + order[type_start[ntypes] + (int)(q - b * nskip)];
         Ei[t] = 0.f;
@@ -497,7 +509,7 @@ dp_fit_tc(const float *__restrict__ Ain, const int *__restrict__ order,
     // nothing issued may still run when the TMEM is freed: one more commit after all of this
     // thread's MMAs, waited for (bounded) by every thread
     __shared__ __align__(8) uint64_t mbar_drain;
-    if (r == 0) {
+    if (tid == 0) {
         tc::mbar_init(&mbar_drain, 1);
         tc::commit(&mbar_drain);
     }
@@ -545,7 +557,7 @@ int launch_fit_tc(bool fast, const float *A, const int32_t *type_map, const floa
     auto k = fast ? dp_fit_tc<true> : dp_fit_tc<false>;
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FIT_SMEM);
     ProfScope ps("dp_fit_tc", s);
-    k<<<grid, FM, FIT_SMEM, s>>>(A, order, type_start, params, tiles, Ei, dA, err, batch, natoms,
+    k<<<grid, FT, FIT_SMEM, s>>>(A, order, type_start, params, tiles, Ei, dA, err, batch, natoms,
                                  ntypes);
     return check_launch("dp_fit_tc");
 }

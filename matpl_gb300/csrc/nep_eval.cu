@@ -5,7 +5,8 @@
 // calculateNepForce / calculateNepVirial (src/op/kernel/calculateNepForce.cu,
 // calculateNepVirial.cu).
 //
-// One warp owns one centre atom at a time (a contiguous run of atoms per warp):
+// One warp owns one centre atom at a time; a run of consecutive atoms belongs to one warp, or to
+// two that take its atoms in turn (see the kernel):
 //   radial    lanes over radial slots: Chebyshev basis f_k(r) (cal_fk, nep_net.py:691-715),
 //             q_n = sum_j sum_k c2[ti,tj,n,k] f_k, warp-reduced;
 //   angular   lanes over angular slots in chunks of 32: g_n(r) and the 24 real harmonics
@@ -18,13 +19,17 @@
 //             form, F_i += f_ij, F_j -= f_ij (float4 reductions into a padded accumulator),
 //             virial[a*3+c] -= f_a r_c kept per lane and reduced once per frame.
 // Nothing per pair or per feature goes to HBM.  Energies and the virial are summed in FP64.
+#include <algorithm>
+
 #include "common.cuh"
 #include "nep_math.cuh"
+#include "tc.cuh"
 
 namespace matpl {
 namespace {
 
-constexpr int kWarpsPerBlock = 8;
+constexpr int kRunsPerBlock = 8;
+constexpr int kTurnPolls = 1 << 24;
 constexpr int kMaxHidden = 128;
 
 struct NepLayout {
@@ -62,6 +67,8 @@ struct EvalArgs {
     int smem_params, warp_bytes;
     int o_stash_g, o_stash_b, o_s, o_dEds, o_fin, o_dq, o_dpre;
     int o_rj, o_rv, o_rgp, o_aj, o_av, o_ag, o_agp;
+    int pair;                // 1: two warps per run
+    int o_vir;               // pair: the run's virial sums, [runs of the block][9][32]
 };
 
 // f64 -> f32, round to nearest even, with integer instructions: the FP64 pipe of this part
@@ -153,22 +160,39 @@ __device__ __forceinline__ void list_pair(const EvalArgs &A, bool radial, long l
 }
 
 template <typename T>
-__device__ __forceinline__ void flush_frame(const EvalArgs &A, int frame, double e, T *vir,
-                                            int lane) {
+__device__ __forceinline__ void flush_virial(const EvalArgs &A, int frame, T *vir, int lane) {
 #pragma unroll
     for (int q = 0; q < 9; ++q) {
         const double v = warp_sum((double)vir[q]);
         if (lane == 0 && v != 0.0) atomicAdd(A.virial + 9 * frame + q, v);
         vir[q] = T(0);
     }
+}
+__device__ __forceinline__ void flush_energy(const EvalArgs &A, int frame, double e, int lane) {
     if (lane == 0 && e != 0.0) atomicAdd(A.Etot + frame, e);
 }
 
+__device__ __forceinline__ void mbar_arrive(uint64_t *mbar) {
+    asm volatile("{\n.reg .b64 t;\nmbarrier.arrive.shared::cta.b64 t, [%0];\n}\n" ::"r"(tc::smem_u32(mbar))
+                 : "memory");
+}
+
+// FP32 at the common sizes; the wide form's lists leave no room for twice the warps
+template <typename T, int NRM>
+constexpr bool can_pair() { return sizeof(T) == 4 && NRM <= 5; }
+
 // NRM / KRM / NAM / KAM: compiled maxima of n_max + 1 and basis_size + 1; EX: the model has
 // exactly these sizes (the size guards inside the unrolled loops then fold away).
+//
+// Bound: latency.  An atom is ~20 dependent phases, half of the issue slots are empty at 16 warps
+// per SM, and the virial ties a run's atoms together: its per-lane sums run over the atoms in order.
+// Where shared memory leaves room for one 8-run block per SM, two warps share a run (`pair`):
+// they take its atoms alternately, and only the force pass (about an eighth of the time), which
+// reads and extends the run's virial sums, is handed from one to the other through a pair of
+// mbarriers.  The sums are the ones a single warp forms, in the same order.
 template <typename T, int NRM, int KRM, int NAM, int KAM, bool CL, bool EX>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32)
-nep_eval_kernel(EvalArgs A, long long atoms_per_warp) {
+__global__ void __launch_bounds__((can_pair<T, NRM>() ? 2 : 1) * kRunsPerBlock * 32)
+nep_eval_kernel(EvalArgs A, long long atoms_per_run) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const NepLayout &L = A.L;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -177,6 +201,10 @@ nep_eval_kernel(EvalArgs A, long long atoms_per_warp) {
     // indices into __constant__ memory are served one address at a time
     __shared__ T c3s[24];
     if (threadIdx.x < 24) c3s[threadIdx.x] = C3<T>(threadIdx.x);
+    // turn[run][w]: warp w of the run may start its next force pass
+    __shared__ __align__(8) uint64_t turn[kRunsPerBlock][2];
+    const int pair = can_pair<T, NRM>() ? A.pair : 0, run = pair ? wib >> 1 : wib, wg = pair ? wib & 1 : 0;
+    if (pair && threadIdx.x < 2 * kRunsPerBlock) tc::mbar_init(&turn[threadIdx.x >> 1][threadIdx.x & 1], 1);
     // parameters: c2, c3, q_scaler as packed; per element W0 rows padded to Hp, b0, W1, b1
     {
         const T *gp = reinterpret_cast<const T *>(A.params);
@@ -212,7 +240,8 @@ nep_eval_kernel(EvalArgs A, long long atoms_per_warp) {
               ka_ = EX ? KAM : L.ka;
     const int kpr_ = EX ? (KRM + 3) / 4 * 4 : L.kpr, kpa_ = EX ? (KAM + 3) / 4 * 4 : L.kpa;
     T *stash_g = reinterpret_cast<T *>(Wb + A.o_stash_g);    // [32][NAMP]
-    T *stash_b = reinterpret_cast<T *>(Wb + A.o_stash_b);    // [32][25]
+    T *stash_b = reinterpret_cast<T *>(Wb + A.o_stash_b);    // [32][25], shares its space with
+                                                             // the next five (used after it)
     T *s_sm = reinterpret_cast<T *>(Wb + A.o_s);             // [NAM][24]
     T *dEds = reinterpret_cast<T *>(Wb + A.o_dEds);          // [24][NAMP]
     T *fin = reinterpret_cast<T *>(Wb + A.o_fin);            // [FMp] scaled features
@@ -225,8 +254,7 @@ nep_eval_kernel(EvalArgs A, long long atoms_per_warp) {
     T *av = reinterpret_cast<T *>(Wb + A.o_av);              //   (x, y, z, 1/r)
     T *ag = reinterpret_cast<T *>(Wb + A.o_ag);              //   g_n(r)    [max_a][NAM]
     T *agp = reinterpret_cast<T *>(Wb + A.o_agp);            //   g_n'(r)   [max_a][NAM]
-    for (int q = lane; q < L.fmp; q += 32) fin[q] = T(0);
-    for (int q = lane; q < L.hp; q += 32) dpre[q] = T(0);
+    T *vsh = reinterpret_cast<T *>(smem_raw + A.o_vir) + run * 9 * 32 + lane;
     __syncthreads();
 
     const T *c2 = P + L.off_c2_s, *c3 = P + L.off_c3_s, *qs = P + L.off_qs_s;
@@ -234,9 +262,9 @@ nep_eval_kernel(EvalArgs A, long long atoms_per_warp) {
     const T rc_r = (T)L.rc_r_d, rc_a = (T)L.rc_a_d;
     const T rcinv_r = T(1) / rc_r, rcinv_a = T(1) / rc_a;
 
-    const long long gw = (long long)blockIdx.x * (blockDim.x >> 5) + wib;
-    const long long a_begin = gw * atoms_per_warp;
-    long long a_end = a_begin + atoms_per_warp;
+    const long long gr = (long long)blockIdx.x * (blockDim.x >> (5 + pair)) + run;
+    const long long a_begin = gr * atoms_per_run;
+    long long a_end = a_begin + atoms_per_run;
     if (a_end > A.natoms) a_end = A.natoms;
     if (a_begin >= a_end) return;
     int frame = 0;
@@ -253,21 +281,55 @@ nep_eval_kernel(EvalArgs A, long long atoms_per_warp) {
     T vir[9];
 #pragma unroll
     for (int q = 0; q < 9; ++q) vir[q] = T(0);
+    unsigned phase = 0;
+    bool in_turn = true;
+    // start of atom i's part of the run's virial sums: this warp's turn, the sums of the atoms
+    // before, and their flush when i opens a new frame
+    auto take_virial = [&](long long i) {
+        if (i == a_begin) return;
+        if (pair) {
+            in_turn &= tc::mbar_wait(&turn[run][wg], phase, kTurnPolls);
+            asm volatile("" ::: "memory");
+            phase ^= 1u;
+#pragma unroll
+            for (int q = 0; q < 9; ++q) vir[q] = vsh[32 * q];
+        }
+        if (i == A.frame_start[frame]) {
+            int f = frame;
+            while (f > 0 && A.frame_start[f] > i - 1) --f;
+            flush_virial<T>(A, f, vir, lane);
+        }
+    };
+    auto pass_virial = [&](long long i) {
+        if (i + 1 >= a_end) {
+            flush_virial<T>(A, frame, vir, lane);
+        } else if (pair) {
+#pragma unroll
+            for (int q = 0; q < 9; ++q) vsh[32 * q] = vir[q];
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&turn[run][wg ^ 1]);
+        }
+    };
 
     // the next atom's element and list lengths are loaded while the current atom is processed
-    long long ti_next = A.type_map[a_begin];
-    long long nr_next = L.two ? list_count<CL>(A, true, a_begin) : 0;
-    long long na_next = L.l3 ? list_count<CL>(A, false, a_begin) : 0;
-    for (long long i = a_begin; i < a_end; ++i) {
+    const int step = 1 + pair;
+    long long i = a_begin + wg;
+    long long ti_next = 0, nr_next = 0, na_next = 0;
+    if (i < a_end) {
+        ti_next = A.type_map[i];
+        nr_next = L.two ? list_count<CL>(A, true, i) : 0;
+        na_next = L.l3 ? list_count<CL>(A, false, i) : 0;
+    }
+    for (; i < a_end; i += step) {
         const int ti = (int)ti_next;
         const long long nr_i = nr_next, na_i = na_next;
-        if (i + 1 < a_end) {
-            ti_next = A.type_map[i + 1];
-            if (L.two) nr_next = list_count<CL>(A, true, i + 1);
-            if (L.l3) na_next = list_count<CL>(A, false, i + 1);
+        if (i + step < a_end) {
+            ti_next = A.type_map[i + step];
+            if (L.two) nr_next = list_count<CL>(A, true, i + step);
+            if (L.l3) na_next = list_count<CL>(A, false, i + step);
         }
         while (i >= frame_end && frame + 1 < A.nframes) {
-            if (!A.feats) flush_frame<T>(A, frame, e_frame, vir, lane);
+            if (!A.feats) flush_energy(A, frame, e_frame, lane);
             e_frame = 0.0;
             ++frame;
             frame_end = A.frame_start[frame + 1];
@@ -276,6 +338,10 @@ nep_eval_kernel(EvalArgs A, long long atoms_per_warp) {
             if (lane == 0) {
                 atomicOr(A.err, MATPL_KERR_BAD_TYPE);
                 if (!A.feats) reinterpret_cast<T *>(A.Ei)[i] = T(0);
+            }
+            if (!A.feats) {
+                take_virial(i);
+                pass_virial(i);
             }
             continue;
         }
@@ -408,10 +474,14 @@ nep_eval_kernel(EvalArgs A, long long atoms_per_warp) {
             }
             __syncwarp();
         }
+        // (the harmonics' stash is done with: its space takes the tables below, whose padding the
+        // 16-byte row reads multiply by zero)
         if (lane < 24) {
 #pragma unroll
             for (int n = 0; n < NAM; ++n) s_sm[n * 24 + lane] = sacc[n];
         }
+        if (lane < L.fmp - L.nfeat) fin[L.nfeat + lane] = T(0);
+        if (lane < L.hp - L.hidden) dpre[L.hidden + lane] = T(0);
         if (lane == 0) {
 #pragma unroll
             for (int n = 0; n < NRM; ++n)
@@ -529,6 +599,7 @@ nep_eval_kernel(EvalArgs A, long long atoms_per_warp) {
         __syncwarp();
 
         // ---------------- forces: radial pairs
+        take_virial(i);
         T fi0 = T(0), fi1 = T(0), fi2 = T(0);
         T dqr[NRM];
 #pragma unroll
@@ -602,9 +673,11 @@ nep_eval_kernel(EvalArgs A, long long atoms_per_warp) {
             reinterpret_cast<T *>(A.Ei)[i] = Ei;
             e_frame += (double)Ei;
         }
+        pass_virial(i);
         __syncwarp();
     }
-    if (!A.feats) flush_frame<T>(A, frame, e_frame, vir, lane);
+    if (!A.feats) flush_energy(A, frame, e_frame, lane);
+    if (!in_turn && lane == 0) atomicOr(A.err, MATPL_KERR_TIMEOUT);
 }
 
 __global__ void nep_frame_start(const long long *__restrict__ num_atom, int nframes,
@@ -717,11 +790,15 @@ int launch_eval(const EvalArgs &A0, cudaStream_t s) {
     constexpr int NAMP = (NAM + 3) / 4 * 4;
     A.o_stash_g = take(32 * NAMP * t);
     A.o_stash_b = take(32 * 25 * t);
+    const int after_b = off;
+    off = A.o_stash_b;
     A.o_s = take(NAM * 24 * t);
     A.o_dEds = take(NAMP * 24 * t);
     A.o_fin = take(L.fmp * t);
     A.o_dq = take(L.fmp * t);
     A.o_dpre = take(L.hp * t);
+    const int tables = off - A.o_stash_b;         // s ... dpre
+    off = std::max(off, after_b);
     A.o_rj = take(mr * 4);
     A.o_rv = take((size_t)mr * 4 * t);
     A.o_rgp = take((size_t)mr * NRM * t);
@@ -731,26 +808,41 @@ int launch_eval(const EvalArgs &A0, cudaStream_t s) {
     A.o_agp = take((size_t)ma * NAM * t);
     A.warp_bytes = off;
     A.smem_params = (int)((L.nparams_s * t + 15) / 16 * 16);
-    int wpb = kWarpsPerBlock;
-    while (wpb > 1 && (size_t)A.smem_params + (size_t)wpb * A.warp_bytes > 220 * 1024) --wpb;
-    const size_t smem = (size_t)A.smem_params + (size_t)wpb * A.warp_bytes;
-    MATPL_REQUIRE(smem <= 220 * 1024, MATPL_ERR_UNSUPPORTED,
+    const size_t limit = 220 * 1024;
+    auto smem_of = [&](int warps, size_t warp_bytes) { return (size_t)A.smem_params + warps * warp_bytes; };
+    // Runs of atoms.  The FP32 virial sums run over a run's atoms in order, so where the runs end
+    // fixes their last bits: as many runs per SM as 8-warp blocks with separate stash and tables
+    // fit (two blocks by registers; V of a four-element box, which nearly cancels, moves by 1e-7
+    // with other runs).  FP64 has no such sums to keep; it takes the same rule.
+    const size_t wide = (size_t)A.warp_bytes + std::min(tables, after_b - A.o_stash_b);
+    int rpb = kRunsPerBlock;
+    while (rpb > 1 && smem_of(rpb, wide) > limit) --rpb;
+    MATPL_REQUIRE(smem_of(rpb, wide) <= limit, MATPL_ERR_UNSUPPORTED,
                   "NEP parameters and per-warp lists do not fit in shared memory "
                   "(max_nn_radial / max_nn_angular too large)");
+    const size_t block = (smem_of(rpb, wide) + 24 * t + 127) / 128 * 128 + 1024;
+    const int blocks = t == 4 && rpb == kRunsPerBlock && 2 * block <= 228 * 1024 ? 2 : 1;
+    const long long sms = device_sms();
+    const long long runs = sms * blocks * rpb;
+    const long long apr = (A.natoms + runs - 1) / runs;
+    const long long nruns = (A.natoms + apr - 1) / apr;
+    // two warps per run where a block of them fits and the runs alone leave an SM 8 warps
+    // (100,000 atoms, lists of 80 / 32: 1.08 -> 0.75 ms; 50,000 atoms, compact lists of 104 / 48:
+    // 0.49 -> 0.32 ms)
+    A.o_vir = (int)smem_of(2 * rpb, A.warp_bytes);
+    const size_t smem_pair = A.o_vir + rpb * 9 * 32 * t;
+    A.pair = can_pair<T, NRM>() && blocks == 1 && apr > 1 && !A.feats && smem_pair <= limit + 4 * 1024;
+    // small batches: fewer runs per block, so that every SM gets one
+    if (nruns < sms * rpb) rpb = (int)std::max<long long>(1, (nruns + sms - 1) / sms);
+    const int wpb = rpb << A.pair;
+    const size_t smem = A.pair ? smem_pair : smem_of(wpb, A.warp_bytes);
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
         cudaSuccess)
         return check_launch("cudaFuncSetAttribute(nep_eval)");
-    int dev = 0, sms = device_sms(), per_sm = 1;
-    cudaGetDevice(&dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * wpb, smem);
-    if (per_sm < 1) per_sm = 1;
-    const long long warps = (long long)sms * per_sm * wpb;
-    const long long apw = (A.natoms + warps - 1) / warps;
-    const long long nwarps = (A.natoms + apw - 1) / apw;
-    const int grid = (int)((nwarps + wpb - 1) / wpb);
+    const int grid = (int)((nruns + rpb - 1) / rpb);
     {
         ProfScope ps(A.feats ? "nep_descriptor" : "nep_eval", s);
-        kern<<<grid, 32 * wpb, smem, s>>>(A, apw);
+        kern<<<grid, 32 * wpb, smem, s>>>(A, apr);
     }
     return check_launch("matpl_nep_eval");
 }

@@ -154,6 +154,32 @@ __host__ __device__ inline float sqrt_to_f32(float y, double v) {
     return y;
 }
 
+// sqrt(a) correctly rounded, a >= 0, with five FP64 operations instead of the eleven of the
+// library call: an FP32 root and reciprocal root, two Heron steps g += (a - g^2) h with the exact
+// residual of a fused multiply-add, and a test of the last residual: |a - g^2| < g ulp(g)
+// (1 - 2^-20) holds only if the root lies within half an ulp of g, so g is its rounding.  What
+// fails the test (near a rounding boundary, a power of two, a far from 1) takes the library call.
+__device__ __forceinline__ double sqrt_checked(double a) {
+    const float af = to_f32(a), y = rsqrtf(af), hf = 0.5f * y;
+    float s = af * y;
+    s = fmaf(fmaf(-s, s, af), hf, s);
+    auto widen = [](float f) {                 // exact, normal f > 0, without a conversion
+        const unsigned u = __float_as_uint(f);
+        return __hiloint2double((int)((u >> 3) + 0x38000000u), (int)(u << 29));
+    };
+    const double h = widen(hf);
+    double g = widen(s);
+    g = __fma_rn(__fma_rn(-g, g, a), h, g);
+    g = __fma_rn(__fma_rn(-g, g, a), h, g);
+    const double e = __fma_rn(-g, g, a);
+    const unsigned hg = (unsigned)__double2hiint(g), he = (unsigned)__double2hiint(e) & 0x7fffffffu;
+    const unsigned bound = (hg & 0xfffffu) | ((2u * (hg >> 20) - 1023u - 52u) << 20);
+    const unsigned ha = (unsigned)__double2hiint(a);
+    const bool ok = he < bound - 1u && ((hg & 0xfffffu) | (unsigned)__double2loint(g)) != 0u &&
+                    ha - 0x3c300000u < 0x07800000u;          // 2^-60 <= a < 2^60
+    return ok ? g : __dsqrt_rn(a);
+}
+
 template <typename TO> __device__ __forceinline__ TO conv(double v);
 template <> __device__ __forceinline__ float conv<float>(double v) { return to_f32(v); }
 template <> __device__ __forceinline__ double conv<double>(double v) { return v; }
@@ -161,7 +187,7 @@ template <> __device__ __forceinline__ double conv<double>(double v) { return v;
 // r = sqrt(dd) of a pair, in the output dtype: f64 correctly rounded; f32 the float nearest to
 // that f64 value, formed with four FP64 operations (sqrt_to_f32).
 template <typename TO> __device__ __forceinline__ TO pair_r(double dd);
-template <> __device__ __forceinline__ double pair_r<double>(double dd) { return __dsqrt_rn(dd); }
+template <> __device__ __forceinline__ double pair_r<double>(double dd) { return sqrt_checked(dd); }
 template <> __device__ __forceinline__ float pair_r<float>(double dd) {
     return sqrt_to_f32(sqrtf(to_f32(dd)), dd);
 }

@@ -12,12 +12,16 @@
 //
 // The reference runs one 256-thread block per frame over all N^2 * num_cell^3 candidates.  Here:
 //  * frames whose cell is at least three cut-off widths thick in every direction (num_cell = 1)
-//    go through a cell list: one warp per atom scans the 27 surrounding cells, drops candidates
-//    with an FP32 distance test (margin far above the FP32 error), recomputes every survivor in
-//    FP64 with the reference's operation order and no FMA (__dmul_rn / __dadd_rn), and sorts the
-//    kept pairs by n2 in shared memory (each n2 occurs once: a single image can lie within rc);
+//    go through a cell list: one warp per atom scans the 27 surrounding cells (nine runs of three
+//    cells, whose atoms lie next to each other in the cell-ordered copy), drops candidates with
+//    an FP32 distance test (margin far above the FP32 error), recomputes every survivor in FP64
+//    with the reference's operation order and no FMA (__dmul_rn / __dadd_rn), and sorts the kept
+//    pairs by n2 in shared memory (each n2 occurs once: a single image can lie within rc);
 //  * other frames (small or thin cells) enumerate (n2, image) in the reference's order with one
-//    warp per atom, so warp ballots give the output positions without sorting.
+//    warp per atom, pass them through the same kind of FP32 test into a queue and recompute its
+//    entries in order, so warp ballots give the output positions without sorting.
+// Both forms are bound by the FP64 pipe (two lanes a clock per SM) and by issue, so the tests
+// that keep work off either of them pay.
 // A list that would exceed max_NN is not written past its end: the kernel records
 // MATPL_KERR_NEIGHBOR_OVERFLOW in err_dev and stores the full count in NN.
 #include "common.cuh"
@@ -44,6 +48,8 @@ struct NepFrame {
     double zdelta[3];     // delta of replica (0, 0, 0), with the reference's signed zeros
     float H[9];           // box_orig as float (columns = lattice vectors)
     float Hinv[9];
+    float bf[18];         // box as float
+    float reach;          // mode 1: largest |x| + |y| + |z| the FP32 test may judge
 };
 
 __device__ __forceinline__ double dm(double a, double b) { return __dmul_rn(a, b); }
@@ -103,6 +109,37 @@ __device__ __forceinline__ double exact_pair_ortho(const double *__restrict__ bo
     return da(da(dm(x, x), dm(y, y)), dm(z, z));
 }
 
+// The same for a whole warp of pairs of one atom, D = the six diagonal entries (h^-1, then h).
+// Where no lane meets a zero (a scaled difference or a component of p1) the signs of the other
+// terms and the replica shift, itself a signed zero, cannot show, and where no lane is past half
+// a cell the fold rounds to zero: what is left is 14 FP64 operations.
+__device__ __forceinline__ double warp_pair_ortho(const NepFrame &F, const double *D,
+                                                  const double *p1, bool p1_zero,
+                                                  const double *p2, double &x, double &y,
+                                                  double &z) {
+    auto mag = [](double v) { return ubits(v) << 1; };
+    x = ds(p2[0], p1[0]);
+    y = ds(p2[1], p1[1]);
+    z = ds(p2[2], p1[2]);
+    double sx = dm(D[0], x), sy = dm(D[1], y), sz = dm(D[2], z);
+    const unsigned long long half = 0x3FE0000000000000ull << 1;
+    const bool zero = p1_zero || mag(sx) == 0 || mag(sy) == 0 || mag(sz) == 0;
+    const bool far = mag(sx) > half || mag(sy) > half || mag(sz) > half;
+    if (__any_sync(0xffffffffu, zero || far)) {
+        if (__any_sync(0xffffffffu, zero)) return exact_pair_ortho(F.box, p1, p2, F.zdelta, x, y, z);
+        sx = ds(sx, nearbyint(sx));
+        sy = ds(sy, nearbyint(sy));
+        sz = ds(sz, nearbyint(sz));
+        // a whole number of cells apart in one direction: back to the signed zeros
+        if (__any_sync(0xffffffffu, mag(sx) == 0 || mag(sy) == 0 || mag(sz) == 0))
+            return exact_pair_ortho(F.box, p1, p2, F.zdelta, x, y, z);
+    }
+    x = dm(D[3], sx);
+    y = dm(D[4], sy);
+    z = dm(D[5], sz);
+    return da(da(dm(x, x), dm(y, y)), dm(z, z));
+}
+
 __device__ __forceinline__ void replica_delta(const double *bo, int ia, int ib, int ic,
                                               double *d) {
     const double a = ia, b = ib, c = ic;
@@ -121,101 +158,132 @@ __device__ __forceinline__ int frame_of(const NepFrame *__restrict__ fr, int nfr
     return lo;
 }
 
-__global__ void nepnb_setup(const long long *__restrict__ num_atom,
-                            const double *__restrict__ box, const double *__restrict__ box_orig,
-                            const long long *__restrict__ num_cell, NepFrame *__restrict__ fr,
-                            int nframes, long long natoms, double rc_max, int *__restrict__ err,
-                            const int *gate) {
+// exclusive prefix sum of v over the warp; `total` = the sum
+__device__ __forceinline__ long long warp_excl(long long v, int lane, long long &total) {
+    long long x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const long long y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    total = __shfl_sync(0xffffffffu, x, 31);
+    return x - v;
+}
+
+// Frame table, one block: offsets by warp scans, then one warp per frame with lanes over the
+// entries and lane k < 3 on direction k (one thread per frame walked 21 FP64 divisions and square
+// roots in a row: 14.5 us a call, now 9).
+__global__ void __launch_bounds__(kSetupThreads)
+nepnb_setup(const long long *__restrict__ num_atom, const double *__restrict__ box,
+            const double *__restrict__ box_orig, const long long *__restrict__ num_cell,
+            NepFrame *__restrict__ fr, int nframes, long long natoms, double rc_max,
+            int *__restrict__ err, const int *gate) {
     if (gate && *gate == 0) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     // frame offsets first; counts that overrun natoms are clipped and reported
-    if (threadIdx.x == 0) {
-        long long a0 = 0;
-        for (int f = 0; f < nframes; ++f) {
-            long long n = num_atom[f];
-            if (n < 0 || a0 + n > natoms) {
-                atomicOr(err, MATPL_KERR_BAD_COUNT);
-                n = n < 0 ? 0 : natoms - a0;
+    if (warp == 0) {
+        long long sum = 0;
+        bool bad = false;
+        for (int f0 = 0; f0 < nframes; f0 += 32) {
+            const int f = f0 + lane;
+            const long long want = f < nframes ? num_atom[f] : 0;
+            long long chunk;
+            const long long before = sum + warp_excl(want > 0 ? want : 0, lane, chunk);
+            if (f < nframes) {
+                const long long a0 = before < natoms ? before : natoms;
+                long long n = want > 0 ? want : 0;
+                if (n > natoms - a0) n = natoms - a0;
+                bad |= n != want;
+                fr[f].atom0 = a0;
+                fr[f].n = (int)n;
             }
-            fr[f].atom0 = a0;
-            fr[f].n = (int)n;
-            a0 += n;
+            sum += chunk;
         }
-        if (a0 != natoms) atomicOr(err, MATPL_KERR_BAD_COUNT);
+        bad |= sum != natoms;
+        if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(err, MATPL_KERR_BAD_COUNT);
     }
     __syncthreads();
-    for (int f = threadIdx.x; f < nframes; f += blockDim.x) {
-        NepFrame F;
-        F.atom0 = fr[f].atom0;
-        F.n = fr[f].n;
-        for (int q = 0; q < 18; ++q) F.box[q] = box[18 * f + q];
-        for (int q = 0; q < 9; ++q) F.bo[q] = box_orig[9 * f + q];
-        replica_delta(F.bo, 0, 0, 0, F.zdelta);
-        {
-            const int off[12] = {1, 2, 3, 5, 6, 7, 10, 11, 12, 14, 15, 16};
-            bool o = true;
-            for (int q = 0; q < 12; ++q) o &= F.box[off[q]] == 0.0;
-            F.ortho = o;
+    for (int f = warp; f < nframes; f += nwarps) {
+        NepFrame &F = fr[f];
+        const double *bx = box + 18 * f, *bo = box_orig + 9 * f;
+        if (lane < 18) {
+            const double v = bx[lane];
+            F.box[lane] = v;
+            F.bf[lane] = (float)v;
         }
-        bool single = true;
-        for (int k = 0; k < 3; ++k) {
-            F.rep[k] = (int)num_cell[3 * f + k];
-            single &= F.rep[k] == 1;
-            if (F.rep[k] < 1) atomicOr(err, MATPL_KERR_BAD_BOX);
+        // The FP32 fold of a vector x errs by less than 5e-7 |x| |h| |h^-1| in length and 5e-7 |x|
+        // |h^-1| in a fraction; both stay inside the test's margins (half of 0.02, 1e-3) up to
+        // here.  Atoms further apart (many cells from each other, needle cells) take the exact test.
+        float hi = lane < 18 ? fabsf((float)bx[lane]) : 0.f, hm = lane < 9 ? hi : 0.f;
+        if (lane < 9) hi = 0.f;
+        for (int o = 16; o > 0; o >>= 1) {
+            hm = fmaxf(hm, __shfl_xor_sync(0xffffffffu, hm, o));
+            hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
         }
-        // cell geometry of the original cell: columns of box_orig are the lattice vectors
-        double a[3], b[3], c[3];
-        for (int k = 0; k < 3; ++k) {
-            a[k] = F.bo[3 * k];
-            b[k] = F.bo[3 * k + 1];
-            c[k] = F.bo[3 * k + 2];
+        if (lane == 0) F.reach = fminf(2e4f / (9.f * hm * hi), 2e3f / (3.f * hi));
+        const unsigned off_diag = __ballot_sync(0xffffffffu, lane < 18 && bx[lane < 18 ? lane : 0] != 0.0) &
+                                  0x1DCEEu;        // entries 1 2 3 5 6 7 10 11 12 14 15 16
+        if (lane < 9) {
+            F.bo[lane] = bo[lane];
+            F.H[lane] = (float)bo[lane];
         }
-        double cr[3][3];
-        const double *uv[3][2] = {{b, c}, {c, a}, {a, b}};
-        for (int k = 0; k < 3; ++k) {
-            const double *p = uv[k][0], *q = uv[k][1];
-            cr[k][0] = p[1] * q[2] - p[2] * q[1];
-            cr[k][1] = p[2] * q[0] - p[0] * q[2];
-            cr[k][2] = p[0] * q[1] - p[1] * q[0];
+        const int k = lane < 3 ? lane : 0;
+        const int rep = (int)num_cell[3 * f + k];
+        if (lane < 3) {
+            F.rep[k] = rep;
+            if (rep < 1) atomicOr(err, MATPL_KERR_BAD_BOX);
         }
-        const double det = a[0] * cr[0][0] + a[1] * cr[0][1] + a[2] * cr[0][2];
+        const bool single = __all_sync(0xffffffffu, rep == 1);
+        // cell geometry of the original cell: columns of box_orig are the lattice vectors; lane k
+        // has the cross product of the two others
+        const int u = (k + 1) % 3, v = (k + 2) % 3;
+        const double p[3] = {bo[u], bo[3 + u], bo[6 + u]}, q[3] = {bo[v], bo[3 + v], bo[6 + v]};
+        const double c0 = p[1] * q[2] - p[2] * q[1], c1 = p[2] * q[0] - p[0] * q[2],
+                     c2 = p[0] * q[1] - p[1] * q[0];
+        const double det = __shfl_sync(0xffffffffu, bo[k] * c0 + bo[3 + k] * c1 + bo[6 + k] * c2, 0);
         const double V = fabs(det);
-        // Hinv rows = (b x c, c x a, a x b) / det
-        for (int k = 0; k < 3; ++k)
-            for (int q = 0; q < 3; ++q) {
-                F.Hinv[3 * k + q] = (float)(cr[k][q] / det);
-                F.H[3 * k + q] = (float)F.bo[3 * k + q];
-            }
         const double width = rc_max * 1.00001 + kPrefilterMargin;
-        long long prod = 1;
-        bool thick = V > 0.0;
-        for (int k = 0; k < 3; ++k) {
-            const double area = sqrt(cr[k][0] * cr[k][0] + cr[k][1] * cr[k][1] +
-                                     cr[k][2] * cr[k][2]);
-            const double h = V / area;
-            long long n = (long long)floor(h / width);
-            if (n > 1024) n = 1024;
-            F.nc[k] = (int)(n < 1 ? 1 : n);
+        if (lane < 3) {            // Hinv rows = (b x c, c x a, a x b) / det
+            F.Hinv[3 * k] = (float)(c0 / det);
+            F.Hinv[3 * k + 1] = (float)(c1 / det);
+            F.Hinv[3 * k + 2] = (float)(c2 / det);
         }
+        const double h = V / sqrt(c0 * c0 + c1 * c1 + c2 * c2);
+        long long nk = (long long)floor(h / width);
+        if (nk > 1024) nk = 1024;
+        if (nk < 1) nk = 1;
+        int nc[3];
+        for (int d = 0; d < 3; ++d) nc[d] = __shfl_sync(0xffffffffu, (int)nk, d);
         // at most n + 27 cells per frame (the workspace bound)
+        long long prod = 1;
         for (;;) {
-            prod = (long long)F.nc[0] * F.nc[1] * F.nc[2];
+            prod = (long long)nc[0] * nc[1] * nc[2];
             if (prod <= (long long)F.n + 27) break;
             int kmax = 0;
-            for (int k = 1; k < 3; ++k)
-                if (F.nc[k] > F.nc[kmax]) kmax = k;
-            F.nc[kmax] = (F.nc[kmax] + 1) / 2;
+            for (int d = 1; d < 3; ++d)
+                if (nc[d] > nc[kmax]) kmax = d;
+            nc[kmax] = (nc[kmax] + 1) / 2;
         }
-        for (int k = 0; k < 3; ++k) thick &= F.nc[k] >= 3;
-        F.mode = (single && thick) ? 0 : 1;
-        F.ncells = F.mode == 0 ? (int)prod : 0;
-        fr[f] = F;
+        if (lane == 0) {
+            F.ortho = off_diag == 0u;
+            replica_delta(bo, 0, 0, 0, F.zdelta);
+            bool thick = V > 0.0;
+            for (int d = 0; d < 3; ++d) {
+                F.nc[d] = nc[d];
+                thick &= nc[d] >= 3;
+            }
+            F.mode = (single && thick) ? 0 : 1;
+            F.ncells = F.mode == 0 ? (int)prod : 0;
+        }
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        long long c0 = 0;
-        for (int f = 0; f < nframes; ++f) {
-            fr[f].cell0 = c0;
-            c0 += fr[f].ncells;
+    if (warp == 0) {
+        long long sum = 0, chunk;
+        for (int f0 = 0; f0 < nframes; f0 += 32) {
+            const int f = f0 + lane;
+            const long long before = sum + warp_excl(f < nframes ? fr[f].ncells : 0, lane, chunk);
+            if (f < nframes) fr[f].cell0 = before;
+            sum += chunk;
         }
     }
 }
@@ -294,9 +362,9 @@ __global__ void nepnb_scan(const NepFrame *__restrict__ fr, const int *__restric
 }
 
 __global__ void nepnb_fill(const NepFrame *__restrict__ fr, int nframes, long long natoms,
-                           const int *__restrict__ cell_of, const int *__restrict__ cell_start,
-                           int *__restrict__ cell_fill, int *__restrict__ cell_atoms,
-                           const int *gate) {
+                           const float4 *__restrict__ spos, const int *__restrict__ cell_of,
+                           const int *__restrict__ cell_start, int *__restrict__ cell_fill,
+                           float4 *__restrict__ cell_pos, const int *gate) {
     if (gate && *gate == 0) return;
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < natoms;
          t += (long long)gridDim.x * blockDim.x) {
@@ -304,7 +372,9 @@ __global__ void nepnb_fill(const NepFrame *__restrict__ fr, int nframes, long lo
         if (cell < 0) continue;
         const NepFrame &F = fr[frame_of(fr, nframes, t)];
         const int slot = atomicAdd(cell_fill + F.cell0 + cell, 1);
-        cell_atoms[F.atom0 + cell_start[F.cell0 + cell] + slot] = (int)(t - F.atom0);
+        float4 p = spos[t];                     // cell order: fractional position, atom index
+        p.w = __int_as_float((int)(t - F.atom0));
+        cell_pos[F.atom0 + cell_start[F.cell0 + cell] + slot] = p;
     }
 }
 
@@ -330,7 +400,7 @@ struct SearchArgs {
     const float4 *spos;
     const int *cell_start;
     const int *cell_count;
-    const int *cell_atoms;
+    const float4 *cell_pos;
     const long long *type_map;
     double rc2_r, rc2_a;
     float pre2;              // FP32 pre-filter radius squared
@@ -379,6 +449,19 @@ __device__ __forceinline__ void write_entry(const SearchArgs &A, bool radial, lo
 
 __device__ __forceinline__ void pad_rows(const SearchArgs &A, long long n1, int cr, int ca,
                                          int lane) {
+    if (A.width == 4) {                         // 16-byte rows, as write_entry stores them
+        for (int s = cr + lane; s < A.max_r; s += 32) {
+            double2 *o = reinterpret_cast<double2 *>(A.Ri_r + (n1 * A.max_r + s) * 4);
+            A.NL_r[n1 * A.max_r + s] = -1;
+            o[0] = o[1] = make_double2(0.0, 0.0);
+        }
+        for (int s = ca + lane; s < A.max_a; s += 32) {
+            double2 *o = reinterpret_cast<double2 *>(A.Ri_a + (n1 * A.max_a + s) * 4);
+            A.NL_a[n1 * A.max_a + s] = -1;
+            o[0] = o[1] = make_double2(0.0, 0.0);
+        }
+        return;
+    }
     for (int s = cr + lane; s < A.max_r; s += 32) {
         A.NL_r[n1 * A.max_r + s] = -1;
         for (int q = 0; q < A.width; ++q) A.Ri_r[(n1 * A.max_r + s) * A.width + q] = 0.0;
@@ -408,16 +491,68 @@ __device__ __forceinline__ void count_types(const SearchArgs &A, const WarpLists
 // are appended to the per-warp lists (list mode) or counted.
 template <bool COUNT, bool TYPED>
 __device__ __forceinline__ void drain(const SearchArgs &A, const NepFrame &F, const double *p1,
-                                      int k, int lane, const WarpLists &W, int &cr, int &ca) {
+                                      bool ortho, const double *D, bool p1_zero, int k, int lane,
+                                      const WarpLists &W, int &cr, int &ca) {
+    const unsigned lt = (1u << lane) - 1u;
+    bool in_r = false, in_a = false;
+    long long n2 = -1;
+    double x = 0, y = 0, z = 0, d2 = 0;
+    {
+        n2 = F.atom0 + W.queue[lane < k ? lane : 0];         // idle lanes repeat the first entry
+        const double p2[3] = {A.pos[3 * n2], A.pos[3 * n2 + 1], A.pos[3 * n2 + 2]};
+        d2 = ortho ? warp_pair_ortho(F, D, p1, p1_zero, p2, x, y, z)
+                   : exact_pair(F.box, p1, p2, F.zdelta, x, y, z);
+        in_r = lane < k && ubits(d2) < ubits(A.rc2_r);       // d2 >= +0 or NaN
+        in_a = lane < k && ubits(d2) < ubits(A.rc2_a);
+    }
+    const unsigned br = __ballot_sync(0xffffffffu, in_r);
+    const unsigned ba = __ballot_sync(0xffffffffu, in_a);
+    if (COUNT) {
+        count_types<TYPED>(A, W, n2, in_r, in_a);
+    } else {
+        const double r = (A.width == 4 && (in_r || in_a)) ? sqrt_checked(d2) : 0.0;
+        if (in_r) {
+            const int slot = cr + __popc(br & lt);
+            if (slot < A.max_r) {
+                W.key_r[slot] = (int)(n2 - F.atom0);
+                double2 *v = reinterpret_cast<double2 *>(W.val_r + 4 * slot);
+                v[0] = make_double2(x, y);
+                v[1] = make_double2(z, r);
+            }
+        }
+        if (in_a) {
+            const int slot = ca + __popc(ba & lt);
+            if (slot < A.max_a) {
+                W.key_a[slot] = (int)(n2 - F.atom0);
+                double2 *v = reinterpret_cast<double2 *>(W.val_a + 4 * slot);
+                v[0] = make_double2(x, y);
+                v[1] = make_double2(z, r);
+            }
+        }
+    }
+    cr += __popc(br);
+    ca += __popc(ba);
+}
+
+// The same for queued (atom, image) entries j * images + image of a replicated frame, kept pairs
+// written (or counted) in queue order.
+template <bool COUNT, bool TYPED>
+__device__ __forceinline__ void drain_images(const SearchArgs &A, const NepFrame &F,
+                                             const double *p1, long long n1, const int *queue,
+                                             int k, int lane, const WarpLists &W, int &cr,
+                                             int &ca) {
     const unsigned lt = (1u << lane) - 1u;
     bool in_r = false, in_a = false;
     long long n2 = -1;
     double x = 0, y = 0, z = 0, d2 = 0;
     if (lane < k) {
-        n2 = F.atom0 + W.queue[lane];
+        const int r1 = F.rep[1], r2 = F.rep[2], e = queue[lane];
+        const int ic = e % r2, ib = e / r2 % r1, ji = e / r2 / r1, ia = ji % F.rep[0];
+        n2 = F.atom0 + ji / F.rep[0];
+        double delta[3];
+        replica_delta(F.bo, ia, ib, ic, delta);
         const double p2[3] = {A.pos[3 * n2], A.pos[3 * n2 + 1], A.pos[3 * n2 + 2]};
-        d2 = F.ortho ? exact_pair_ortho(F.box, p1, p2, F.zdelta, x, y, z)
-                     : exact_pair(F.box, p1, p2, F.zdelta, x, y, z);
+        d2 = exact_pair(F.box, p1, p2, delta, x, y, z);
         in_r = d2 < A.rc2_r;
         in_a = d2 < A.rc2_a;
     }
@@ -426,31 +561,46 @@ __device__ __forceinline__ void drain(const SearchArgs &A, const NepFrame &F, co
     if (COUNT) {
         count_types<TYPED>(A, W, n2, in_r, in_a);
     } else {
-        const double r = (A.width == 4 && (in_r || in_a)) ? sqrt(d2) : 0.0;
+        const double r = (A.width == 4 && (in_r || in_a)) ? sqrt_checked(d2) : 0.0;
         if (in_r) {
             const int slot = cr + __popc(br & lt);
-            if (slot < A.max_r) {
-                W.key_r[slot] = (int)(n2 - F.atom0);
-                double *v = W.val_r + 4 * slot;
-                v[0] = x; v[1] = y; v[2] = z; v[3] = r;
-            }
+            if (slot < A.max_r) write_entry(A, true, n1, slot, n2, x, y, z, r);
         }
         if (in_a) {
             const int slot = ca + __popc(ba & lt);
-            if (slot < A.max_a) {
-                W.key_a[slot] = (int)(n2 - F.atom0);
-                double *v = W.val_a + 4 * slot;
-                v[0] = x; v[1] = y; v[2] = z; v[3] = r;
-            }
+            if (slot < A.max_a) write_entry(A, false, n1, slot, n2, x, y, z, r);
         }
     }
     cr += __popc(br);
     ca += __popc(ba);
 }
 
+// Appends the lanes' passing entries to the queue; returns true once it holds 32 to be drained.
+__device__ __forceinline__ bool enqueue(int *queue, int &qn, bool pass, int v, int lane) {
+    const unsigned b = __ballot_sync(0xffffffffu, pass);
+    if (pass) queue[qn + __popc(b & ((1u << lane) - 1u))] = v;
+    qn += __popc(b);
+    if (qn < 32) return false;
+    __syncwarp();
+    return true;
+}
+// Drops the 32 drained entries.
+__device__ __forceinline__ void dequeue32(int *queue, int &qn, int lane) {
+    qn -= 32;
+    const int v = lane < qn ? queue[32 + lane] : 0;
+    __syncwarp();
+    if (lane < qn) queue[lane] = v;
+    __syncwarp();
+}
+
 // COUNT: only count neighbors (calculate_maxneigh); TYPED: counts per neighbor element.
+// Bound by the FP64 pipe (70 % active) and issue.  The cell-ordered FP32 positions are read in runs
+// (no index, no gather), the exact test skips the orthorhombic zeros, and the root takes five FP64
+// operations: 575 -> 454 us for 100,000 atoms in one frame, and 62 -> 30 us for 6 x 72 replicated
+// atoms (FP32 test ahead of the exact one, one warp per block so that every SM has some).  Six blocks
+// an SM: seven and eight spill, 459 and 458 us.
 template <bool COUNT, bool TYPED>
-__global__ void __launch_bounds__(128) nepnb_search(SearchArgs A, int warps_per_block) {
+__global__ void __launch_bounds__(128, 6) nepnb_search(SearchArgs A, int warps_per_block) {
     if (A.gate && *A.gate == 0) return;
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -494,143 +644,191 @@ __global__ void __launch_bounds__(128) nepnb_search(SearchArgs A, int warps_per_
             float H[9];
 #pragma unroll
             for (int q = 0; q < 9; ++q) H[q] = F.H[q];
-            // the 27 neighbor cells, one per lane: start, count and periodic shift, read in
-            // parallel; the candidates of all cells are then walked as one flat range, 32 at a
-            // time (the kept pairs are rank-sorted by n2 afterwards, so the order of the walk
-            // does not matter)
-            int cbeg = 0, ccnt = 0, csh = 0;
-            if (lane < 27) {
-                const int d[3] = {lane / 9 - 1, (lane / 3) % 3 - 1, lane % 3 - 1};
-                int c[3], sh[3];
-                for (int k = 0; k < 3; ++k) {
-                    c[k] = c1[k] + d[k];
-                    sh[k] = 0;
-                    if (c[k] < 0) { c[k] += F.nc[k]; sh[k] = -1; }
-                    if (c[k] >= F.nc[k]) { c[k] -= F.nc[k]; sh[k] = 1; }
+            // the 27 neighbor cells as 9 columns of three z-neighbors: lane 2 col + part holds
+            // the column's run of atoms inside the cell (part 0) or the wrapped end (part 1) and
+            // the atom's position seen from it
+            int rbeg = 0, rlen = 0;
+            float ox = 0.f, oy = 0.f, oz = 0.f;
+            if (lane < 18) {
+                const int col = lane >> 1, part = lane & 1;
+                int cx = c1[0] + col / 3 - 1, cy = c1[1] + col % 3 - 1, shx = 0, shy = 0, shz = 0;
+                if (cx < 0) { cx += F.nc[0]; shx = -1; }
+                if (cx >= F.nc[0]) { cx -= F.nc[0]; shx = 1; }
+                if (cy < 0) { cy += F.nc[1]; shy = -1; }
+                if (cy >= F.nc[1]) { cy -= F.nc[1]; shy = 1; }
+                int z0 = max(c1[2] - 1, 0), z1 = min(c1[2] + 1, F.nc[2] - 1);
+                if (part) {
+                    z0 = 1; z1 = 0;
+                    if (c1[2] == 0) { z0 = z1 = F.nc[2] - 1; shz = -1; }
+                    else if (c1[2] == F.nc[2] - 1) { z0 = z1 = 0; shz = 1; }
                 }
-                const long long cell = F.cell0 + (c[0] * F.nc[1] + c[1]) * F.nc[2] + c[2];
-                cbeg = A.cell_start[cell];
-                ccnt = A.cell_count[cell];
-                csh = (sh[0] + 1) | ((sh[1] + 1) << 2) | ((sh[2] + 1) << 4);
+                if (z0 <= z1) {
+                    const long long row = F.cell0 + ((long long)cx * F.nc[1] + cy) * F.nc[2];
+                    rbeg = A.cell_start[row + z0];
+                    rlen = A.cell_start[row + z1] + A.cell_count[row + z1] - rbeg;
+                }
+                ox = s1.x - (float)shx;
+                oy = s1.y - (float)shy;
+                oz = s1.z - (float)shz;
             }
-            int incl = ccnt;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += y;
-            }
-            const int excl = incl - ccnt;
-            const int total = __shfl_sync(0xffffffffu, incl, 31);
+            const int self = (int)(n1 - F.atom0);
+            const bool ortho = F.ortho, p1_zero = p1[0] == 0.0 || p1[1] == 0.0 || p1[2] == 0.0;
+            const double D[6] = {F.box[9], F.box[13], F.box[17], F.box[0], F.box[4], F.box[8]};
+            const float4 *cell_pos = A.cell_pos + F.atom0;
             int qn = 0;
-            for (int base = 0; base < total; base += 32) {
-                const int e = base + lane;
-                // the last cell q with excl_q <= e (it holds e: cells with no atoms share
-                // their start with the next one)
-                int lo = 0, hi = 26;
-#pragma unroll
-                for (int it = 0; it < 5; ++it) {
-                    const int mid = (lo + hi + 1) >> 1;
-                    const int em = __shfl_sync(0xffffffffu, excl, mid);
-                    if (em <= e) lo = mid; else hi = mid - 1;
-                }
-                const int q = lo;
-                const int qbeg = __shfl_sync(0xffffffffu, cbeg, q);
-                const int qex = __shfl_sync(0xffffffffu, excl, q);
-                const int qsh = __shfl_sync(0xffffffffu, csh, q);
-                bool pass = false;
-                int loc = -1;
-                if (e < total) {
-                    loc = A.cell_atoms[F.atom0 + qbeg + (e - qex)];
-                    if (F.atom0 + loc != n1) {
-                        const float4 s2 = A.spos[F.atom0 + loc];
-                        const float f0 = s2.x + (float)((qsh & 3) - 1) - s1.x,
-                                    f1 = s2.y + (float)(((qsh >> 2) & 3) - 1) - s1.y,
-                                    f2 = s2.z + (float)(((qsh >> 4) & 3) - 1) - s1.z;
+            for (unsigned runs = __ballot_sync(0xffffffffu, rlen > 0); runs; runs &= runs - 1) {
+                const int q = __ffs(runs) - 1;
+                const int len = __shfl_sync(0xffffffffu, rlen, q);
+                const float4 *cp = cell_pos + __shfl_sync(0xffffffffu, rbeg, q);
+                const float qx = __shfl_sync(0xffffffffu, ox, q), qy = __shfl_sync(0xffffffffu, oy, q),
+                            qz = __shfl_sync(0xffffffffu, oz, q);
+                for (int base = 0; base < len; base += 32) {
+                    const int e = base + lane;
+                    bool pass = false;
+                    int loc = 0;
+                    if (e < len) {
+                        const float4 s2 = cp[e];
+                        loc = __float_as_int(s2.w);
+                        const float f0 = s2.x - qx, f1 = s2.y - qy, f2 = s2.z - qz;
                         const float xf = H[0] * f0 + H[1] * f1 + H[2] * f2;
                         const float yf = H[3] * f0 + H[4] * f1 + H[5] * f2;
                         const float zf = H[6] * f0 + H[7] * f1 + H[8] * f2;
-                        pass = xf * xf + yf * yf + zf * zf < A.pre2;
+                        pass = xf * xf + yf * yf + zf * zf < A.pre2 && loc != self;
                     }
-                }
-                const unsigned b = __ballot_sync(0xffffffffu, pass);
-                if (pass) W.queue[qn + __popc(b & lt)] = loc;
-                qn += __popc(b);
-                if (qn >= 32) {
-                    __syncwarp();
-                    drain<COUNT, TYPED>(A, F, p1, 32, lane, W, cr, ca);
-                    const int left = qn - 32;
-                    const int v = lane < left ? W.queue[32 + lane] : 0;
-                    __syncwarp();
-                    if (lane < left) W.queue[lane] = v;
-                    __syncwarp();
-                    qn = left;
+                    if (enqueue(W.queue, qn, pass, loc, lane)) {
+                        drain<COUNT, TYPED>(A, F, p1, ortho, D, p1_zero, 32, lane, W, cr, ca);
+                        dequeue32(W.queue, qn, lane);
+                    }
                 }
             }
             if (qn > 0) {
                 __syncwarp();
-                drain<COUNT, TYPED>(A, F, p1, qn, lane, W, cr, ca);
+                drain<COUNT, TYPED>(A, F, p1, ortho, D, p1_zero, qn, lane, W, cr, ca);
             }
             if (!COUNT) {
                 __syncwarp();
-                // rank sort by n2 (keys are distinct) and store in order
+                // rank sort by n2 (keys are distinct) and store in order; keys are read four at a
+                // time where their row is 16-byte aligned
                 for (int pass = 0; pass < 2; ++pass) {
                     const bool radial = pass == 0;
                     const int n = min(radial ? cr : ca, radial ? A.max_r : A.max_a);
                     const int *key = radial ? W.key_r : W.key_a;
                     const double *val = radial ? W.val_r : W.val_a;
+                    const int n4 = radial || A.max_r % 4 == 0 ? n & ~3 : 0;
                     for (int e = lane; e < n; e += 32) {
                         const int k = key[e];
                         int rank = 0;
-                        for (int o = 0; o < n; ++o) rank += key[o] < k;
-                        const double *v = val + 4 * e;
-                        write_entry(A, radial, n1, rank, F.atom0 + k, v[0], v[1], v[2], v[3]);
+                        for (int o = 0; o < n4; o += 4) {
+                            const int4 k4 = *reinterpret_cast<const int4 *>(key + o);
+                            rank += (k4.x < k) + (k4.y < k) + (k4.z < k) + (k4.w < k);
+                        }
+                        for (int o = n4; o < n; ++o) rank += key[o] < k;
+                        const double2 *v = reinterpret_cast<const double2 *>(val + 4 * e);
+                        const double2 v0 = v[0], v1 = v[1];
+                        write_entry(A, radial, n1, rank, F.atom0 + k, v0.x, v0.y, v1.x, v1.y);
                     }
                 }
                 __syncwarp();
             }
         } else {
-            // enumerate (n2, image) in the reference's order; ballots keep that order
-            const int nimg = F.rep[0] * F.rep[1] * F.rep[2];
-            const long long total = (long long)F.n * nimg;
-            const long long self = n1 - F.atom0;
-            for (long long base = 0; base < total; base += 32) {
-                const long long qq = base + lane;
-                bool in_r = false, in_a = false;
-                long long n2 = -1;
-                double x = 0, y = 0, z = 0, d2 = 0;
-                if (qq < total) {
-                    const long long j = qq / nimg;
-                    const int im = (int)(qq - j * nimg);
-                    const int ia = im / (F.rep[1] * F.rep[2]);
-                    const int ib = (im / F.rep[2]) % F.rep[1];
-                    const int ic = im % F.rep[2];
-                    if (!(im == 0 && j == self)) {
-                        n2 = F.atom0 + j;
-                        double delta[3];
-                        replica_delta(F.bo, ia, ib, ic, delta);
-                        const double p2[3] = {A.pos[3 * n2], A.pos[3 * n2 + 1], A.pos[3 * n2 + 2]};
-                        d2 = exact_pair(F.box, p1, p2, delta, x, y, z);
-                        in_r = d2 < A.rc2_r;
-                        in_a = d2 < A.rc2_a;
+            // enumerate (n2, image) in the reference's order: an FP32 test, then the queue in
+            // order.  An entry near the fold's tie goes to the exact test whatever its length.
+            const int r0 = F.rep[0], r1 = F.rep[1], r2 = F.rep[2];
+            const long long nimg = (long long)r0 * r1 * r2;
+            const long long total = r0 > 0 && r1 > 0 && r2 > 0 ? F.n * nimg : 0;
+            const int self = (int)(n1 - F.atom0);
+            if (total < (1LL << 31)) {
+                float B[18], H[9];
+#pragma unroll
+                for (int q = 0; q < 18; ++q) B[q] = F.bf[q];
+#pragma unroll
+                for (int q = 0; q < 9; ++q) H[q] = F.H[q];
+                const float reach = F.reach;
+                // entry (j, ia, ib, ic) in mixed radix, advanced by 32 without divisions
+                const int s2 = 32 % max(r2, 1), t2 = 32 / max(r2, 1), s1 = t2 % max(r1, 1),
+                          t1 = t2 / max(r1, 1), s0 = t1 % max(r0, 1), sj = t1 / max(r0, 1);
+                int ic = lane % max(r2, 1), ib = lane / max(r2, 1), ia = ib / max(r1, 1);
+                ib %= max(r1, 1);
+                int j = ia / max(r0, 1);
+                ia %= max(r0, 1);
+                int qn = 0;
+                for (long long base = 0; base < total; base += 32) {
+                    bool pass = false;
+                    if (base + lane < total && !(j == self && (ia | ib | ic) == 0)) {
+                        const double *p2 = A.pos + 3 * (F.atom0 + j);
+                        const float x0 = to_f32(ds(p2[0], p1[0])), y0 = to_f32(ds(p2[1], p1[1])),
+                                    z0 = to_f32(ds(p2[2], p1[2]));
+                        const float x = x0 + (H[0] * ia + H[1] * ib + H[2] * ic);
+                        const float y = y0 + (H[3] * ia + H[4] * ib + H[5] * ic);
+                        const float z = z0 + (H[6] * ia + H[7] * ib + H[8] * ic);
+                        float u = B[9] * x + B[10] * y + B[11] * z;
+                        float v = B[12] * x + B[13] * y + B[14] * z;
+                        float w = B[15] * x + B[16] * y + B[17] * z;
+                        u -= rintf(u);
+                        v -= rintf(v);
+                        w -= rintf(w);
+                        const float far = fmaxf(fabsf(u), fmaxf(fabsf(v), fabsf(w)));
+                        const float xf = B[0] * u + B[1] * v + B[2] * w;
+                        const float yf = B[3] * u + B[4] * v + B[5] * w;
+                        const float zf = B[6] * u + B[7] * v + B[8] * w;
+                        pass = far > 0.499f || !(fabsf(x) + fabsf(y) + fabsf(z) <= reach) ||
+                               !(xf * xf + yf * yf + zf * zf >= A.pre2);
+                    }
+                    const int e = (int)(base + lane);
+                    ic += s2;
+                    if (ic >= r2) { ic -= r2; ++ib; }
+                    ib += s1;
+                    if (ib >= r1) { ib -= r1; ++ia; }
+                    ia += s0;
+                    if (ia >= r0) { ia -= r0; ++j; }
+                    j += sj;
+                    if (enqueue(W.queue, qn, pass, e, lane)) {
+                        drain_images<COUNT, TYPED>(A, F, p1, n1, W.queue, 32, lane, W, cr, ca);
+                        dequeue32(W.queue, qn, lane);
                     }
                 }
-                const unsigned br = __ballot_sync(0xffffffffu, in_r);
-                const unsigned ba = __ballot_sync(0xffffffffu, in_a);
-                if (COUNT) {
-                    count_types<TYPED>(A, W, n2, in_r, in_a);
-                } else {
-                    const double r = (A.width == 4 && (in_r || in_a)) ? sqrt(d2) : 0.0;
-                    if (in_r) {
-                        const int slot = cr + __popc(br & lt);
-                        if (slot < A.max_r) write_entry(A, true, n1, slot, n2, x, y, z, r);
-                    }
-                    if (in_a) {
-                        const int slot = ca + __popc(ba & lt);
-                        if (slot < A.max_a) write_entry(A, false, n1, slot, n2, x, y, z, r);
-                    }
+                if (qn > 0) {
+                    __syncwarp();
+                    drain_images<COUNT, TYPED>(A, F, p1, n1, W.queue, qn, lane, W, cr, ca);
                 }
-                cr += __popc(br);
-                ca += __popc(ba);
+                __syncwarp();
+            } else {
+                for (long long base = 0; base < total; base += 32) {
+                    const long long qq = base + lane;
+                    bool in_r = false, in_a = false;
+                    long long n2 = -1;
+                    double x = 0, y = 0, z = 0, d2 = 0;
+                    if (qq < total) {
+                        const long long j = qq / nimg;
+                        const int im = (int)(qq - j * nimg);
+                        if (!(im == 0 && j == self)) {
+                            n2 = F.atom0 + j;
+                            double delta[3];
+                            replica_delta(F.bo, im / (r1 * r2), im / r2 % r1, im % r2, delta);
+                            const double p2[3] = {A.pos[3 * n2], A.pos[3 * n2 + 1], A.pos[3 * n2 + 2]};
+                            d2 = exact_pair(F.box, p1, p2, delta, x, y, z);
+                            in_r = d2 < A.rc2_r;
+                            in_a = d2 < A.rc2_a;
+                        }
+                    }
+                    const unsigned br = __ballot_sync(0xffffffffu, in_r);
+                    const unsigned ba = __ballot_sync(0xffffffffu, in_a);
+                    if (COUNT) {
+                        count_types<TYPED>(A, W, n2, in_r, in_a);
+                    } else {
+                        const double r = (A.width == 4 && (in_r || in_a)) ? sqrt_checked(d2) : 0.0;
+                        if (in_r) {
+                            const int slot = cr + __popc(br & lt);
+                            if (slot < A.max_r) write_entry(A, true, n1, slot, n2, x, y, z, r);
+                        }
+                        if (in_a) {
+                            const int slot = ca + __popc(ba & lt);
+                            if (slot < A.max_a) write_entry(A, false, n1, slot, n2, x, y, z, r);
+                        }
+                    }
+                    cr += __popc(br);
+                    ca += __popc(ba);
+                }
             }
         }
         if (COUNT) {
@@ -728,7 +926,8 @@ __global__ void nepnb_skin_frac(const double *__restrict__ pos, const NepFrame *
 constexpr int kFilterWarps = 8;
 
 // Exact FP64 test of the first k (<= 32) queued skin entries, written in queue order.
-__device__ __forceinline__ void skin_drain(const NepFrame &F, const double *__restrict__ pos,
+__device__ __forceinline__ void skin_drain(const NepFrame &F, bool ortho, const double *D,
+                                           bool p1_zero, const double *__restrict__ pos,
                                            const double *p1, const int *queue, int k, int lane,
                                            long long n1, double rc2_r, double rc2_a, int max_r,
                                            int max_a, int width, long long *__restrict__ NL_r,
@@ -739,17 +938,17 @@ __device__ __forceinline__ void skin_drain(const NepFrame &F, const double *__re
     bool in_r = false, in_a = false;
     long long n2 = -1;
     double x = 0, y = 0, z = 0, d2 = 0;
-    if (lane < k) {
-        n2 = queue[lane];
+    {
+        n2 = queue[lane < k ? lane : 0];                     // idle lanes repeat the first entry
         const double p2[3] = {pos[3 * n2], pos[3 * n2 + 1], pos[3 * n2 + 2]};
-        d2 = F.ortho ? exact_pair_ortho(F.box, p1, p2, F.zdelta, x, y, z)
-                     : exact_pair(F.box, p1, p2, F.zdelta, x, y, z);
-        in_r = d2 < rc2_r;
-        in_a = d2 < rc2_a;
+        d2 = ortho ? warp_pair_ortho(F, D, p1, p1_zero, p2, x, y, z)
+                   : exact_pair(F.box, p1, p2, F.zdelta, x, y, z);
+        in_r = lane < k && ubits(d2) < ubits(rc2_r);         // d2 >= +0 or NaN
+        in_a = lane < k && ubits(d2) < ubits(rc2_a);
     }
     const unsigned br = __ballot_sync(0xffffffffu, in_r);
     const unsigned ba = __ballot_sync(0xffffffffu, in_a);
-    const double r = (width == 4 && (in_r || in_a)) ? sqrt(d2) : 0.0;
+    const double r = (width == 4 && (in_r || in_a)) ? sqrt_checked(d2) : 0.0;
     for (int pass = 0; pass < 2; ++pass) {
         const bool radial = pass == 0;
         if (!(radial ? in_r : in_a)) continue;
@@ -790,6 +989,8 @@ nepnb_skin_filter(const NepFrame *__restrict__ fr, int nframes, long long natoms
          n1 += nw) {
         const NepFrame &F = fr[frame_of(fr, nframes, n1)];
         const double p1[3] = {pos[3 * n1], pos[3 * n1 + 1], pos[3 * n1 + 2]};
+        const bool ortho = F.ortho, p1_zero = p1[0] == 0.0 || p1[1] == 0.0 || p1[2] == 0.0;
+        const double D[6] = {F.box[9], F.box[13], F.box[17], F.box[0], F.box[4], F.box[8]};
         const float4 s1 = spos[n1];
         float H[9];
 #pragma unroll
@@ -821,8 +1022,8 @@ nepnb_skin_filter(const NepFrame *__restrict__ fr, int nframes, long long natoms
             qn += __popc(b);
             if (qn >= 32) {
                 __syncwarp();
-                skin_drain(F, pos, p1, queue, 32, lane, n1, rc2_r, rc2_a, max_r, max_a, width,
-                           NL_r, NL_a, Ri_r, Ri_a, cr, ca);
+                skin_drain(F, ortho, D, p1_zero, pos, p1, queue, 32, lane, n1, rc2_r, rc2_a, max_r,
+                           max_a, width, NL_r, NL_a, Ri_r, Ri_a, cr, ca);
                 const int left = qn - 32;
                 const int v = lane < left ? queue[32 + lane] : 0;
                 __syncwarp();
@@ -833,8 +1034,8 @@ nepnb_skin_filter(const NepFrame *__restrict__ fr, int nframes, long long natoms
         }
         if (qn > 0) {
             __syncwarp();
-            skin_drain(F, pos, p1, queue, qn, lane, n1, rc2_r, rc2_a, max_r, max_a, width, NL_r,
-                       NL_a, Ri_r, Ri_a, cr, ca);
+            skin_drain(F, ortho, D, p1_zero, pos, p1, queue, qn, lane, n1, rc2_r, rc2_a, max_r, max_a,
+                       width, NL_r, NL_a, Ri_r, Ri_a, cr, ca);
         }
         __syncwarp();
         for (int s = min(cr, max_r) + lane; s < max_r; s += 32) {
@@ -920,7 +1121,8 @@ nepnb_skin_filter_compact(long long natoms, const int *__restrict__ skin,
 struct Workspace {
     NepFrame *fr;
     float4 *spos;
-    int *cell_of, *cell_count, *cell_start, *cell_fill, *cell_atoms;
+    float4 *cell_pos;
+    int *cell_of, *cell_count, *cell_start, *cell_fill;
 };
 
 size_t workspace_layout(int nframes, long long natoms, unsigned char *base, Workspace *w) {
@@ -935,7 +1137,7 @@ size_t workspace_layout(int nframes, long long natoms, unsigned char *base, Work
     tmp.fr = (NepFrame *)take(sizeof(NepFrame) * (size_t)nframes);
     tmp.spos = (float4 *)take(sizeof(float4) * (size_t)natoms);
     tmp.cell_of = (int *)take(sizeof(int) * (size_t)natoms);
-    tmp.cell_atoms = (int *)take(sizeof(int) * (size_t)natoms);
+    tmp.cell_pos = (float4 *)take(sizeof(float4) * (size_t)natoms);
     tmp.cell_count = (int *)take(sizeof(int) * (size_t)cells);
     tmp.cell_fill = (int *)take(sizeof(int) * (size_t)cells);
     tmp.cell_start = (int *)take(sizeof(int) * (size_t)cells);
@@ -984,11 +1186,11 @@ int run(int nframes, long long natoms, const long long *num_atom, const long lon
     nepnb_bin<<<g1, 256, 0, s>>>(pos, w.fr, nframes, natoms, w.spos, w.cell_of, w.cell_count,
                                  nullptr, nullptr, nullptr);
     nepnb_scan<<<nframes, 1024, 0, s>>>(w.fr, w.cell_count, w.cell_start, nullptr);
-    nepnb_fill<<<g1, 256, 0, s>>>(w.fr, nframes, natoms, w.cell_of, w.cell_start, w.cell_fill,
-                                  w.cell_atoms, nullptr);
+    nepnb_fill<<<g1, 256, 0, s>>>(w.fr, nframes, natoms, w.spos, w.cell_of, w.cell_start,
+                                  w.cell_fill, w.cell_pos, nullptr);
     SearchArgs A;
     A.fr = w.fr; A.nframes = nframes; A.natoms = natoms; A.pos = pos; A.spos = w.spos;
-    A.cell_start = w.cell_start; A.cell_count = w.cell_count; A.cell_atoms = w.cell_atoms;
+    A.cell_start = w.cell_start; A.cell_count = w.cell_count; A.cell_pos = w.cell_pos;
     A.type_map = type_map; A.rc2_r = rc_r * rc_r; A.rc2_a = rc_a * rc_a;
     const float pre = (float)(rc_max * 1.00001) + kPrefilterMargin;
     A.pre2 = pre * pre;
@@ -999,6 +1201,8 @@ int run(int nframes, long long natoms, const long long *num_atom, const long lon
     const size_t per_warp = warp_scratch(count_only, typed, max_r, max_a, ntypes);
     int wpb = 4;
     while (wpb > 1 && per_warp * wpb > 96 * 1024) wpb >>= 1;
+    // small batches: one-warp blocks, so that every SM gets its share of the FP64 work
+    if (natoms < 16LL * device_sms()) wpb = 1;
     const size_t smem = align_up(per_warp * wpb, 16);
     const int grid = blocks_for(natoms, wpb, device_sms() * 64);
     if (count_only) {
@@ -1053,11 +1257,11 @@ int run_skin_update(int nframes, long long natoms, const long long *num_atom, co
     nepnb_bin<<<g1, 256, 0, s>>>(pos, w.fr, nframes, natoms, w.spos, w.cell_of, w.cell_count,
                                  gate, x_ref, delta);
     nepnb_scan<<<nframes, 1024, 0, s>>>(w.fr, w.cell_count, w.cell_start, gate);
-    nepnb_fill<<<g1, 256, 0, s>>>(w.fr, nframes, natoms, w.cell_of, w.cell_start, w.cell_fill,
-                                  w.cell_atoms, gate);
+    nepnb_fill<<<g1, 256, 0, s>>>(w.fr, nframes, natoms, w.spos, w.cell_of, w.cell_start,
+                                  w.cell_fill, w.cell_pos, gate);
     SearchArgs A;
     A.fr = w.fr; A.nframes = nframes; A.natoms = natoms; A.pos = pos; A.spos = w.spos;
-    A.cell_start = w.cell_start; A.cell_count = w.cell_count; A.cell_atoms = w.cell_atoms;
+    A.cell_start = w.cell_start; A.cell_count = w.cell_count; A.cell_pos = w.cell_pos;
     A.type_map = nullptr; A.rc2_r = r_list * r_list; A.rc2_a = 0.0;
     const float pre = (float)(r_list * 1.00001) + kPrefilterMargin;
     A.pre2 = pre * pre;

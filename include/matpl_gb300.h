@@ -492,7 +492,7 @@ int matpl_env_stats(int batch, int natoms, int nslots, int ntypes, const int32_t
  * mode 0 (forward):  q [N, ldQ] = the part's features (radial n_max; angular n_max per
  *                    l = 1..l_max_3b, then the 4-body and 5-body blocks).
  * mode 1 (backward): for G [N, ldG] = dL/dq writes grad_d12 [N, max_nn, 4] = G . dq/dd12
- *                    (partials in the four columns; caller zero-fills) and W, zero-filled by
+ *                    (partials in the four columns; written whole, 0 in empty slots) and W, zero-filled by
  *                    the caller: radial [N, T, n_base] = sum over neighbors of type t of
  *                    f_k(r) (dL/dc[t_i, t, n, k] = sum_i G[i, n] W[i, t, k]); angular
  *                    [N, T, n_max, n_base] (dL/dc[t_i] = sum_i W[i]).  Either output may be
@@ -509,6 +509,20 @@ int matpl_nep_feat_op(int dtype, int part, int mode, int natoms, int max_nn, int
                       const long long *type_map, const void *G, long long ldG, const void *H,
                       void *q, long long ldQ, void *grad_d12, void *W, int *err_dev,
                       void *stream);
+
+/* matpl_nep_feat_grad: mode 1 or 2 of matpl_nep_feat_op together with the coefficient gradient dc
+ *   [ntypes, ntypes, n_max, n_base] (zeroed, then accumulated) in place of W; grad_d12 (mode 1) may
+ *   be NULL, gso [N, ldQ] belongs to mode 2.  The workspace has the stated size: FP64 sums of dc
+ *   where a block's share fits in shared memory, W otherwise.
+ *   As with matpl_nep_cgrad the last bits of dc may differ between runs. */
+size_t matpl_nep_feat_grad_workspace_bytes(int dtype, int part, int natoms, int ntypes, int n_max,
+                                           int n_base);
+int matpl_nep_feat_grad(int dtype, int part, int mode, int natoms, int max_nn, int ntypes,
+                        int n_max, int n_base, int l_max_3b, int l_max_4b, int l_max_5b,
+                        double cutoff, const void *coeff, const void *d12, const long long *NL,
+                        const long long *type_map, const void *G, long long ldG, const void *H,
+                        void *gso, long long ldQ, void *grad_d12, void *dc, void *workspace,
+                        size_t workspace_bytes, int *err_dev, void *stream);
 
 /* matpl_nep_cgrad: the coefficient gradient dL/dc [ntypes, ntypes, n_max, n_base] (zeroed,
  *   then accumulated) from the per-atom table W of matpl_nep_feat_op's backward modes, summed

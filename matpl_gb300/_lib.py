@@ -104,6 +104,9 @@ SIGNATURES = {
                                   _vp, _i, _vp, _vp, _vp, _vp, _vp, _sz, _vp]),
     "matpl_env_stats": (_i, [_i, _i, _i, _i, _vp, _vp, _vp, _d, _d, _vp, _vp, _vp]),
     "matpl_nep_feat_op": (_i, [_i] * 11 + [_d] + [_vp] * 5 + [_ll, _vp, _vp, _ll] + [_vp] * 4),
+    "matpl_nep_feat_grad_workspace_bytes": (_sz, [_i] * 6),
+    "matpl_nep_feat_grad": (_i, [_i] * 11 + [_d] + [_vp] * 5 + [_ll, _vp, _vp, _ll] + [_vp] * 3 +
+                            [_sz, _vp, _vp]),
     "matpl_nep_cgrad": (_i, [_i] * 6 + [_vp, _vp, _ll, _vp, _vp, _vp, _vp]),
     "matpl_dp_desc_dual": (_i, [_i, _ll, _i] + [_vp] * 6),
     "matpl_dp_desc_dual_grad": (_i, [_i, _ll, _i] + [_vp] * 8),

@@ -28,6 +28,7 @@ namespace matpl {
 namespace {
 
 constexpr int kFeatWarps = 4;
+constexpr size_t kTableBytes = 16 * 1024;   // see matpl_nep_feat_grad_workspace_bytes
 enum { kFwd = 0, kBwd = 1, kBwd2 = 2 };
 
 struct FeatArgs {
@@ -42,8 +43,12 @@ struct FeatArgs {
     const void *H;              // [N, nn, 4] (BWD2)
     void *q;                    // [N, ldQ] (FWD) or gso (BWD2)
     long long ldQ;
-    void *grad_d12;             // [N, nn, 4] (BWD), zero-filled by the caller
+    void *grad_d12;             // [N, nn, 4] (BWD), written whole
     void *W;                    // partial c-gradient per atom, zero-filled by the caller
+    void *dc;                   // or the c-gradient [T, T, nmax, nbase] itself
+    double *sum;                // and its FP64 sums over the blocks, followed by the count of blocks
+                                // that have added theirs (zero-filled)
+    bool vec;                   // d12, H, grad_d12 on 16-byte boundaries
     int l3, four, five;         // angular: l_max of the 3-body part, 4-/5-body present
     int *err;
 };
@@ -51,23 +56,93 @@ struct FeatArgs {
 template <typename T>
 __device__ __forceinline__ T ld(const void *p, long long k) { return static_cast<const T *>(p)[k]; }
 
+// the four values of slot ps of a [N, nn, 4] array, one or two wide accesses where it is aligned
+template <typename T>
+__device__ __forceinline__ void ld4(const void *p, long long ps, bool vec, T *v) {
+    const T *a = static_cast<const T *>(p) + 4 * ps;
+    if (!vec) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) v[c] = a[c];
+    } else if (sizeof(T) == 4) {
+        const float4 f = *reinterpret_cast<const float4 *>(a);
+        v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+    } else {
+        const double2 f = reinterpret_cast<const double2 *>(a)[0],
+                      g = reinterpret_cast<const double2 *>(a)[1];
+        v[0] = f.x; v[1] = f.y; v[2] = g.x; v[3] = g.y;
+    }
+}
+template <typename T>
+__device__ __forceinline__ void st4(void *p, long long ps, bool vec, T a, T b, T c, T d) {
+    T *o = static_cast<T *>(p) + 4 * ps;
+    if (vec) {
+        store4(o, a, b, c, d);
+    } else {
+        o[0] = a; o[1] = b; o[2] = c; o[3] = d;
+    }
+}
+// zeros for slots s0, s0 + 1, ... of atom i's row (empty slots have no gradient)
+template <typename T>
+__device__ __forceinline__ void zero_slots(const FeatArgs &A, long long i, int s0, int lane) {
+    for (int s = s0 + lane; s < A.nn; s += 32)
+        st4<T>(A.grad_d12, i * A.nn + s, A.vec, T(0), T(0), T(0), T(0));
+}
+
+// The c-gradient without a per-atom table in memory: every warp adds its atoms' terms to a table
+// [T, T, nmax, nbase] of its own in shared memory, a block adds its four to FP64 sums and the last
+// block rounds those.  (A table per atom is 14 MB written, zeroed before and read again for 20,000 atoms
+// of four types; FP32 sums over this many blocks would round more than those over its 313.)
+template <typename T>
+__device__ __forceinline__ void flush_tables(const T *tab, int E, const FeatArgs &A) {
+    __shared__ bool last;
+    __syncthreads();
+    for (int e = threadIdx.x; e < E; e += blockDim.x) {
+        double v = 0.0;
+        for (int w = 0; w < kFeatWarps; ++w) v += (double)tab[w * E + e];
+        if (v != 0.0) atomicAdd(A.sum + e, v);
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0)
+        last = atomicAdd(reinterpret_cast<unsigned *>(A.sum + E), 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int e = threadIdx.x; e < E; e += blockDim.x) static_cast<T *>(A.dc)[e] = (T)__ldcg(A.sum + e);
+}
+
 // ---------------------------------------------------------------- radial (calculateNepFeat)
+// Bound by issue: the sums over pairs of one type (W) take as long as basis and features.  Empty slots
+// are written here, so no caller clears grad_d12.
 template <typename T, int MODE, int NM, int KM>
-__global__ void __launch_bounds__(32 * kFeatWarps) nep2b_op(FeatArgs A) {
+__global__ void __launch_bounds__(32 * kFeatWarps, sizeof(T) == 4 && NM <= 5 ? 8 : 1) nep2b_op(FeatArgs A) {
     __shared__ T s_st[kFeatWarps][32][KM + 1];
-    __shared__ int s_tj[kFeatWarps][32];
+    __shared__ __align__(16) int s_tj[kFeatWarps][32];
+    extern __shared__ __align__(16) unsigned char mb_raw[];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int T_ = A.ntypes, n_ = A.nmax, K = A.nbase;
     const T rc = (T)A.rc, rcinv = T(1) / rc;
     const T *c = static_cast<const T *>(A.coeff);
     const long long gw = (long long)blockIdx.x * kFeatWarps + wib;
     const long long nw = (long long)gridDim.x * kFeatWarps;
+    const bool want_c = MODE == kBwd2 || (MODE == kBwd && (A.W || A.dc));
+    const int E = T_ * T_ * n_ * K;
+    T *tab = reinterpret_cast<T *>(mb_raw) + wib * E;
+    T *wsum = reinterpret_cast<T *>(mb_raw) + kFeatWarps * E + wib * T_ * K;   // W of one atom
+    if (want_c && A.dc) {
+        for (int e = lane; e < E; e += 32) tab[e] = T(0);
+        for (int e = lane; e < T_ * K; e += 32) wsum[e] = T(0);
+        __syncwarp();
+    }
     for (long long i = gw; i < A.natoms; i += nw) {
         const int ti = (int)A.type[i];
         if (ti < 0 || ti >= T_) {
             if (lane == 0) atomicOr(A.err, MATPL_KERR_BAD_TYPE);
+            if (MODE != kBwd && lane < n_) static_cast<T *>(A.q)[i * A.ldQ + lane] = T(0);
+            if (MODE == kBwd && A.grad_d12) zero_slots<T>(A, i, 0, lane);
             continue;
         }
+        T *w = A.dc ? wsum : static_cast<T *>(A.W) + i * (long long)T_ * K;
         T G[NM], acc[NM];
 #pragma unroll
         for (int n = 0; n < NM; ++n) {
@@ -80,7 +155,10 @@ __global__ void __launch_bounds__(32 * kFeatWarps) nep2b_op(FeatArgs A) {
             const long long j = slot < A.nn ? A.NL[ps] : -1;
             const bool ok = j >= 0 && j < A.natoms;
             if (j >= A.natoms) atomicOr(A.err, MATPL_KERR_BAD_COUNT);
-            if (!__any_sync(0xffffffffu, ok)) break;
+            if (!__any_sync(0xffffffffu, ok)) {
+                if (MODE == kBwd && A.grad_d12) zero_slots<T>(A, i, base, lane);
+                break;
+            }
             T f[KM], df[KM];
             int tj = -1;
             if (ok) {
@@ -106,8 +184,9 @@ __global__ void __launch_bounds__(32 * kFeatWarps) nep2b_op(FeatArgs A) {
                         acc[n] += g;
                     }
             } else if (MODE == kBwd) {
-                if (use && A.grad_d12) {
+                if (A.grad_d12 && slot < A.nn) {
                     T gp = T(0);
+                    if (use)
 #pragma unroll
                     for (int n = 0; n < NM; ++n) {
                         if (n >= n_) break;
@@ -117,11 +196,10 @@ __global__ void __launch_bounds__(32 * kFeatWarps) nep2b_op(FeatArgs A) {
                             if (k < K) d += cr[n * K + k] * df[k];
                         gp += G[n] * d;
                     }
-                    static_cast<T *>(A.grad_d12)[ps * 4] = gp;
+                    st4<T>(A.grad_d12, ps, A.vec, gp, T(0), T(0), T(0));
                 }
 #pragma unroll
                 for (int k = 0; k < KM; ++k) s_st[wib][lane][k] = use ? f[k] : T(0);
-                s_tj[wib][lane] = use ? tj : -1;
             } else {
                 const T h0 = use ? ld<T>(A.H, ps * 4) : T(0);
                 if (use)
@@ -136,20 +214,53 @@ __global__ void __launch_bounds__(32 * kFeatWarps) nep2b_op(FeatArgs A) {
                     }
 #pragma unroll
                 for (int k = 0; k < KM; ++k) s_st[wib][lane][k] = use ? h0 * df[k] : T(0);
-                s_tj[wib][lane] = use ? tj : -1;
             }
-            if (MODE == kBwd2 || (MODE == kBwd && A.W)) {
+            if (want_c) {
+                s_tj[wib][lane] = use ? tj : -1;
                 __syncwarp();
-                T *W = static_cast<T *>(A.W) + i * (long long)T_ * K;
-                for (int e = lane; e < T_ * K; e += 32) {
-                    const int t = e / K, k = e - t * K;
-                    T sum = T(0);
-                    for (int p = 0; p < 32; ++p)
-                        if (s_tj[wib][p] == t) sum += s_st[wib][p][k];
-                    W[e] += sum;
+                if (sizeof(T) == 8) {
+                    // few additions, for the FP64 pipe: the slots of one type after another, lane k (and
+                    // k + 16, on the upper slots) sums column k
+                    for (unsigned rem = __ballot_sync(0xffffffffu, use); rem;) {
+                        const int t = __shfl_sync(0xffffffffu, tj, __ffs(rem) - 1);
+                        const unsigned mine = __ballot_sync(0xffffffffu, use && tj == t);
+                        rem &= ~mine;
+                        const int k0 = lane & 15;
+                        T sum = T(0);
+                        for (unsigned m = mine & (lane < 16 ? 0xffffu : 0xffff0000u); m; m &= m - 1)
+                            if (k0 < K) sum += s_st[wib][__ffs(m) - 1][k0];
+                        __syncwarp();
+                        sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+                        if (lane < K) w[t * K + lane] += sum;
+                    }
+                } else {
+                    // FP32: every lane an entry (t, k), a loop without branches
+                    for (int e = lane; e < T_ * K; e += 32) {
+                        const int t = e / K, k = e - t * K;
+                        T sum = T(0);
+#pragma unroll
+                        for (int p = 0; p < 32; p += 4) {
+                            const int4 j4 = *reinterpret_cast<const int4 *>(s_tj[wib] + p);
+                            if (j4.x == t) sum += s_st[wib][p][k];
+                            if (j4.y == t) sum += s_st[wib][p + 1][k];
+                            if (j4.z == t) sum += s_st[wib][p + 2][k];
+                            if (j4.w == t) sum += s_st[wib][p + 3][k];
+                        }
+                        w[e] += sum;
+                    }
                 }
                 __syncwarp();
             }
+        }
+        if (want_c && A.dc) {
+            T *tt = tab + ti * T_ * n_ * K;
+            for (int e = lane; e < T_ * n_ * K; e += 32) {
+                const int t = e / (n_ * K), n = e / K - t * n_, k = e % K;
+                tt[e] += ld<T>(A.G, i * A.ldG + n) * w[t * K + k];
+            }
+            __syncwarp();
+            for (int e = lane; e < T_ * K; e += 32) w[e] = T(0);
+            __syncwarp();
         }
         if (MODE != kBwd) {
 #pragma unroll
@@ -159,6 +270,7 @@ __global__ void __launch_bounds__(32 * kFeatWarps) nep2b_op(FeatArgs A) {
             }
         }
     }
+    if (want_c && A.dc) flush_tables<T>(reinterpret_cast<T *>(mb_raw), E, A);
 }
 
 // ---------------------------------------------------------------- angular (calculateNepMbFeat)
@@ -226,15 +338,34 @@ __device__ __forceinline__ T sbar_dot(const T *c3, int m, const T *sv, const T *
     return v;
 }
 
-// per warp shared memory of the angular operator
-template <typename T, int NM, int KM>
-struct MbSmem {
-    T s[NM][24], sd[NM][24], sb[NM][24], sbd[NM][24];
-    T ga[32][NM], gb[32][NM];        // pass 1: g_n, g_n dot; pass 2: B_n / P_n, Q_n
-    T ba[32][25], bb[32][25];        // pass 1: b_m, b_m dot
-    T fa[32][KM + 1], fb[32][KM + 1];// pass 2: f_k, f_k'
-    int tj[32];
+// per warp shared memory of the angular operator; the tangents (sd, sbd, gb, bb, fb) exist in BWD2
+// only and pass 2's f_k take the place of pass 1's b_m: 4.6 KB a warp in BWD, 9.7 in BWD2 (FP32)
+template <typename T, int MODE, int NM, int KM>
+struct alignas(16) MbSmem {
+    static constexpr int NP = (NM + 3) / 4 * 4, D = MODE == kBwd2 ? 1 : 0, G = MODE == kFwd ? 0 : 1;
+    static constexpr int F0 = KM + 1 > 25 ? KM + 1 : 25;
+    T ga[32][NP], gb[D ? 32 : 1][NP];      // pass 1: g_n, g_n dot; pass 2: B_n / P_n, Q_n
+    T ba[32][F0], bb[D ? 32 : 1][F0];      // pass 1: b_m, b_m dot; pass 2: f_k, f_k'
+    T s[NM][24], sd[D ? NM : 1][24], sb[G ? NM : 1][24], sbd[D ? NM : 1][24];
 };
+
+// a row of NP values in shared memory, 16 bytes at a time
+template <int NP>
+__device__ __forceinline__ void row_of(const float *p, float *v) {
+#pragma unroll
+    for (int q = 0; q < NP; q += 4) {
+        const float4 f = *reinterpret_cast<const float4 *>(p + q);
+        v[q] = f.x; v[q + 1] = f.y; v[q + 2] = f.z; v[q + 3] = f.w;
+    }
+}
+template <int NP>
+__device__ __forceinline__ void row_of(const double *p, double *v) {
+#pragma unroll
+    for (int q = 0; q < NP; q += 2) {
+        const double2 f = *reinterpret_cast<const double2 *>(p + q);
+        v[q] = f.x; v[q + 1] = f.y;
+    }
+}
 
 // pair quantities of slot ps: f, f' (K), g_n, g_n' (n), the unit vector and 1/r (0 outside
 // (1e-5, rc), where b_lm is zero)
@@ -242,7 +373,9 @@ template <typename T, int NM, int KM>
 __device__ __forceinline__ void mb_pair(const FeatArgs &A, const T *cr, long long ps, T *f, T *df, T *g,
                                         T *gp, T &ux, T &uy, T &uz, T &ri) {
     const T rc = (T)A.rc, rcinv = T(1) / rc;
-    const T r = ld<T>(A.d12, ps * 4);
+    T d4[4];
+    ld4<T>(A.d12, ps, A.vec, d4);
+    const T r = d4[0];
     basis<T, KM>(r, rc, rcinv, A.nbase, f, df);
 #pragma unroll
     for (int n = 0; n < NM; ++n) {
@@ -259,9 +392,9 @@ __device__ __forceinline__ void mb_pair(const FeatArgs &A, const T *cr, long lon
     }
     const bool in = r < rc && r > T(1e-5);
     ri = in ? T(1) / r : T(0);
-    ux = ld<T>(A.d12, ps * 4 + 1) * ri;
-    uy = ld<T>(A.d12, ps * 4 + 2) * ri;
-    uz = ld<T>(A.d12, ps * 4 + 3) * ri;
+    ux = d4[1] * ri;
+    uy = d4[2] * ri;
+    uz = d4[3] * ri;
 }
 
 // b_m and its partials in r and in (x, y, z) (= grad_u b / r; d/dr = -(u . grad_u b) / r)
@@ -277,10 +410,16 @@ __device__ __forceinline__ void harm_d(int m, T ux, T uy, T uz, T ri, T &b, T &b
     br = -(gx * ux + gy * uy + gz * uz) * ri;
 }
 
+// Bound by issue and shared loads (FP64: by the FP64 pipe).  Pass 1 has lanes over m with all n in
+// registers, so a pair's b_m is read once instead of once per n; the c-terms walk the pairs of one type
+// instead of testing every pair for every entry.  20,000 atoms, four types, 22 pairs each, FP32, with the
+// c-gradient: backward 167 -> 108 us, second backward 209 -> 162; 100,000: 786 -> 508, 1119 -> 791.  Five blocks an SM
+// in FP32 (102 registers): with 128 the backward takes 117 us.
 template <typename T, int MODE, int NM, int KM>
-__global__ void __launch_bounds__(32 * kFeatWarps) nepmb_op(FeatArgs A) {
+__global__ void __launch_bounds__(32 * kFeatWarps, sizeof(T) == 4 && NM <= 5 ? 5 : 1) nepmb_op(FeatArgs A) {
     extern __shared__ __align__(16) unsigned char mb_raw[];
-    using Sm = MbSmem<T, NM, KM>;
+    using Sm = MbSmem<T, MODE, NM, KM>;
+    constexpr int NP = Sm::NP;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     Sm &S = reinterpret_cast<Sm *>(mb_raw)[wib];
     const int T_ = A.ntypes, n_ = A.nmax, K = A.nbase;
@@ -293,17 +432,26 @@ __global__ void __launch_bounds__(32 * kFeatWarps) nepmb_op(FeatArgs A) {
     // served one address at a time
     __shared__ T c3s[24];
     if (threadIdx.x < 24) c3s[threadIdx.x] = C3<T>(threadIdx.x);
+    const bool want_c = MODE == kBwd2 || (MODE == kBwd && (A.W || A.dc));
+    const int E = T_ * T_ * n_ * K;
+    T *tabs = reinterpret_cast<T *>(mb_raw + sizeof(Sm) * kFeatWarps), *tab = tabs + wib * E;
+    if (want_c && A.dc)
+        for (int e = lane; e < E; e += 32) tab[e] = T(0);
     __syncthreads();
     for (long long i = gw; i < A.natoms; i += nw) {
         const int ti = (int)A.type[i];
         if (ti < 0 || ti >= T_) {
             if (lane == 0) atomicOr(A.err, MATPL_KERR_BAD_TYPE);
+            if (MODE != kBwd)
+                for (int e = lane; e < n_ * (A.l3 + four + five); e += 32)
+                    static_cast<T *>(A.q)[i * A.ldQ + e] = T(0);
+            if (MODE == kBwd && A.grad_d12) zero_slots<T>(A, i, 0, lane);
             continue;
         }
         // ---- pass 1: s_nm (and its tangent along H)
-        T sacc[6], sdacc[6];     // entries e = lane + 32 q of the n x 24 table (n <= 8)
+        T sacc[NP], sdacc[NP];   // lane m < 24 has column m
 #pragma unroll
-        for (int q = 0; q < 6; ++q) sacc[q] = sdacc[q] = T(0);
+        for (int n = 0; n < NP; ++n) sacc[n] = sdacc[n] = T(0);
         int nvalid = 0;
         for (int base = 0; base < A.nn; base += 32) {
             const int slot = base + lane;
@@ -321,17 +469,13 @@ __global__ void __launch_bounds__(32 * kFeatWarps) nepmb_op(FeatArgs A) {
             T f[KM], df[KM], g[NM], gp[NM], ux, uy, uz, ri;
             const T *cr = c + ((long long)(ti * T_ + (ok ? tj : 0)) * n_) * K;
             mb_pair<T, NM, KM>(A, cr, ok ? ps : 0, f, df, g, gp, ux, uy, uz, ri);
-            T h0 = T(0), h1 = T(0), h2 = T(0), h3 = T(0);
-            if (MODE == kBwd2 && ok) {
-                h0 = ld<T>(A.H, ps * 4);
-                h1 = ld<T>(A.H, ps * 4 + 1);
-                h2 = ld<T>(A.H, ps * 4 + 2);
-                h3 = ld<T>(A.H, ps * 4 + 3);
-            }
+            T h[4] = {T(0), T(0), T(0), T(0)};
+            if (MODE == kBwd2 && ok) ld4<T>(A.H, ps, A.vec, h);
 #pragma unroll
-            for (int n = 0; n < NM; ++n) {
-                S.ga[lane][n] = ok ? g[n] : T(0);
-                if (MODE == kBwd2) S.gb[lane][n] = ok ? gp[n] * h0 : T(0);
+            for (int n = 0; n < NP; ++n) {
+                const int q = n < NM ? n : 0;
+                S.ga[lane][n] = ok && n < NM ? g[q] : T(0);
+                if (MODE == kBwd2) S.gb[lane][n] = ok && n < NM ? gp[q] * h[0] : T(0);
             }
 #pragma unroll
             for (int m = 0; m < 24; ++m) {
@@ -339,33 +483,40 @@ __global__ void __launch_bounds__(32 * kFeatWarps) nepmb_op(FeatArgs A) {
                 harm_d<T>(m, ux, uy, uz, ri, b, br, bx, by, bz);
                 S.ba[lane][m] = ok ? b : T(0);
                 if (MODE == kBwd2)
-                    S.bb[lane][m] = ok ? br * h0 + bx * h1 + by * h2 + bz * h3 : T(0);
+                    S.bb[lane][m] = ok ? br * h[0] + bx * h[1] + by * h[2] + bz * h[3] : T(0);
             }
             __syncwarp();
+            // lanes over m, all n in registers: the pairs' g_n are read as broadcast rows
+            const int np = 32 - __clz(__ballot_sync(0xffffffffu, ok)), m = lane < 24 ? lane : 0;
+            T a[NP], d[NP];
 #pragma unroll
-            for (int q = 0; q < 6; ++q) {
-                const int e = lane + 32 * q;
-                if (e < nlm) {
-                    const int n = e / 24, m = e - n * 24;
-                    T a = T(0), d = T(0);
-                    for (int p = 0; p < 32; ++p) {
-                        a += S.ga[p][n] * S.ba[p][m];
-                        if (MODE == kBwd2) d += S.gb[p][n] * S.ba[p][m] + S.ga[p][n] * S.bb[p][m];
-                    }
-                    sacc[q] += a;
-                    sdacc[q] += d;
+            for (int n = 0; n < NP; ++n) a[n] = d[n] = T(0);
+            for (int p = 0; p < np; ++p) {
+                T ga[NP], gb[NP];
+                row_of<NP>(S.ga[p], ga);
+                const T b = S.ba[p][m];
+#pragma unroll
+                for (int n = 0; n < NM; ++n) a[n] += ga[n] * b;
+                if (MODE == kBwd2) {
+                    row_of<NP>(S.gb[p], gb);
+                    const T bd = S.bb[p][m];
+#pragma unroll
+                    for (int n = 0; n < NM; ++n) d[n] += gb[n] * b + ga[n] * bd;
                 }
             }
+#pragma unroll
+            for (int n = 0; n < NM; ++n) {
+                sacc[n] += a[n];
+                sdacc[n] += d[n];
+            }
             __syncwarp();
         }
+        if (lane < 24)
 #pragma unroll
-        for (int q = 0; q < 6; ++q) {
-            const int e = lane + 32 * q;
-            if (e < nlm) {
-                S.s[e / 24][e % 24] = sacc[q];
-                S.sd[e / 24][e % 24] = sdacc[q];
+            for (int n = 0; n < NM; ++n) {
+                S.s[n][lane] = sacc[n];
+                if (MODE == kBwd2) S.sd[n][lane] = sdacc[n];
             }
-        }
         __syncwarp();
         // ---- features (FWD) / their tangent (BWD2); Sbar, Sbar dot (BWD, BWD2)
         if (MODE == kFwd || MODE == kBwd2) {
@@ -373,7 +524,7 @@ __global__ void __launch_bounds__(32 * kFeatWarps) nepmb_op(FeatArgs A) {
             for (int e = lane; e < n_ * (A.l3 + four + five); e += 32) {
                 const int blk = e / n_, n = e - blk * n_;
                 const T *sv = S.s[n];
-                const T *sd = S.sd[n];
+                const T *sd = S.sd[MODE == kBwd2 ? n : 0];
                 T v = T(0);
                 if (blk < A.l3) {
                     const int m0 = blk == 0 ? 0 : blk == 1 ? 3 : blk == 2 ? 8 : 15;
@@ -418,6 +569,7 @@ __global__ void __launch_bounds__(32 * kFeatWarps) nepmb_op(FeatArgs A) {
         // ---- pass 2: grad_d12 (BWD) and the per-atom c-gradient table W (either may be
         // skipped in BWD: null pointer)
         T *W = A.W ? static_cast<T *>(A.W) + i * (long long)T_ * n_ * K : nullptr;
+        if (MODE == kBwd && A.grad_d12) zero_slots<T>(A, i, nvalid, lane);
         for (int base = 0; base < nvalid; base += 32) {
             const int slot = base + lane;
             const long long ps = i * A.nn + slot;
@@ -468,21 +620,12 @@ __global__ void __launch_bounds__(32 * kFeatWarps) nepmb_op(FeatArgs A) {
                     cz += g[n] * Bz[n];
                     S.ga[lane][n] = ok ? Bn[n] : T(0);
                 }
-                if (ok) {
-                    T *o = static_cast<T *>(A.grad_d12) + ps * 4;
-                    o[0] = c0;
-                    o[1] = cx;
-                    o[2] = cy;
-                    o[3] = cz;
-                }
+                if (slot < A.nn)
+                    st4<T>(A.grad_d12, ps, A.vec, ok ? c0 : T(0), ok ? cx : T(0), ok ? cy : T(0),
+                           ok ? cz : T(0));
             } else {
-                T h0 = T(0), h1 = T(0), h2 = T(0), h3 = T(0);
-                if (ok) {
-                    h0 = ld<T>(A.H, ps * 4);
-                    h1 = ld<T>(A.H, ps * 4 + 1);
-                    h2 = ld<T>(A.H, ps * 4 + 2);
-                    h3 = ld<T>(A.H, ps * 4 + 3);
-                }
+                T h[4] = {T(0), T(0), T(0), T(0)};
+                if (ok) ld4<T>(A.H, ps, A.vec, h);
                 T P[NM], Q[NM];
 #pragma unroll
                 for (int n = 0; n < NM; ++n) P[n] = Q[n] = T(0);
@@ -490,7 +633,7 @@ __global__ void __launch_bounds__(32 * kFeatWarps) nepmb_op(FeatArgs A) {
                 for (int m = 0; m < 24; ++m) {
                     T b, br, bx, by, bz;
                     harm_d<T>(m, ux, uy, uz, ri, b, br, bx, by, bz);
-                    const T bd = br * h0 + bx * h1 + by * h2 + bz * h3;
+                    const T bd = br * h[0] + bx * h[1] + by * h[2] + bz * h[3];
 #pragma unroll
                     for (int n = 0; n < NM; ++n) {
                         const T w = n < n_ ? S.sb[n][m] : T(0);
@@ -501,51 +644,92 @@ __global__ void __launch_bounds__(32 * kFeatWarps) nepmb_op(FeatArgs A) {
                 }
 #pragma unroll
                 for (int n = 0; n < NM; ++n) {
-                    S.ga[lane][n] = ok ? P[n] * h0 : T(0);
+                    S.ga[lane][n] = ok ? P[n] * h[0] : T(0);
                     S.gb[lane][n] = ok ? Q[n] : T(0);
                 }
             }
-            if (MODE == kBwd && !A.W) continue;     // grad_d12 only
+            if (!want_c) continue;     // grad_d12 only
 #pragma unroll
             for (int k = 0; k < KM; ++k) {
-                S.fa[lane][k] = ok ? f[k] : T(0);
-                S.fb[lane][k] = ok ? df[k] : T(0);
+                S.ba[lane][k] = ok ? f[k] : T(0);
+                if (MODE == kBwd2) S.bb[lane][k] = ok ? df[k] : T(0);
             }
-            S.tj[lane] = ok ? tj : -1;
             __syncwarp();
-            for (int e = lane; e < T_ * n_ * K; e += 32) {
-                const int t = e / (n_ * K), rem = e - t * n_ * K, n = rem / K, k = rem - n * K;
-                T sum = T(0);
-                for (int p = 0; p < 32; ++p) {
-                    if (S.tj[p] != t) continue;
-                    if (MODE == kBwd) sum += S.ga[p][n] * S.fa[p][k];
-                    else sum += S.ga[p][n] * S.fb[p][k] + S.gb[p][n] * S.fa[p][k];
+            // the pairs of one neighbor type after another, lanes over the (n, k) entries
+            constexpr int Q = (NM * KM + 31) / 32;
+            int en[Q], ek[Q];
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                const int e = min(lane + 32 * q, n_ * K - 1);
+                en[q] = e / K;
+                ek[q] = e - en[q] * K;
+            }
+            for (unsigned rem = __ballot_sync(0xffffffffu, ok); rem;) {
+                const int t = __shfl_sync(0xffffffffu, tj, __ffs(rem) - 1);
+                unsigned mine = __ballot_sync(0xffffffffu, ok && tj == t);
+                rem &= ~mine;
+                T sum[Q];
+#pragma unroll
+                for (int q = 0; q < Q; ++q) sum[q] = T(0);
+                for (; mine; mine &= mine - 1) {
+                    const int p = __ffs(mine) - 1;
+#pragma unroll
+                    for (int q = 0; q < Q; ++q) {
+                        if (MODE == kBwd2)
+                            sum[q] += S.ga[p][en[q]] * S.bb[p][ek[q]] + S.gb[p][en[q]] * S.ba[p][ek[q]];
+                        else
+                            sum[q] += S.ga[p][en[q]] * S.ba[p][ek[q]];
+                    }
                 }
-                W[e] += sum;
+                T *o = A.dc ? tab + (ti * T_ + t) * n_ * K : W + t * n_ * K;
+#pragma unroll
+                for (int q = 0; q < Q; ++q)
+                    if (lane + 32 * q < n_ * K) o[lane + 32 * q] += sum[q];
             }
             __syncwarp();
         }
     }
+    if (want_c && A.dc) flush_tables<T>(tabs, E, A);
+}
+
+// Blocks: enough for every atom's warp, but where each leaves a table behind, one wave of them.
+template <typename K>
+int feat_blocks(const FeatArgs &A, K k, size_t smem) {
+    const long long need = (A.natoms + kFeatWarps - 1) / kFeatWarps;
+    int per_sm = 32;
+    if (A.dc && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 32 * kFeatWarps, smem) != cudaSuccess)
+        per_sm = 1;
+    return (int)std::max<long long>(1, std::min<long long>(need, (long long)device_sms() * std::max(per_sm, 1)));
+}
+
+template <typename T>
+size_t table_bytes(const FeatArgs &A) {
+    return A.dc ? sizeof(T) * kFeatWarps * A.ntypes * A.ntypes * A.nmax * A.nbase : 0;
 }
 
 template <typename T, int MODE, int NM, int KM>
 int launch_mb(const FeatArgs &A, cudaStream_t s) {
-    const size_t smem = sizeof(MbSmem<T, NM, KM>) * kFeatWarps;
+    const size_t smem = sizeof(MbSmem<T, MODE, NM, KM>) * kFeatWarps + table_bytes<T>(A);
     auto k = nepmb_op<T, MODE, NM, KM>;
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
         cudaSuccess) {
         set_error("matpl_nep_feat: shared-memory attribute rejected");
         return MATPL_ERR_CUDA;
     }
-    const long long blocks = std::min<long long>((A.natoms + kFeatWarps - 1) / kFeatWarps, (long long)device_sms() * 32);
-    k<<<(int)std::max<long long>(blocks, 1), 32 * kFeatWarps, smem, s>>>(A);
+    k<<<feat_blocks(A, k, smem), 32 * kFeatWarps, smem, s>>>(A);
     return check_launch("matpl_nep_feat");
 }
 
 template <typename T, int MODE, int NM, int KM>
 int launch_2b(const FeatArgs &A, cudaStream_t s) {
-    const long long blocks = std::min<long long>((A.natoms + kFeatWarps - 1) / kFeatWarps, (long long)device_sms() * 32);
-    nep2b_op<T, MODE, NM, KM><<<(int)std::max<long long>(blocks, 1), 32 * kFeatWarps, 0, s>>>(A);
+    const size_t smem = A.dc ? table_bytes<T>(A) + sizeof(T) * kFeatWarps * A.ntypes * A.nbase : 0;
+    auto k = nep2b_op<T, MODE, NM, KM>;
+    if (smem && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+                    cudaSuccess) {
+        set_error("matpl_nep_feat: shared-memory attribute rejected");
+        return MATPL_ERR_CUDA;
+    }
+    k<<<feat_blocks(A, k, smem), 32 * kFeatWarps, smem, s>>>(A);
     return check_launch("matpl_nep_feat");
 }
 
@@ -905,12 +1089,12 @@ extern "C" int matpl_nep_force_virial_grad(int dtype, int natoms, int max_nn, in
     return check_launch("matpl_nep_force_virial_grad");
 }
 
-extern "C" int matpl_nep_feat_op(int dtype, int part, int mode, int natoms, int max_nn,
-                                 int ntypes, int n_max, int n_base, int l_max_3b, int l_max_4b,
-                                 int l_max_5b, double cutoff, const void *coeff, const void *d12,
-                                 const long long *NL, const long long *type_map, const void *G,
-                                 long long ldG, const void *H, void *q, long long ldQ,
-                                 void *grad_d12, void *W, int *err_dev, void *stream) {
+static int feat_op(int dtype, int part, int mode, int natoms, int max_nn, int ntypes, int n_max,
+                   int n_base, int l_max_3b, int l_max_4b, int l_max_5b, double cutoff,
+                   const void *coeff, const void *d12, const long long *NL,
+                   const long long *type_map, const void *G, long long ldG, const void *H, void *q,
+                   long long ldQ, void *grad_d12, void *W, void *dc, void *sum, int *err_dev,
+                   void *stream) {
     MATPL_REQUIRE(dtype == MATPL_F32 || dtype == MATPL_F64, MATPL_ERR_DTYPE,
                   "matpl_nep_feat_op: dtype is MATPL_F32 or MATPL_F64");
     MATPL_REQUIRE(part == 0 || part == 1, MATPL_ERR_INVALID, "part: 0 radial, 1 angular");
@@ -925,9 +1109,9 @@ extern "C" int matpl_nep_feat_op(int dtype, int part, int mode, int natoms, int 
     MATPL_REQUIRE(err_dev && coeff && type_map && (natoms == 0 || (d12 && NL)), MATPL_ERR_INVALID,
                   "null pointer argument");
     MATPL_REQUIRE(mode != 0 || q, MATPL_ERR_INVALID, "fwd needs q");
-    MATPL_REQUIRE(mode != 1 || (G && (W || grad_d12)), MATPL_ERR_INVALID,
+    MATPL_REQUIRE(mode != 1 || (G && (W || dc || grad_d12)), MATPL_ERR_INVALID,
                   "bwd needs G and grad_d12 or W");
-    MATPL_REQUIRE(mode != 2 || (G && H && q && W), MATPL_ERR_INVALID, "bwd2 needs G, H, gso, W");
+    MATPL_REQUIRE(mode != 2 || (G && H && q && (W || dc)), MATPL_ERR_INVALID, "bwd2 needs G, H, gso, W");
     if (natoms == 0 || max_nn == 0) return MATPL_OK;
     MATPL_REQUIRE_ON_DEVICE(d12, "matpl_nep_feat_op");
     FeatArgs A{};
@@ -948,6 +1132,9 @@ extern "C" int matpl_nep_feat_op(int dtype, int part, int mode, int natoms, int 
     A.ldQ = ldQ;
     A.grad_d12 = grad_d12;
     A.W = W;
+    A.dc = dc;
+    A.sum = static_cast<double *>(sum);
+    A.vec = (((uintptr_t)d12 | (uintptr_t)H | (uintptr_t)grad_d12) & 15u) == 0;
     A.l3 = l_max_3b;
     A.four = l_max_4b > 0;
     A.five = l_max_5b > 0;
@@ -963,4 +1150,73 @@ extern "C" int matpl_nep_feat_op(int dtype, int part, int mode, int natoms, int 
     if (mode == 0) return dispatch<float, kFwd>(ang, A, s);
     if (mode == 1) return dispatch<float, kBwd>(ang, A, s);
     return dispatch<float, kBwd2>(ang, A, s);
+}
+
+extern "C" int matpl_nep_feat_op(int dtype, int part, int mode, int natoms, int max_nn,
+                                 int ntypes, int n_max, int n_base, int l_max_3b, int l_max_4b,
+                                 int l_max_5b, double cutoff, const void *coeff, const void *d12,
+                                 const long long *NL, const long long *type_map, const void *G,
+                                 long long ldG, const void *H, void *q, long long ldQ,
+                                 void *grad_d12, void *W, int *err_dev, void *stream) {
+    return feat_op(dtype, part, mode, natoms, max_nn, ntypes, n_max, n_base, l_max_3b, l_max_4b,
+                   l_max_5b, cutoff, coeff, d12, NL, type_map, G, ldG, H, q, ldQ, grad_d12, W,
+                   nullptr, nullptr, err_dev, stream);
+}
+
+// Tables in shared memory up to 16 KB a block (four types of n 5, K 9 in FP32 take 11.5): the backward of
+// 20,000 atoms takes 65 us radial and 108 angular, by a per-atom table in W 72 and 123.  Beyond that the
+// tables cost more blocks on an SM than the passes over W (eight types, 46 KB: 149 and 183 us against
+// 105 and 157), except in a batch of no more blocks than fit side by side anyway: up to 1,024 atoms
+// eight types take 36 and 40 us against 53 and 42, so there 48 KB is allowed.
+static bool feat_tabled(int dtype, int natoms, int ntypes, int n_max, int n_base) {
+    const size_t esz = dtype == MATPL_F64 ? sizeof(double) : sizeof(float);
+    const size_t tables = esz * kFeatWarps * ntypes * ntypes * n_max * n_base;
+    return tables <= kTableBytes || (tables <= 3 * kTableBytes && natoms <= 1024);
+}
+
+extern "C" size_t matpl_nep_feat_grad_workspace_bytes(int dtype, int part, int natoms, int ntypes,
+                                                      int n_max, int n_base) {
+    const size_t row = (size_t)ntypes * n_max * n_base;
+    if (feat_tabled(dtype, natoms, ntypes, n_max, n_base)) return 8 * (row * ntypes + 1);
+    return (dtype == MATPL_F64 ? sizeof(double) : sizeof(float)) * natoms *
+           (part == 0 ? (size_t)ntypes * n_base : row);
+}
+
+extern "C" int matpl_nep_feat_grad(int dtype, int part, int mode, int natoms, int max_nn,
+                                   int ntypes, int n_max, int n_base, int l_max_3b, int l_max_4b,
+                                   int l_max_5b, double cutoff, const void *coeff,
+                                   const void *d12, const long long *NL,
+                                   const long long *type_map, const void *G, long long ldG,
+                                   const void *H, void *gso, long long ldQ, void *grad_d12,
+                                   void *dc, void *workspace, size_t workspace_bytes,
+                                   int *err_dev, void *stream) {
+    MATPL_REQUIRE(dtype == MATPL_F32 || dtype == MATPL_F64, MATPL_ERR_DTYPE,
+                  "matpl_nep_feat_grad: dtype is MATPL_F32 or MATPL_F64");
+    MATPL_REQUIRE(part == 0 || part == 1, MATPL_ERR_INVALID, "part: 0 radial, 1 angular");
+    MATPL_REQUIRE(mode == kBwd || mode == kBwd2, MATPL_ERR_INVALID, "mode: 1 bwd, 2 bwd2");
+    MATPL_REQUIRE(natoms >= 0 && max_nn >= 0 && ntypes >= 1, MATPL_ERR_INVALID, "bad sizes");
+    MATPL_REQUIRE(n_max >= 1 && n_max <= 8 && n_base >= 1 && n_base <= 16, MATPL_ERR_UNSUPPORTED,
+                  "compiled for n_max <= 8 and basis size <= 16 (coefficient dims 2, 3)");
+    MATPL_REQUIRE(dc, MATPL_ERR_INVALID, "null pointer argument");
+    const size_t need =
+        matpl_nep_feat_grad_workspace_bytes(dtype, part, natoms, ntypes, n_max, n_base);
+    MATPL_REQUIRE(need == 0 || (workspace && workspace_bytes >= need), MATPL_ERR_INVALID,
+                  "workspace too small");
+    MATPL_REQUIRE_ON_DEVICE(dc, "matpl_nep_feat_grad");
+    cudaStream_t s = as_stream(stream);
+    const size_t esz = dtype == MATPL_F64 ? sizeof(double) : sizeof(float);
+    const bool tabled = feat_tabled(dtype, natoms, ntypes, n_max, n_base);
+    if (cudaMemsetAsync(workspace, 0, need, s) != cudaSuccess ||
+        ((natoms == 0 || max_nn == 0) &&
+         cudaMemsetAsync(dc, 0, esz * ntypes * ntypes * n_max * n_base, s) != cudaSuccess)) {
+        set_error("matpl_nep_feat_grad: memset failed");
+        return MATPL_ERR_CUDA;
+    }
+    const int st = feat_op(dtype, part, mode, natoms, max_nn, ntypes, n_max, n_base, l_max_3b,
+                           l_max_4b, l_max_5b, cutoff, coeff, d12, NL, type_map, G, ldG, H, gso,
+                           ldQ, grad_d12, tabled ? nullptr : workspace, tabled ? dc : nullptr,
+                           workspace, err_dev, stream);
+    if (st != MATPL_OK || tabled || natoms == 0 || max_nn == 0) return st;
+    return matpl_nep_cgrad(dtype, part, natoms, ntypes, n_max, n_base, type_map, G, ldG, workspace,
+                           dc, err_dev, stream);
 }

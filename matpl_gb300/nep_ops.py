@@ -16,8 +16,7 @@ summed per image of ``num_atom`` and its backward uses each image's own gradient
 reference's CUDA backward applies the first image's to all atoms).
 
 For ``nep_train.NEPTrain`` the module also has the training step's own forms: ``nep_feat_d12``
-(the descriptor's d12 gradient alone, the force path), the c-gradient reduction
-``matpl_nep_cgrad`` behind every backward, ``nep_force_virial`` (forces and per-image virial
+(the descriptor's d12 gradient alone, the force path), ``nep_force_virial`` (forces and per-image virial
 from dE and the (r, x, y, z) rows, calculate_Ri formed in the kernel) and ``nep_zbl`` (the ZBL
 term, nep_net.py:916-991).
 """
@@ -70,63 +69,62 @@ def _nfeat(part, nmax, l3, l4, l5):
     return nmax * (l3 + (1 if l4 > 0 else 0) + (1 if l5 > 0 else 0))
 
 
+def _as(t, dt):
+    """``t`` as a contiguous tensor of dtype ``dt`` (itself where it is one)."""
+    if t.dtype != dt:
+        t = t.to(dt)
+    return t if t.is_contiguous() else t.contiguous()
+
+
+def _rows(t, dt):
+    """``t`` [N, F] of dtype ``dt`` and its row stride; a slice of a wider array stays in place."""
+    if t.dtype != dt:
+        t = t.to(dt)
+    if t.stride(1) != 1 or t.stride(0) < t.shape[1]:
+        t = t.contiguous()
+    return t, max(t.stride(0), t.shape[1])
+
+
 @_lib.on_device
 def _feat_call(part, mode, coeff, d12, NL, atom_map, rc, l3=0, l4=0, l5=0, G=None, H=None,
                want_d=True, want_c=True):
-    """One launch of ``matpl_nep_feat_op``; returns (q or gso, grad_d12, W).  In the backward
-    mode ``want_d`` / ``want_c`` select grad_d12 and the c-gradient table (None if not)."""
+    """One call of the descriptor operator; returns (q or gso, grad_d12, dL/dc).  In the backward
+    mode ``want_d`` / ``want_c`` select grad_d12 and dL/dc (None if not)."""
     _require_cuda(coeff, d12, NL, atom_map)
     N, NN = NL.shape
     T, _, nmax, K = coeff.shape
     dev, dt = d12.device, d12.dtype
     code = _dtype_code(d12)
-    c = coeff.detach().to(dt).contiguous()
-    dd = d12.detach().contiguous()
-    nl = NL.contiguous().to(torch.int64)
-    tm = atom_map.contiguous().to(torch.int64)
+    c, dd = _as(coeff, dt), _as(d12, dt)
+    nl, tm = _as(NL, torch.int64), _as(atom_map, torch.int64)
     F = _nfeat(part, nmax, l3, l4, l5)
     err = _err_word(dev)
-    q = gd = W = None
-    Gc = G.detach().to(dt).contiguous() if G is not None else None
-    Hc = H.detach().to(dt).contiguous() if H is not None else None
-    if mode in (MODE_FWD, MODE_BWD2):
-        q = torch.empty(N, F, dtype=dt, device=dev) if mode == MODE_FWD else \
-            torch.zeros(N, F, dtype=dt, device=dev)
-        if N * NN == 0:
-            q.zero_()
-    if mode == MODE_BWD and want_d:
-        gd = torch.zeros(N, NN, 4, dtype=dt, device=dev)
-    if mode == MODE_BWD2 or (mode == MODE_BWD and want_c):
-        shape = (N, T, K) if part == PART_RADIAL else (N, T, nmax, K)
-        W = torch.zeros(shape, dtype=dt, device=dev)
-    check(_lib.load().matpl_nep_feat_op(
-        code, part, mode, N, NN, T, nmax, K, l3, l4, l5, float(rc), ptr(c), ptr(dd), ptr(nl),
-        ptr(tm), ptr(Gc), F, ptr(Hc), ptr(q), F, ptr(gd), ptr(W), ptr(err), _stream(dev)),
-        "matpl_nep_feat_op")
+    Gc, ldG = _rows(G, dt) if G is not None else (None, F)
+    q = gd = gc = None
+    if mode != MODE_BWD:
+        q = (torch.zeros if N * NN == 0 else torch.empty)(N, F, dtype=dt, device=dev)
+    elif want_d:
+        gd = torch.empty(N, NN, 4, dtype=dt, device=dev)
+    lib, stream = _lib.load(), _stream(dev)
+    if mode == MODE_FWD or (mode == MODE_BWD and not want_c):
+        check(lib.matpl_nep_feat_op(
+            code, part, mode, N, NN, T, nmax, K, l3, l4, l5, float(rc), ptr(c), ptr(dd), ptr(nl),
+            ptr(tm), ptr(Gc), ldG, 0, ptr(q), F, ptr(gd), 0, ptr(err), stream),
+            "matpl_nep_feat_op")
+    else:
+        Hc = _as(H, dt) if H is not None else None
+        gc = torch.empty(T, coeff.shape[1], nmax, K, dtype=dt, device=dev)
+        nbytes = lib.matpl_nep_feat_grad_workspace_bytes(code, part, N, T, nmax, K)
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=dev) if nbytes else None
+        check(lib.matpl_nep_feat_grad(
+            code, part, mode, N, NN, T, nmax, K, l3, l4, l5, float(rc), ptr(c), ptr(dd), ptr(nl),
+            ptr(tm), ptr(Gc), ldG, ptr(Hc), ptr(q), F, ptr(gd), ptr(gc), ptr(ws), nbytes, ptr(err),
+            stream), "matpl_nep_feat_grad")
+        if gc.dtype != coeff.dtype:
+            gc = gc.to(coeff.dtype)
     if _check_each_call:
         check_errors(dev)
-    return q, gd, W
-
-
-@_lib.on_device
-def _c_grad(part, W, G, atom_map, T):
-    """dL/dc [T, T, n, K] from the per-atom tables (``matpl_nep_cgrad``): radial
-    sum_i G[i, n] W[i, t, k]; angular sum_i W[i] (G already folded in), each into row t_i."""
-    dev, dt = W.device, W.dtype
-    N = W.shape[0]
-    if part == PART_RADIAL:
-        _, Tt, K = W.shape
-        Gc = G.detach().to(dt).contiguous()
-        n = Gc.shape[1]
-    else:
-        _, Tt, n, K = W.shape
-        Gc = None
-    out = torch.empty(T, Tt, n, K, dtype=dt, device=dev)
-    tm = atom_map.contiguous().to(torch.int64)
-    check(_lib.load().matpl_nep_cgrad(_dtype_code(W), part, N, T, n, K, ptr(tm), ptr(Gc),
-                                      n, ptr(W.contiguous()), ptr(out), ptr(_err_word(dev)),
-                                      _stream(dev)), "matpl_nep_cgrad")
-    return out
+    return q, gd, gc
 
 
 def _second_backward(ctx, g_gd):
@@ -134,10 +132,9 @@ def _second_backward(ctx, g_gd):
     second backward mode (gso = dq/dd12 . g_gd, and the c-terms)."""
     G, coeff, d12, NL, atom_map = ctx.saved_tensors
     part, rc, l3, l4, l5 = ctx.meta
-    gso, _, W2 = _feat_call(part, MODE_BWD2, coeff, d12, NL, atom_map, rc, l3, l4, l5,
-                            G=G, H=g_gd)
-    gsc = _c_grad(part, W2, G.detach(), atom_map, coeff.shape[0]).to(coeff.dtype)
-    return gso.to(G.dtype), gsc
+    gso, _, gsc = _feat_call(part, MODE_BWD2, coeff, d12, NL, atom_map, rc, l3, l4, l5,
+                             G=G, H=g_gd)
+    return gso if gso.dtype == G.dtype else gso.to(G.dtype), gsc
 
 
 class _NepFeatGrad(torch.autograd.Function):
@@ -145,8 +142,8 @@ class _NepFeatGrad(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, G, coeff, d12, NL, atom_map, part, rc, l3, l4, l5):
-        _, gd, W = _feat_call(part, MODE_BWD, coeff, d12, NL, atom_map, rc, l3, l4, l5, G=G)
-        gc = _c_grad(part, W, G.detach(), atom_map, coeff.shape[0]).to(coeff.dtype)
+        _, gd, gc = _feat_call(part, MODE_BWD, coeff, d12, NL, atom_map, rc, l3, l4, l5, G=G)
+        ctx.set_materialize_grads(False)       # no zeros for an output that no loss uses
         ctx.save_for_backward(G, coeff, d12, NL, atom_map)
         ctx.meta = (part, rc, l3, l4, l5)
         return gc, gd
@@ -154,7 +151,8 @@ class _NepFeatGrad(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g_gc, g_gd):
         if g_gd is None:
-            return (None,) * 10
+            G, coeff = ctx.saved_tensors[:2]
+            return (torch.zeros_like(G), torch.zeros_like(coeff)) + (None,) * 8
         gso, gsc = _second_backward(ctx, g_gd)
         return gso, gsc, None, None, None, None, None, None, None, None
 
@@ -181,9 +179,8 @@ class _NepFeatCGrad(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, G, coeff, d12, NL, atom_map, part, rc, l3, l4, l5):
-        _, _, W = _feat_call(part, MODE_BWD, coeff, d12, NL, atom_map, rc, l3, l4, l5, G=G,
-                             want_d=False)
-        return _c_grad(part, W, G.detach(), atom_map, coeff.shape[0]).to(coeff.dtype)
+        return _feat_call(part, MODE_BWD, coeff, d12, NL, atom_map, rc, l3, l4, l5, G=G,
+                          want_d=False)[2]
 
     @staticmethod
     @torch.autograd.function.once_differentiable

@@ -194,12 +194,19 @@ def ptr(t) -> int:
 
 
 def _cuda_devices(objs, found):
+    """The device index of the CUDA tensors among ``objs`` and what their lists hold: ``found`` (-1:
+    none so far) when there is no other, a set when there are several."""
     for o in objs:
         if isinstance(o, torch.Tensor):
-            if o.is_cuda:
-                found.add(o.device.index)
+            d = o.get_device()             # -1 on the host
+            if d >= 0 and d != found:
+                if found == -1:
+                    found = d
+                else:
+                    found = (found if isinstance(found, set) else {found}) | {d}
         elif isinstance(o, (list, tuple)):
-            _cuda_devices(o, found)
+            found = _cuda_devices(o, found)
+    return found
 
 
 def on_device(fn):
@@ -211,14 +218,14 @@ def on_device(fn):
     duration of the call (a no-op when it already is)."""
     @functools.wraps(fn)
     def wrapper(*args, **kwargs):
-        found = set()
-        _cuda_devices(args, found)
-        _cuda_devices(kwargs.values(), found)
-        if not found:
-            return fn(*args, **kwargs)
-        if len(found) > 1:
+        found = _cuda_devices(args, -1)
+        if kwargs:
+            found = _cuda_devices(kwargs.values(), found)
+        if isinstance(found, set):
             raise MatplError(f"{fn.__qualname__}: CUDA tensors on several devices "
                              f"{sorted(found)}; put every argument on one GPU")
-        with torch.cuda.device(found.pop()):
+        if found < 0 or found == torch.cuda.current_device():
+            return fn(*args, **kwargs)
+        with torch.cuda.device(found):
             return fn(*args, **kwargs)
     return wrapper

@@ -211,11 +211,11 @@ class DP(torch.nn.Module):
                    "Force": torch.empty(B, N + nghost, 3, dtype=self.dtype, device=dev),
                    "Virial": torch.empty(B, 9, dtype=torch.float64, device=dev)}
         lib = _lib.load()
-        from .ops import workspace
+        from .ops import _stream, workspace
         nbytes = lib.matpl_dp_workspace_bytes(self.code, B, N)
         ws = workspace(dev, nbytes, "dp")
         model = self._model_struct(present)
-        stream = torch.cuda.current_stream(dev).cuda_stream
+        stream = _stream(dev)
         if num_neigh is None:
             check(lib.matpl_dp_eval(self.code, ctypes.byref(model), B, N, S, nghost, ptr(ln),
                                     ptr(idr), ptr(tm), ptr(out["Ei_atom"]), ptr(out["Etot"]),

@@ -336,7 +336,7 @@ class NEP(torch.nn.Module):
         import ctypes
         from . import _lib
         from ._lib import check, ptr
-        from .ops import workspace
+        from .ops import _stream, workspace
         if not Ri_radial.is_cuda:
             raise _lib.MatplError("NEP.evaluate takes CUDA tensors (no CPU fallback)")
         dev = Ri_radial.device
@@ -354,7 +354,7 @@ class NEP(torch.nn.Module):
             raise _lib.MatplError("Ri_radial / Ri_angular must be (r, x, y, z) (with_rij = True)")
         lib = _lib.load()
         ws = workspace(dev, lib.matpl_nep_workspace_bytes(self.code, B, N), "nep")
-        stream = torch.cuda.current_stream(dev).cuda_stream
+        stream = _stream(dev)
         if Ri_radial.dtype == torch.float32 and NL_radial.dtype == torch.int32:
             return self._evaluate_compact(NN_radial, NL_radial, Ri_radial, NN_angular, NL_angular,
                                           Ri_angular, na, tm, ws, stream, out, descriptor_only)

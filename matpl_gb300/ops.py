@@ -9,6 +9,7 @@ mirrors ``src/pre_data/dpuni_data_loader.py:595-650`` on the GPU and ``env_mat``
 Every op runs on the current CUDA stream of its inputs' device, goes through the C ABI of
 ``libmatpl_gb300.so`` and raises ``MatplError`` on failure; there is no CPU fallback.
 """
+import math
 from typing import List, Optional, Sequence, Tuple, Union
 
 import torch
@@ -20,7 +21,9 @@ _DT = {torch.float32: MATPL_F32, torch.float64: MATPL_F64}
 
 
 def _stream(dev: torch.device) -> int:
-    return torch.cuda.current_stream(dev).cuda_stream
+    """The raw handle of torch's current stream on ``dev``."""
+    index = dev.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
 def _dtype_code(t: torch.Tensor) -> int:
@@ -39,12 +42,21 @@ def _nghost(n) -> int:
     return int(n.item()) if isinstance(n, torch.Tensor) else int(n)
 
 
+def _slots(list_neigh) -> int:
+    """Slots of one atom's list [B, N, ...]."""
+    if list_neigh.shape[1] == 0:
+        return 0
+    if list_neigh.shape[0] == 0:
+        raise IndexError("list_neigh holds atoms but no configuration")
+    return math.prod(list_neigh.shape[2:])
+
+
 class _CalculateForce(torch.autograd.Function):
     @staticmethod
     @_lib.on_device
     def forward(ctx, list_neigh, dE, Ri_d, F, nghost: int):
         B, N = list_neigh.shape[0], list_neigh.shape[1]
-        S = list_neigh[0, 0].numel() if N > 0 else 0
+        S = _slots(list_neigh)
         nl = list_neigh.contiguous().to(torch.int32)
         dE_c, Rd = dE.contiguous(), Ri_d.contiguous()
         out = torch.empty(B, N + nghost, 3, dtype=dE.dtype, device=dE.device)
@@ -75,7 +87,7 @@ class _CalculateVirial(torch.autograd.Function):
     @_lib.on_device
     def forward(ctx, list_neigh, dE, Rij, Ri_d, nghost: int):
         B, N = list_neigh.shape[0], list_neigh.shape[1]
-        S = list_neigh[0, 0].numel() if N > 0 else 0
+        S = _slots(list_neigh)
         nl = list_neigh.contiguous().to(torch.int32)
         dE_c, Rj, Rd = dE.contiguous(), Rij.contiguous().to(dE.dtype), Ri_d.contiguous()
         vir = torch.empty(B, 9, dtype=dE.dtype, device=dE.device)
@@ -87,6 +99,7 @@ class _CalculateVirial(torch.autograd.Function):
         ctx.save_for_backward(nl, Rj, Rd)
         ctx.meta = (B, N, S, dE.shape)
         ctx.mark_non_differentiable(avir)
+        ctx.set_materialize_grads(False)       # no zeros in place of avir's gradient
         return vir, avir
 
     @staticmethod
@@ -191,8 +204,8 @@ def workspace(device: torch.device, nbytes: int, tag: str) -> torch.Tensor:
     (they could overlap on the GPU), and a buffer that is replaced by a larger one was only
     ever used on that stream, so the allocator may hand it out again in stream order."""
     device = torch.device(device)
-    stream = torch.cuda.current_stream(device).cuda_stream
-    key = (str(device), stream, tag)
+    stream = _stream(device)
+    key = (device, stream, tag)
     buf = _ws_cache.get(key)
     if buf is None or buf.numel() < nbytes:
         buf = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device)

@@ -218,7 +218,9 @@ __device__ __forceinline__ void stage_weights(const T *__restrict__ src, T *dst,
 }
 
 // --------------------------------------------------------------------------- dp_embed_fwd
-template <typename T, bool WS, bool CMP>
+// SPLIT: the block's warps share one atom, each taking every kWarps-th run of 32 slots, and warp 0 adds
+// their sums in order (FP64 only: in FP32 a caller's FP64 totals would show the regrouping).
+template <typename T, bool WS, bool CMP, bool SPLIT>
 __global__ void __launch_bounds__(kWarps * 32)
 dp_embed_fwd(const int32_t *__restrict__ list_neigh, const T *__restrict__ idr,
              const int32_t *__restrict__ type_map, const T *__restrict__ params,
@@ -239,13 +241,15 @@ dp_embed_fwd(const int32_t *__restrict__ list_neigh, const T *__restrict__ idr,
     if (WS) stage_weights(params, wsm, wcount);
     const int S = P.nslots;
     const long long total = (long long)P.batch * P.natoms;
-    for (long long t = (long long)blockIdx.x * nwarps + warp; t < total;
-         t += (long long)gridDim.x * nwarps) {
+    const int atoms = SPLIT ? 1 : nwarps, stride = SPLIT ? 32 * nwarps : 32;
+    for (long long t = (long long)blockIdx.x * atoms + (SPLIT ? 0 : warp); t < total;
+         t += (long long)gridDim.x * atoms) {
         const int i = (int)(t % P.natoms);
         const int ti = type_map[i];
         T *Arow = Aout + t * NA;
         if (ti < 0 || ti >= P.ntypes || !((P.present_mask >> ti) & 1)) {
-            for (int e = lane; e < NA; e += 32) Arow[e] = T(0);
+            if (!SPLIT || warp == 0)
+                for (int e = lane; e < NA; e += 32) Arow[e] = T(0);
             continue;
         }
         const int cnt = scan_slots(list_neigh + t * S, P.num_neigh ? P.num_neigh + t * P.ntypes : nullptr,
@@ -253,7 +257,7 @@ dp_embed_fwd(const int32_t *__restrict__ list_neigh, const T *__restrict__ idr,
         T acc[4] = {T(0), T(0), T(0), T(0)};
         const T *avg = davg + 4 * ti;
         const T *sd = dstd + 4 * ti;
-        for (int c0 = 0; c0 < cnt; c0 += 32) {
+        for (int c0 = SPLIT ? 32 * warp : 0; c0 < cnt; c0 += stride) {
             const int k = c0 + lane;
             T x[E], t3[E], rh[4] = {T(0), T(0), T(0), T(0)};
             int tj = 0;
@@ -290,6 +294,20 @@ dp_embed_fwd(const int32_t *__restrict__ list_neigh, const T *__restrict__ idr,
                     acc[q] = a;
                 }
             }
+        }
+        if (SPLIT) {
+            __syncwarp();
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (lane + 32 * q < NA) Gs[lane + 32 * q] = acc[q];
+            __syncthreads();
+            if (warp == 0)
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    for (int w = 1; w < nwarps; ++w)
+                        if (lane + 32 * q < NA) acc[q] += Gs_all[w * 32 * (E + 1) + lane + 32 * q];
+            __syncthreads();
+            if (warp != 0) continue;
         }
         // empty slots: n_empty(t_j) * R_pad (x) G(s_pad)
         for (int tj = 0; tj < P.ntypes; ++tj) {
@@ -540,7 +558,7 @@ int launch_fit(const T *A, const int32_t *type_map, const T *params, T *Ei, T *d
 }
 
 // --------------------------------------------------------------------------- dp_embed_bwd
-template <typename T, bool WS, bool CMP>
+template <typename T, bool WS, bool CMP, bool SPLIT>
 __global__ void __launch_bounds__(kWarps * 32)
 dp_embed_bwd(const int32_t *__restrict__ list_neigh, const T *__restrict__ idr,
              const int32_t *__restrict__ type_map, const T *__restrict__ params,
@@ -563,8 +581,9 @@ dp_embed_bwd(const int32_t *__restrict__ list_neigh, const T *__restrict__ idr,
     const int S = P.nslots;
     const int nall = P.natoms + P.nghost;
     const long long total = (long long)P.batch * P.natoms;
-    for (long long t = (long long)blockIdx.x * nwarps + warp; t < total;
-         t += (long long)gridDim.x * nwarps) {
+    const int atoms = SPLIT ? 1 : nwarps, stride = SPLIT ? 32 * nwarps : 32;
+    for (long long t = (long long)blockIdx.x * atoms + (SPLIT ? 0 : warp); t < total;
+         t += (long long)gridDim.x * atoms) {
         const int b = (int)(t / P.natoms);
         const int i = (int)(t - (long long)b * P.natoms);
         const int ti = type_map[i];
@@ -579,7 +598,7 @@ dp_embed_bwd(const int32_t *__restrict__ list_neigh, const T *__restrict__ idr,
             const T *avg = davg + 4 * ti;
             const T *sd = dstd + 4 * ti;
             T fi[3] = {T(0), T(0), T(0)};
-            for (int c0 = 0; c0 < cnt; c0 += 32) {
+            for (int c0 = SPLIT ? 32 * warp : 0; c0 < cnt; c0 += stride) {
                 const int k = c0 + lane;
                 int tj = 0, j = -1;
                 T R = T(0), px = T(0), py = T(0), pz = T(0);
@@ -677,9 +696,23 @@ dp_embed_bwd(const int32_t *__restrict__ list_neigh, const T *__restrict__ idr,
         }
 #pragma unroll
         for (int q = 0; q < 9; ++q) vir[q] = warp_sum(vir[q]);
-        if (lane == 0)
+        if (SPLIT) {
+            double *part = reinterpret_cast<double *>(act_all);     // [nwarps][9], activations done
+            __syncthreads();
+            if (lane == 0)
+#pragma unroll
+                for (int q = 0; q < 9; ++q) part[warp * 9 + q] = vir[q];
+            __syncthreads();
+            if (threadIdx.x < 9) {
+                double v = 0.0;
+                for (int w = 0; w < nwarps; ++w) v += part[w * 9 + threadIdx.x];
+                atom_vir[t * 9 + threadIdx.x] = v;
+            }
+            __syncthreads();
+        } else if (lane == 0) {
 #pragma unroll
             for (int q = 0; q < 9; ++q) atom_vir[t * 9 + q] = vir[q];
+        }
         __syncwarp();
     }
 }
@@ -800,25 +833,32 @@ int launch_eval(int mode, const matpl_dp_model *M, const EvalParams &P,
         dp_pad<T><<<(nnet + 3) / 4, 128, 0, s>>>(params, davg, dstd, pad, P.ntypes, P);
     }
 
-    // A small batch runs one-warp blocks, so that its atoms reach every SM before any SM takes a
-    // second: FP64 issues two lanes a clock per SM, and 108 atoms in four-warp blocks kept 27 SMs
-    // busy (forward + backward 1.5 ms, 0.97 ms in one-warp blocks).  Above 16 atoms per SM both
-    // shapes fill the chip and the four-warp block stages the nets a quarter as often.
-    const int nwarps = total < 16LL * device_sms() ? 1 : kWarps;
-    const long long nwarp_blocks = (total + nwarps - 1) / nwarps;
-    const int gridw = (int)std::max<long long>(
-        1, std::min<long long>(nwarp_blocks, (long long)device_sms() * 8 * (kWarps / nwarps)));
+    // A small batch runs one atom per block, so that its atoms reach every SM before any SM takes a
+    // second: FP64 issues two lanes a clock per SM, and 108 atoms in four-warp blocks of four atoms
+    // kept 27 SMs busy (forward + backward 1.5 ms, 0.97 ms in one-warp blocks).  In FP64 the block's
+    // four warps then share the atom: one warp fills less than half of the pipe (0.97 -> 0.33 ms).
+    // Above 16 atoms per SM both shapes fill the chip and the four-atom block stages the nets a
+    // quarter as often.
     const size_t wbytes = sizeof(T) * (size_t)nnet * EmbOff::SIZE;
     const bool ws_ok = wbytes <= 128 * 1024 && P.ctab == nullptr;   // tables: no net weights
     const size_t wpart = ws_ok ? wbytes : 0;
-    const size_t smem_f = wpart + sizeof(T) * nwarps * 32 * (E + 1 + 4) +
-                          sizeof(int) * nwarps * P.nslots;
-    const size_t smem_b = wpart + sizeof(T) * nwarps * (2 * E * 32 + NA) +
-                          sizeof(int) * nwarps * P.nslots;
-    auto kf = P.ctab ? dp_embed_fwd<T, false, true>
-                     : (ws_ok ? dp_embed_fwd<T, true, false> : dp_embed_fwd<T, false, false>);
-    auto kb = P.ctab ? dp_embed_bwd<T, false, true>
-                     : (ws_ok ? dp_embed_bwd<T, true, false> : dp_embed_bwd<T, false, false>);
+    auto smem_of = [&](int w, bool backward) {
+        return wpart + sizeof(T) * w * (backward ? 2 * E * 32 + NA : 32 * (E + 1 + 4)) +
+               sizeof(int) * w * P.nslots;
+    };
+    const bool small = total < 16LL * device_sms();
+    const bool split = small && sizeof(T) == 8 && smem_of(kWarps, true) <= 220 * 1024;
+    const int nwarps = small && !split ? 1 : kWarps, atoms = small ? 1 : kWarps;
+    const int gridw = (int)std::max<long long>(
+        1, std::min<long long>((total + atoms - 1) / atoms, (long long)device_sms() * 8 * (kWarps / nwarps)));
+    const size_t smem_f = smem_of(nwarps, false), smem_b = smem_of(nwarps, true);
+    constexpr bool D = sizeof(T) == 8;
+    auto kf = P.ctab ? (split ? dp_embed_fwd<T, false, true, D> : dp_embed_fwd<T, false, true, false>)
+              : ws_ok ? (split ? dp_embed_fwd<T, true, false, D> : dp_embed_fwd<T, true, false, false>)
+                      : (split ? dp_embed_fwd<T, false, false, D> : dp_embed_fwd<T, false, false, false>);
+    auto kb = P.ctab ? (split ? dp_embed_bwd<T, false, true, D> : dp_embed_bwd<T, false, true, false>)
+              : ws_ok ? (split ? dp_embed_bwd<T, true, false, D> : dp_embed_bwd<T, true, false, false>)
+                      : (split ? dp_embed_bwd<T, false, false, D> : dp_embed_bwd<T, false, false, false>);
     int st = MATPL_OK;
     // compressed models take the SIMT embedding kernels in every form (the table polynomial is
     // no GEMM); the mixed forms still run the fitting nets on the tensor cores

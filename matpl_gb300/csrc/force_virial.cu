@@ -62,45 +62,61 @@ __global__ void force_scatter(const int32_t *__restrict__ nl, const T *__restric
     }
 }
 
+// Forces and vectors of 32 slots staged per warp, then 27 lanes add three pairs at a time, lane
+// (pair, component): the nine components of a neighbor's row are one 72-byte run (36 in FP32), so
+// an atomic instruction touches about 10 sectors instead of 32, and a lane always sums the same
+// component of the total.  6,000 atoms, 45 pairs each, FP64: 155 -> 47 us.
 template <typename T>
-__global__ void virial_scatter(const int32_t *__restrict__ nl, const T *__restrict__ dE,
-                               const T *__restrict__ Rij, const T *__restrict__ Rd,
-                               T *__restrict__ virial, T *__restrict__ atom_virial, int batch,
-                               int natoms, int nslots, int nghost) {
+__global__ void __launch_bounds__(kThreads)
+virial_scatter(const int32_t *__restrict__ nl, const T *__restrict__ dE,
+               const T *__restrict__ Rij, const T *__restrict__ Rd, T *__restrict__ virial,
+               T *__restrict__ atom_virial, int batch, int natoms, int nslots, int nghost) {
     // Each block covers slots of one configuration at a time; per-block FP64 partials.
-    __shared__ double part[kThreads / 32][9];
+    __shared__ double part[kThreads / 32][27];
+    __shared__ T fr_all[kThreads / 32][32][7];       // f, Rij of the occupied slots (odd rows)
+    __shared__ int j_all[kThreads / 32][32];
     const long long per_b = (long long)natoms * nslots;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    T(*fr)[7] = fr_all[warp];
+    int *jn = j_all[warp];
+    const int q = lane % 9, sub = lane / 9;          // lane < 27: component, pair of three
     for (int b = 0; b < batch; ++b) {
-        double acc[9];
+        double acc = 0.0;
+        T *base = atom_virial + (long long)b * (natoms + nghost) * 9;
+        for (long long t0 = ((long long)blockIdx.x * kThreads + warp * 32); t0 < per_b;
+             t0 += (long long)gridDim.x * kThreads) {
+            const long long s = b * per_b + t0 + lane;
+            const int j = t0 + lane < per_b ? nl[s] : -1;
+            const unsigned mk = __ballot_sync(0xffffffffu, j >= 0);
+            if (!mk) continue;
+            if (j >= 0) {
+                const int at = __popc(mk & ((1u << lane) - 1u));
+                T f[3];
+                slot_f(dE, Rd, s, f);
+                jn[at] = j;
 #pragma unroll
-        for (int q = 0; q < 9; ++q) acc[q] = 0.0;
-        for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < per_b;
-             t += (long long)gridDim.x * blockDim.x) {
-            const long long s = b * per_b + t;
-            const int j = nl[s];
-            if (j < 0) continue;
-            T f[3];
-            slot_f(dE, Rd, s, f);
-            const T r[3] = {Rij[s * 3], Rij[s * 3 + 1], Rij[s * 3 + 2]};
-            T *dst = atom_virial + ((long long)b * (natoms + nghost) + j) * 9;
-#pragma unroll
-            for (int a = 0; a < 3; ++a)
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const T v = f[a] * r[c];   // calculateVirial.cu:80 order: (Ri_d comp, Rij comp)
-                    atomicAdd(dst + 3 * a + c, v);
-                    acc[3 * a + c] += (double)v;
+                for (int a = 0; a < 3; ++a) {
+                    fr[at][a] = f[a];
+                    fr[at][3 + a] = Rij[s * 3 + a];
                 }
+            }
+            __syncwarp();
+            const int n = __popc(mk);
+            if (lane < 27)
+                for (int p = sub; p < n; p += 3) {
+                    // calculateVirial.cu:80 order: (Ri_d component, Rij component)
+                    const T v = fr[p][q / 3] * fr[p][3 + q % 3];
+                    atomicAdd(base + (long long)jn[p] * 9 + q, v);
+                    acc += (double)v;
+                }
+            __syncwarp();
         }
-#pragma unroll
-        for (int q = 0; q < 9; ++q) acc[q] = warp_sum(acc[q]);
-        if (lane == 0)
-            for (int q = 0; q < 9; ++q) part[warp][q] = acc[q];
+        if (lane < 27) part[warp][lane] = acc;
         __syncthreads();
         if (threadIdx.x < 9) {
             double v = 0.0;
-            for (int w = 0; w < kThreads / 32; ++w) v += part[w][threadIdx.x];
+            for (int w = 0; w < kThreads / 32; ++w)
+                for (int u = 0; u < 3; ++u) v += part[w][9 * u + threadIdx.x];
             atomicAdd(virial + b * 9 + threadIdx.x, (T)v);
         }
         __syncthreads();
@@ -127,13 +143,13 @@ __global__ void force_grad_kernel(const int32_t *__restrict__ nl, const T *__res
             const T *p = gF + (b * (natoms + nghost) + (j % natoms)) * 3;
             gj[0] = p[0]; gj[1] = p[1]; gj[2] = p[2];
         }
+        // FP64: the pipe issues two lanes a clock, so the two dot products are one with the
+        // difference (15 operations instead of 28)
+        const T g0 = gj[0] - gc[0], g1 = gj[1] - gc[1], g2 = gj[2] - gc[2];
         const T *d = Rd + s * 12;
 #pragma unroll
-        for (int w = 0; w < 4; ++w) {
-            const T dw0 = d[3 * w], dw1 = d[3 * w + 1], dw2 = d[3 * w + 2];
-            grad[s * 4 + w] = -(gc[0] * dw0 + gc[1] * dw1 + gc[2] * dw2)
-                              + (gj[0] * dw0 + gj[1] * dw1 + gj[2] * dw2);
-        }
+        for (int w = 0; w < 4; ++w)
+            grad[s * 4 + w] = g0 * d[3 * w] + g1 * d[3 * w + 1] + g2 * d[3 * w + 2];
     }
 }
 

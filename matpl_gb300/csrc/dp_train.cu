@@ -49,6 +49,7 @@ template <typename T>
 __device__ __forceinline__ void load_nets(T *dst, const T *__restrict__ params, int nnet,
                                           int stride) {
     const bool tr = stride == NetS::BWD;
+#pragma unroll 8
     for (int q = threadIdx.x; q < nnet * stride; q += blockDim.x) {
         const int n = q / stride, e = q - n * stride;
         const T *src = params + (long long)n * EmbOff::SIZE;
@@ -199,7 +200,7 @@ __device__ __forceinline__ void layer_res(const T *w, int OW, int OB, int OD, T 
 constexpr int kFwdRow = 2 * kStg + 8;
 
 template <typename T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1)
 dp_dual_fwd(const int32_t *__restrict__ list_neigh, const T *__restrict__ idr,
             const int32_t *__restrict__ type_map, const T *__restrict__ params,
             const T *__restrict__ davg, const T *__restrict__ dstd, const T *__restrict__ gF,

@@ -162,24 +162,6 @@ __device__ __forceinline__ void pre_act(const T *w, int OW, int OB, const T *x, 
     }
 }
 
-// acc[i] += sum_o W[i][o] z[o] and accd[i] += sum_o W[i][o] zd[o] (z, zd in shared memory;
-// WT: the padded transpose W^T[out][in] in the NetS copy).
-template <typename T>
-__device__ __forceinline__ void back_act(const T *WT, const T *z, const T *zd, T acc[E],
-                                         T accd[E]) {
-#pragma unroll 1
-    for (int o = 0; o < E; ++o) {
-        const T zo = z[o], zdo = zd[o];
-        T wc[kRp];
-        ld_row(WT + o * kRp, wc);
-#pragma unroll
-        for (int i = 0; i < E; ++i) {
-            acc[i] += wc[i] * zo;
-            accd[i] += wc[i] * zdo;
-        }
-    }
-}
-
 // Residual layer applied in place to a lane's shared-memory rows x, xd:
 // x <- tanh(x W + b) dt + x with its tangent.
 template <typename T>
@@ -296,19 +278,57 @@ struct Stage {
     static constexpr int ROW = 5 * kStg + 3;          // + (s, sdot, pad)
 };
 
-// Adds, for every net present among the chunk's lanes, sum over its lanes of the layer's
-// gradient terms into the CTA accumulator gacc (shared).  lay = 1 or 2 (W/b/dt of that layer),
-// lay = 0: W0 / b0 from (s, sdot).
+// The backward kernel gives every 32 slots to two warps: each has 13 of the 25 columns of every layer,
+// from o0 = 0 or 12 (both have column 12, so that rows stay 16-byte aligned), and they meet at a named
+// barrier between the steps.
+constexpr int kHalf = 13, kHalfRow = 16;
+
+__device__ __forceinline__ void ld_half(const float *p, float v[kHalfRow]) {
+#pragma unroll
+    for (int q = 0; q < kHalfRow / 4; ++q) {
+        const float4 f = reinterpret_cast<const float4 *>(p)[q];
+        v[4 * q] = f.x; v[4 * q + 1] = f.y; v[4 * q + 2] = f.z; v[4 * q + 3] = f.w;
+    }
+}
+__device__ __forceinline__ void ld_half(const double *p, double v[kHalfRow]) {
+#pragma unroll
+    for (int q = 0; q < kHalfRow / 2; ++q) {
+        const double2 f = reinterpret_cast<const double2 *>(p)[q];
+        v[2 * q] = f.x; v[2 * q + 1] = f.y;
+    }
+}
+
+// h[q] += sum_i x[i] W[i][o0 + q] and the same for the second stream (rows x, xd in shared memory)
 template <typename T>
-__device__ __forceinline__ void reduce_layer(const T *stg, int nv, int ti, int ntypes,
-                                             unsigned tmask[], int lay, T *gacc, int lane) {
+__device__ __forceinline__ void half_gemm(const T *W, const T *x, const T *xd, T h[kHalf],
+                                          T hd[kHalf]) {
+#pragma unroll 5
+    for (int i = 0; i < E; ++i) {
+        const T xi = x[i], xdi = xd[i];
+        T w[kHalfRow];
+        ld_half(W + i * kRp, w);
+#pragma unroll
+        for (int q = 0; q < kHalf; ++q) {
+            h[q] += xi * w[q];
+            hd[q] += xdi * w[q];
+        }
+    }
+}
+
+// Adds, for every net present among the chunk's lanes, sum over its lanes of the layer's
+// gradient terms into the CTA accumulator gacc (shared), each warp of the pair its columns.
+// lay = 1 or 2 (W/b/dt of that layer), lay = 0: W0 / b0 from (s, sdot).
+template <typename T>
+__device__ __forceinline__ void reduce_layer(const T *stg, int ti, int ntypes, unsigned tmask[],
+                                             int lay, T *gacc, int lane, int half) {
     for (int tj = 0; tj < ntypes; ++tj) {
         const unsigned mk = tmask[tj];
         if (!mk) continue;
         const int lo = __ffs(mk) - 1, hi = 32 - __clz(mk);
         T *g = gacc + (ti * ntypes + tj) * EmbOff::SIZE;
+        const int e = lane + 32 * half;
         if (lay == 0) {
-            for (int e = lane; e < 2 * E; e += 32) {
+            if (e < 2 * E) {
                 const int o = e < E ? e : e - E;
                 T acc = T(0);
                 for (int l = lo; l < hi; ++l) {
@@ -323,17 +343,19 @@ __device__ __forceinline__ void reduce_layer(const T *stg, int nv, int ti, int n
         const int OW = lay == 1 ? EmbOff::W1 : EmbOff::W2;
         const int OB = lay == 1 ? EmbOff::B1 : EmbOff::B2;
         const int OD = lay == 1 ? EmbOff::DT1 : EmbOff::DT2;
-        // weight gradient sum_l x_i zb_o + xd_i zdb_o: lane < 25 owns a 5 x 5 block (i, o), so
-        // a row costs 20 shared loads for 50 FMAs
-        static_assert(E == 25, "5 x 5 register blocks of the 25 x 25 weight gradient");
-        if (lane < 25) {
-            const int i0 = 5 * (lane / 5), o0 = 5 * (lane % 5);
-            T acc[5][5];
+        // weight gradient sum_l x_i zb_o + xd_i zdb_o: a lane owns 5 rows i and 4 columns o (5 at
+        // the end) of the warp's 12 or 13, for one half of the slots (alternate slots would share
+        // banks), so a slot costs 20 shared loads for 50 FMAs
+        static_assert(E == 25, "blocks of the 25 x 25 weight gradient");
+        const int mid = (lo + hi + 1) / 2;
+        const int par = lane / 15, u = lane - 15 * par, i0 = 5 * (u / 3), o0 = 12 * half + 4 * (u % 3);
+        T acc[5][5];
 #pragma unroll
-            for (int a = 0; a < 5; ++a)
+        for (int a = 0; a < 5; ++a)
 #pragma unroll
-                for (int b = 0; b < 5; ++b) acc[a][b] = T(0);
-            for (int l = lo; l < hi; ++l) {
+            for (int b = 0; b < 5; ++b) acc[a][b] = T(0);
+        if (par < 2)
+            for (int l = par ? mid : lo; l < (par ? hi : mid); ++l) {
                 const T *r = stg + l * Stage::ROW;
                 T xi[5], xdi[5], zo[5], zdo[5];
 #pragma unroll
@@ -348,22 +370,30 @@ __device__ __forceinline__ void reduce_layer(const T *stg, int nv, int ti, int n
 #pragma unroll
                     for (int b = 0; b < 5; ++b) acc[a][b] += xi[a] * zo[b] + xdi[a] * zdo[b];
             }
+        __syncwarp();
+        const int nb = half && u % 3 == 2 ? 5 : 4;
 #pragma unroll
-            for (int a = 0; a < 5; ++a)
+        for (int a = 0; a < 5; ++a)
 #pragma unroll
-                for (int b = 0; b < 5; ++b) atomicAdd(g + OW + (i0 + a) * E + o0 + b, acc[a][b]);
-        }
-        for (int o = lane; o < 2 * E; o += 32) {
-            T acc = T(0);
-            const int col = o < E ? Stage::ZB + o : Stage::Q + (o - E);
-            for (int l = lo; l < hi; ++l) acc += stg[l * Stage::ROW + col];
-            atomicAdd(g + (o < E ? OB + o : OD + (o - E)), acc);
+            for (int b = 0; b < 5; ++b) {
+                const T v = acc[a][b] + __shfl_down_sync(0xffffffffu, acc[a][b], 15);
+                if (lane < 15 && b < nb) atomicAdd(g + OW + (i0 + a) * E + o0 + b, v);
+            }
+        if (e < 2 * E) {
+            T sum = T(0);
+            const int col = e < E ? Stage::ZB + e : Stage::Q + (e - E);
+            for (int l = lo; l < hi; ++l) sum += stg[l * Stage::ROW + col];
+            atomicAdd(g + (e < E ? OB + e : OD + (e - E)), sum);
         }
     }
 }
 
+// Bound: latency and the broadcast loads of the weights (a load serves two FMAs).  The staged rows of 32
+// slots (17 KB) and the nets leave room for eight such groups on an SM: with a warp each 8 warps
+// issued in 37 % of the cycles, so two warps share a group.  64
+// configurations of 32 to 512 atoms, two elements, 63 neighbors each, FP32: 1268 -> 1140 us.
 template <typename T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(sizeof(T) == 4 ? 512 : 256)
 dp_dual_bwd(const int32_t *__restrict__ list_neigh, const T *__restrict__ idr,
             const int32_t *__restrict__ type_map, const T *__restrict__ params,
             const T *__restrict__ davg, const T *__restrict__ dstd, const T *__restrict__ gF,
@@ -371,27 +401,30 @@ dp_dual_bwd(const int32_t *__restrict__ list_neigh, const T *__restrict__ idr,
             T *__restrict__ grad, TrainParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int nnet = P.ntypes * P.ntypes, S = P.nslots;
-    const int warps = blockDim.x >> 5;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int pairs = blockDim.x >> 6, pair = threadIdx.x >> 6;
+    const int lane = threadIdx.x & 31, half = (threadIdx.x >> 5) & 1, o0 = 12 * half;
     T *wsm = reinterpret_cast<T *>(smem_raw);                   // weights (NetS layout)
     T *gacc = wsm + nnet * NetS::BWD;                           // gradient accumulator
-    T *stg_all = gacc + nnet * EmbOff::SIZE;                    // [warps][32][Stage::ROW]
-    T *ab_all = stg_all + warps * 32 * Stage::ROW;              // [warps][2][NA]
-    int *list_all = reinterpret_cast<int *>(ab_all + warps * 2 * NA);
-    T *stg = stg_all + warp * 32 * Stage::ROW;
-    T *ab = ab_all + warp * 2 * NA;
-    int *list = list_all + warp * S;
+    T *stg_all = gacc + nnet * EmbOff::SIZE;                    // [pairs][32][Stage::ROW]
+    T *ab_all = stg_all + pairs * 32 * Stage::ROW;              // [pairs][2][NA]
+    int *list_all = reinterpret_cast<int *>(ab_all + pairs * 2 * NA);
+    T *stg = stg_all + pair * 32 * Stage::ROW;
+    T *ab = ab_all + pair * 2 * NA;
+    int *list = list_all + pair * S;
     T *my = stg + lane * Stage::ROW;
+    auto meet = [&] { asm volatile("bar.sync %0, 64;" ::"r"(1 + pair) : "memory"); };
     load_nets(wsm, params, nnet, NetS::BWD);
     for (int q = threadIdx.x; q < nnet * EmbOff::SIZE; q += blockDim.x) gacc[q] = T(0);
     __syncthreads();
     const T k = (T)P.inv_mT;
     const long long total = (long long)P.batch * P.natoms;
-    for (long long t = (long long)blockIdx.x * warps + warp; t < total;
-         t += (long long)gridDim.x * warps) {
+    for (long long t = (long long)blockIdx.x * pairs + pair; t < total;
+         t += (long long)gridDim.x * pairs) {
         const int ti = type_map[t % P.natoms];
         if (ti < 0 || ti >= P.ntypes || !((P.present_mask >> ti) & 1)) continue;
         const long long cfg0 = (t / P.natoms) * P.natoms;
+        meet();                                  // the last atom's list and ab are done with
+        // both warps write the same list and the same values of ab
         const int cnt = occupied_slots(list_neigh + t * S, S, P.m, P.present_mask, list, lane);
         for (int e = lane; e < NA; e += 32) {
             ab[e] = Abar[t * NA + e] * k;
@@ -413,86 +446,99 @@ dp_dual_bwd(const int32_t *__restrict__ list_neigh, const T *__restrict__ idr,
 #pragma unroll
             for (int q = 0; q < 16; ++q)
                 tmask[q] = q < P.ntypes ? __ballot_sync(0xffffffffu, valid && tj == q) : 0u;
-            const int nv = min(32, cnt - c0);
             const T *w = wsm + (ti * P.ntypes + tj) * NetS::BWD;
             // seeds: Gbar = k (R Abar + Rdot Adbar), Gdotbar = k R Adbar (k folded into ab)
-            T gb[E], gdb[E];
+            T gb[kHalf], gdb[kHalf];
 #pragma unroll
-            for (int p = 0; p < E; ++p) {
+            for (int q = 0; q < kHalf; ++q) {
+                const int p = o0 + q;
                 T s0 = T(0), s1 = T(0);
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     s0 += rh[c] * ab[c * E + p] + rd[c] * ab[NA + c * E + p];
                     s1 += rh[c] * ab[NA + c * E + p];
                 }
-                gb[p] = valid ? s0 : T(0);
-                gdb[p] = valid ? s1 : T(0);
+                gb[q] = valid ? s0 : T(0);
+                gdb[q] = valid ? s1 : T(0);
             }
-            __syncwarp();
+            auto layer0_half = [&] {
+#pragma unroll
+                for (int q = 0; q < kHalf; ++q) {
+                    const int o = o0 + q;
+                    const T x = dev_tanh(rh[0] * w[NetS::W0 + o] + w[NetS::B0 + o]);
+                    my[Stage::X + o] = x;
+                    my[Stage::XD + o] = (T(1) - x * x) * rd[0] * w[NetS::W0 + o];
+                }
+            };
+            T h[kHalf], hd[kHalf];
+            auto pre = [&](int OW, int OB) {
+#pragma unroll
+                for (int q = 0; q < kHalf; ++q) {
+                    h[q] = w[OB + o0 + q];
+                    hd[q] = T(0);
+                }
+                half_gemm(w + OW + o0, my + Stage::X, my + Stage::XD, h, hd);
+            };
+            // tanh, its adjoints and the dt term of a residual layer's columns
+            auto reverse = [&](int OD) {
+#pragma unroll
+                for (int q = 0; q < kHalf; ++q) {
+                    const int o = o0 + q;
+                    const T th = dev_tanh(h[q]);
+                    const T dt = w[OD + o], g = T(1) - th * th;
+                    const T tb = gb[q] * dt, tdb = gdb[q] * dt;
+                    my[Stage::Q + o] = gb[q] * th + gdb[q] * g * hd[q];
+                    my[Stage::ZB + o] = g * (tb - T(2) * th * hd[q] * tdb);
+                    my[Stage::ZDB + o] = g * tdb;
+                }
+            };
+            meet();
             // ---- layer 2: recompute its input x1 (staged in X / XD), reverse through it
-            {
-                T x[E], xd[E];
-                layer0(w, rh[0], rd[0], x, xd);
+            layer0_half();
+            meet();
+            pre(NetS::M1, NetS::B1);
+            meet();                                              // x0 read by both
 #pragma unroll
-                for (int p = 0; p < E; ++p) { my[Stage::X + p] = x[p]; my[Stage::XD + p] = xd[p]; }
+            for (int q = 0; q < kHalf; ++q) {
+                const int o = o0 + q;
+                const T th = dev_tanh(h[q]), dt = w[NetS::DT1 + o];
+                if (q == kHalf - 1 && half == 0) continue;       // column 12: one update
+                my[Stage::X + o] = th * dt + my[Stage::X + o];
+                my[Stage::XD + o] = (T(1) - th * th) * hd[q] * dt + my[Stage::XD + o];
             }
-            layer_res(w, NetS::M1, NetS::B1, NetS::DT1, my + Stage::X, my + Stage::XD);
-            {
-                T h[E], hd[E];
-                pre_act(w, NetS::M2, NetS::B2, my + Stage::X, my + Stage::XD, h, hd);
-#pragma unroll
-                for (int o = 0; o < E; ++o) {
-                    const T t2 = dev_tanh(h[o]);
-                    const T dt = w[NetS::DT2 + o], g = T(1) - t2 * t2;
-                    const T tb = gb[o] * dt, tdb = gdb[o] * dt;
-                    my[Stage::Q + o] = gb[o] * t2 + gdb[o] * g * hd[o];
-                    my[Stage::ZB + o] = g * (tb - T(2) * t2 * hd[o] * tdb);
-                    my[Stage::ZDB + o] = g * tdb;
-                }
-            }
+            meet();
+            pre(NetS::M2, NetS::B2);
+            reverse(NetS::DT2);
+            meet();
             // x1bar = Gbar + W2 zb2, x1dotbar = Gdotbar + W2 zdb2
-            back_act(w + NetS::M2T, my + Stage::ZB, my + Stage::ZDB, gb, gdb);
+            half_gemm(w + NetS::M2T + o0, my + Stage::ZB, my + Stage::ZDB, gb, gdb);
             __syncwarp();
-            reduce_layer(stg, nv, ti, P.ntypes, tmask, 2, gacc, lane);
-            __syncwarp();
+            reduce_layer(stg, ti, P.ntypes, tmask, 2, gacc, lane, half);
+            meet();
             // ---- layer 1: recompute its input x0 (staged), reverse through it
-            {
-                T x[E], xd[E];
-                layer0(w, rh[0], rd[0], x, xd);
-#pragma unroll
-                for (int p = 0; p < E; ++p) { my[Stage::X + p] = x[p]; my[Stage::XD + p] = xd[p]; }
-            }
-            {
-                T h[E], hd[E];
-                pre_act(w, NetS::M1, NetS::B1, my + Stage::X, my + Stage::XD, h, hd);
-#pragma unroll
-                for (int o = 0; o < E; ++o) {
-                    const T t1 = dev_tanh(h[o]);
-                    const T dt = w[NetS::DT1 + o], g = T(1) - t1 * t1;
-                    const T tb = gb[o] * dt, tdb = gdb[o] * dt;
-                    my[Stage::Q + o] = gb[o] * t1 + gdb[o] * g * hd[o];
-                    my[Stage::ZB + o] = g * (tb - T(2) * t1 * hd[o] * tdb);
-                    my[Stage::ZDB + o] = g * tdb;
-                }
-            }
-            back_act(w + NetS::M1T, my + Stage::ZB, my + Stage::ZDB, gb, gdb);
+            layer0_half();
+            meet();
+            pre(NetS::M1, NetS::B1);
+            reverse(NetS::DT1);
+            meet();
+            half_gemm(w + NetS::M1T + o0, my + Stage::ZB, my + Stage::ZDB, gb, gdb);
             __syncwarp();
-            reduce_layer(stg, nv, ti, P.ntypes, tmask, 1, gacc, lane);
-            __syncwarp();
+            reduce_layer(stg, ti, P.ntypes, tmask, 1, gacc, lane, half);
+            meet();
             // ---- layer 0: x0 = tanh(s W0 + b0), x0dot = (1 - x0^2) sdot W0 (x0 still staged)
 #pragma unroll
-            for (int o = 0; o < E; ++o) {
+            for (int q = 0; q < kHalf; ++q) {
+                const int o = o0 + q;
                 const T x0 = my[Stage::X + o];
                 const T g = T(1) - x0 * x0;
                 const T zd0 = rd[0] * w[NetS::W0 + o];
-                my[Stage::ZB + o] = g * (gb[o] - T(2) * x0 * zd0 * gdb[o]);
-                my[Stage::ZDB + o] = g * gdb[o];
+                my[Stage::ZB + o] = g * (gb[q] - T(2) * x0 * zd0 * gdb[q]);
+                my[Stage::ZDB + o] = g * gdb[q];
             }
             my[5 * kStg] = rh[0];
             my[5 * kStg + 1] = rd[0];
-            __syncwarp();
-            reduce_layer(stg, nv, ti, P.ntypes, tmask, 0, gacc, lane);
-            __syncwarp();
+            meet();
+            reduce_layer(stg, ti, P.ntypes, tmask, 0, gacc, lane, half);
         }
     }
     __syncthreads();
@@ -951,7 +997,7 @@ int launch(bool backward, const matpl_dp_model *md, int batch, int natoms, int n
             (const T *)md->dstd, (const T *)gF, (const T *)gV, (T *)out0, (T *)out1, P);
         return check_launch("matpl_dp_dual_forward");
     }
-    int warps = 8;
+    int warps = sizeof(T) == 4 ? 8 : 4;               // groups of 32 slots, two warps each
     auto need = [&](int w) {
         return wb + wbytes + (size_t)w * 32 * Stage::ROW * sizeof(T) +
                (size_t)w * 2 * NA * sizeof(T) + (size_t)w * nslots * sizeof(int);
@@ -964,7 +1010,7 @@ int launch(bool backward, const matpl_dp_model *md, int batch, int natoms, int n
     if (grid > (long long)sms * 4) grid = (long long)sms * 4;
     cudaMemsetAsync(out0, 0, wbytes, s);
     ProfScope ps("dp_dual_bwd", s);
-    dp_dual_bwd<T><<<(int)grid, 32 * warps, smem, s>>>(
+    dp_dual_bwd<T><<<(int)grid, 64 * warps, smem, s>>>(
         ln, (const T *)idr, tm, (const T *)md->params, (const T *)md->davg, (const T *)md->dstd,
         (const T *)gF, (const T *)gV, (const T *)a_in, (const T *)ad_in, (T *)out0, P);
     return check_launch("matpl_dp_dual_backward");

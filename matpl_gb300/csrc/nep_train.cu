@@ -1206,7 +1206,7 @@ extern "C" int matpl_nep_feat_grad(int dtype, int part, int mode, int natoms, in
     cudaStream_t s = as_stream(stream);
     const size_t esz = dtype == MATPL_F64 ? sizeof(double) : sizeof(float);
     const bool tabled = feat_tabled(dtype, natoms, ntypes, n_max, n_base);
-    if (cudaMemsetAsync(workspace, 0, need, s) != cudaSuccess ||
+    if ((need && cudaMemsetAsync(workspace, 0, need, s) != cudaSuccess) ||
         ((natoms == 0 || max_nn == 0) &&
          cudaMemsetAsync(dc, 0, esz * ntypes * ntypes * n_max * n_base, s) != cudaSuccess)) {
         set_error("matpl_nep_feat_grad: memset failed");

@@ -179,13 +179,21 @@ class DP(torch.nn.Module):
         return m
 
     def _grouped_perm(self, tmap: torch.Tensor, present: List[int]) -> torch.Tensor:
-        key = (tmap.data_ptr(), tmap.numel(), tuple(present))
-        p = self._perm_cache.get(key)
-        if p is None:
-            tl = tmap.long()
-            p = torch.cat([torch.nonzero(tl == t).flatten() for t in present])
-            self._perm_cache = {key: p}
-        return p
+        """Atoms of ``tmap`` (the caller's type map) grouped by element, on the model's device."""
+        def grouped(m):
+            return torch.cat([torch.nonzero(m == t).flatten() for t in present])
+        if not tmap.is_cuda:
+            return grouped(tmap).to(self.packed.device)
+        # finding them on the device costs a synchronisation, so the last map's order is kept; the
+        # entry holds the map, so that no other tensor can take that address, and an in-place write
+        # changes the version
+        key = (tmap.data_ptr(), tuple(tmap.shape), tmap.stride(), tmap.dtype,
+               None if tmap.is_inference() else tmap._version, tuple(present))
+        hit = self._perm_cache.get(key)
+        if hit is None:
+            hit = (grouped(tmap), tmap)
+            self._perm_cache = {key: hit}
+        return hit[0]
 
     @_lib.on_device
     def evaluate(self, list_neigh: torch.Tensor, Imagetype_map: torch.Tensor, present: List[int],
@@ -246,7 +254,7 @@ class DP(torch.nn.Module):
         present = self.present_types(atom_type)
         tm = Imagetype_map.to(device=ImageDR.device, dtype=torch.int32)
         r = self.evaluate(list_neigh, tm, present, ImageDR, int(nghost))
-        perm = self._grouped_perm(tm, present)
+        perm = self._grouped_perm(Imagetype_map, present)
         Ei = r["Ei_atom"][:, perm]
         Etot = r["Etot"].to(self.dtype).unsqueeze(-1)
         Egroup = None

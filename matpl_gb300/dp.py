@@ -116,6 +116,36 @@ def per_type_stats(arr: torch.Tensor, ntypes: int) -> torch.Tensor:
     return a[:, 0, :].contiguous()
 
 
+class LastMap:
+    """What a type map on the device leads to (finding its atoms by element costs a host read and
+    several launches), kept until another map comes.  Neither a tensor's address nor its version says
+    that it holds the same values (inference tensors, ``.data``, a graph's replay), so a copy of the
+    map is kept and compared: one host read per call.  An entry belongs to the stream it was made
+    on: no other stream reads its tensors before they are written or after they are freed."""
+
+    def __init__(self):
+        self._entry = None
+
+    def get(self, tmap: torch.Tensor, key, make):
+        from .ops import _stream
+        key = (_stream(tmap.device), key)
+        e = self._entry
+        if e is not None and e[0] == key and e[1].shape == tmap.shape and \
+                e[1].dtype == tmap.dtype and e[1].device == tmap.device and torch.equal(e[1], tmap):
+            return e[2]
+        with torch.inference_mode(False):         # the entry serves calls in every mode
+            value = make(tmap)
+            self._entry = (key, tmap.detach().clone(), value)
+        return value
+
+    def last(self, tmap: torch.Tensor, key):
+        """The value of the last call, for a capture (which cannot read on the host)."""
+        e = self._entry
+        if e is None or e[0][1] != key or e[1].shape != tmap.shape:
+            raise _lib.MatplError("make one call with this type map before capturing it in a graph")
+        return e[2]
+
+
 class DP(torch.nn.Module):
     """Inference DP se_e2_a on GB300.
 
@@ -145,7 +175,7 @@ class DP(torch.nn.Module):
         dstd = torch.as_tensor(dstd)
         self.register_buffer("davg4", per_type_stats(davg, cfg.ntypes).to(dev, self.dtype))
         self.register_buffer("dstd4", per_type_stats(dstd, cfg.ntypes).to(dev, self.dtype))
-        self._perm_cache = {}
+        self._order = LastMap()
         # compressed model: the tables of compress.build_table (ckpt_compress.py) in the fused
         # kernels instead of the embedding nets
         self.compress = compress
@@ -181,19 +211,21 @@ class DP(torch.nn.Module):
     def _grouped_perm(self, tmap: torch.Tensor, present: List[int]) -> torch.Tensor:
         """Atoms of ``tmap`` (the caller's type map) grouped by element, on the model's device."""
         def grouped(m):
-            return torch.cat([torch.nonzero(m == t).flatten() for t in present])
+            return [torch.nonzero(m == t).flatten() for t in present]
         if not tmap.is_cuda:
-            return grouped(tmap).to(self.packed.device)
-        # finding them on the device costs a synchronisation, so the last map's order is kept; the
-        # entry holds the map, so that no other tensor can take that address, and an in-place write
-        # changes the version
-        key = (tmap.data_ptr(), tuple(tmap.shape), tmap.stride(), tmap.dtype,
-               None if tmap.is_inference() else tmap._version, tuple(present))
-        hit = self._perm_cache.get(key)
-        if hit is None:
-            hit = (grouped(tmap), tmap)
-            self._perm_cache = {key: hit}
-        return hit[0]
+            return torch.cat(grouped(tmap)).to(self.packed.device)
+        key = (self.packed.device, tuple(present))
+        if torch.cuda.is_current_stream_capturing():
+            # a graph reads the map at every replay: the element counts are those of the last call,
+            # the order is found in the graph (a stable sort puts an element's atoms first)
+            counts = self._order.last(tmap, key)[1]
+            return torch.cat([torch.sort((tmap != t).to(torch.int32), stable=True)[1][:n]
+                              for t, n in zip(present, counts)])
+
+        def make(m):
+            parts = grouped(m)
+            return torch.cat(parts), [q.numel() for q in parts]
+        return self._order.get(tmap, key, make)[0]
 
     @_lib.on_device
     def evaluate(self, list_neigh: torch.Tensor, Imagetype_map: torch.Tensor, present: List[int],

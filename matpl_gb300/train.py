@@ -447,6 +447,7 @@ class FusedTrainer:
         self.davg4 = self.evaluator.davg4
         self.dstd4 = self.evaluator.dstd4
         self._present = None
+        self._order = _dp.LastMap()
         compiled = (list(cfg.fit_sizes) == [_dp.F] * 3 + [1] and cfg.M2 == _dp.M2 and
                     list(cfg.emb_sizes) == [_dp.E] * 3)
         self.fit_kernel = bool(fit_kernel) and compiled
@@ -493,11 +494,15 @@ class FusedTrainer:
 
     def _type_index(self, tm32: torch.Tensor, present, B: int):
         """Atom rows of the [B*N] batch grouped by present element, b-major inside each
-        element ([B, n] blocks), and each element's (start, count) in that order (cached per
-        type map and batch size: one host sync when it changes)."""
-        key = (self._tm_src.data_ptr(), tm32.numel(), tuple(present), B)
-        if getattr(self, "_tidx_key", None) != key:
-            tl = tm32.long()
+        element ([B, n] blocks), and each element's (start, count) in that order: of the map's
+        values, found once until they change; in a capture, those of the last call."""
+        key = (tuple(present), B)
+        if tm32.is_cuda and torch.cuda.is_current_stream_capturing():
+            self._order.last(tm32, key)
+            return self._rows, self._blocks
+
+        def make(tm):
+            tl = tm.long()
             N = tl.numel()
             base = torch.arange(B, device=tl.device).reshape(B, 1) * N
             rows, blocks, off = [], {}, 0
@@ -507,9 +512,8 @@ class FusedTrainer:
                 rows.append((base + idx.reshape(1, n)).reshape(-1))
                 blocks[ti] = (off, n)
                 off += B * n
-            self._rows = torch.cat(rows).contiguous()
-            self._blocks = blocks
-            self._tidx_key = key
+            return torch.cat(rows).contiguous(), blocks
+        self._rows, self._blocks = self._order.get(tm32, key, make)
         return self._rows, self._blocks
 
     def _loss_and_backward(self, batch: dict, w_f: float, w_e: float):
@@ -523,7 +527,6 @@ class FusedTrainer:
         idr = batch["ImageDR"]
         idr = idr if idr.dtype == model.dtype and idr.is_contiguous() else idr.to(model.dtype).contiguous()
         tm32 = batch["type_map"]
-        self._tm_src = tm32
         tm32 = tm32 if tm32.dtype == torch.int32 else tm32.to(device=dev, dtype=torch.int32).contiguous()
         present = [cfg.atom_type.index(int(a)) for a in batch["atom_type"]
                    if int(a) in cfg.atom_type]

@@ -13,7 +13,7 @@ and ``train_step`` applies the reference loss (dp_trainer.py:172-272 with ``dp_l
 prefactors, ``src/loss/dploss.py:18-66``) and the optimizer.  Configurations are evaluated one
 composition cluster at a time, as the reference does (``_classify_batchs``, dp_trainer.py:536).
 """
-from typing import Dict, List, Optional, Sequence
+from typing import Dict, List, NamedTuple, Optional, Sequence
 
 import torch
 
@@ -516,6 +516,14 @@ class FusedTrainer:
         self._rows, self._blocks = self._order.get(tm32, key, make)
         return self._rows, self._blocks
 
+    def _present_types(self, batch):
+        cfg = self.model.cfg
+        return [cfg.atom_type.index(int(a)) for a in batch["atom_type"] if int(a) in cfg.atom_type]
+
+    def _type_index_of(self, batch):
+        tm = batch["type_map"].to(device=batch["list_neigh"].device, dtype=torch.int32)
+        return self._type_index(tm.contiguous(), self._present_types(batch), batch["list_neigh"].shape[0])
+
     def _loss_and_backward(self, batch: dict, w_f: float, w_e: float):
         """Steps 1-5 with device tensors only (no host synchronisation once the type index is
         cached): returns (loss, le, lf) as 0-d tensors and leaves the gradients in .grad."""
@@ -528,8 +536,7 @@ class FusedTrainer:
         idr = idr if idr.dtype == model.dtype and idr.is_contiguous() else idr.to(model.dtype).contiguous()
         tm32 = batch["type_map"]
         tm32 = tm32 if tm32.dtype == torch.int32 else tm32.to(device=dev, dtype=torch.int32).contiguous()
-        present = [cfg.atom_type.index(int(a)) for a in batch["atom_type"]
-                   if int(a) in cfg.atom_type]
+        present = self._present_types(batch)
         self._present = present
         rows, blocks = self._type_index(tm32, present, B)
         # 1. E, F with the current parameters
@@ -610,11 +617,13 @@ class FusedTrainer:
 
 
 class GraphedTrainer:
-    """The fused training step (FusedTrainer) captured once per batch shape in a CUDA graph:
-    loss, both dual kernels, the fitting part, the backward and the optimizer update replay as
-    one graph launch, so the step costs no host work beyond copying the batch into the graph's
-    static buffers.  The optimizer must keep its state on the device (torch.optim.Adam /
-    AdamW with capturable=True, or SGD).  ``step`` returns the loss as a device tensor."""
+    """The fused training step (FusedTrainer) captured in a CUDA graph, once per batch shape and
+    element counts: loss, both dual kernels, the fitting part, the backward and the optimizer update
+    replay as one graph launch, so the step costs no host work beyond copying the batch into the
+    graph's static buffers and one read that tells whether its type map is the last one (if it is
+    not, the element-grouped rows are found again).  The optimizer must keep its state on the device
+    (torch.optim.Adam / AdamW with capturable=True, or SGD).  ``step`` returns the loss as a
+    device tensor."""
 
     KEYS = ("list_neigh", "ImageDR", "type_map", "Etot", "Force")
 
@@ -622,7 +631,7 @@ class GraphedTrainer:
                  w_f: float = 1.0, w_e: float = 1.0, warmup: int = 3):
         self.tr, self.opt = trainer, optimizer
         self.w_f, self.w_e, self.warmup = w_f, w_e, warmup
-        self.graphs = {}
+        self.graphs = {}            # shape key -> captured steps, the last used first
 
     def _keys(self, batch):
         return self.KEYS + (("config_of_atom",) if "config_of_atom" in batch else ())
@@ -637,25 +646,55 @@ class GraphedTrainer:
                 self.opt.zero_grad(set_to_none=True)
                 self.tr._loss_and_backward(static, self.w_f, self.w_e)
                 self.opt.step()
+            if self.warmup:                         # the graph's own: ``step`` writes them
+                self.tr._rows = self.tr._rows.clone()
         torch.cuda.current_stream().wait_stream(side)
         g = torch.cuda.CUDAGraph()
         self.opt.zero_grad(set_to_none=True)
         with torch.cuda.graph(g, stream=side):   # the warm-up's workspaces are reused
             loss, le, lf = self.tr._loss_and_backward(static, self.w_f, self.w_e)
             self.opt.step()
-        # the graph reads the trainer's type-grouped rows and this stream's workspaces by
-        # address: a later batch shape replaces them, so they live as long as the graph does
-        keep = (self.tr._rows, ops.stream_workspaces(side.cuda_stream))
-        return g, static, loss, keep
+        # the graph reads its type-grouped rows and this stream's workspaces by address: a later
+        # batch shape replaces them, so they live as long as the graph does
+        return _Captured(g, static, loss, self.tr._rows, getattr(self.tr, "_blocks", None),
+                         ops.stream_workspaces(side.cuda_stream))
+
+    @staticmethod
+    def _load(captured, batch, keys):
+        for k in keys:
+            if batch[k].data_ptr() != captured.static[k].data_ptr():
+                captured.static[k].copy_(batch[k], non_blocking=True)
 
     def step(self, batch):
         keys = self._keys(batch)
         key = tuple(tuple(batch[k].shape) for k in keys) + (tuple(batch["atom_type"]),)
-        if key not in self.graphs:
-            self.graphs[key] = self._capture(batch)
-        g, static, loss, _ = self.graphs[key]
-        for k in keys:
-            if batch[k].data_ptr() != static[k].data_ptr():
-                static[k].copy_(batch[k], non_blocking=True)
-        g.replay()
-        return loss
+        steps = self.graphs.setdefault(key, [])
+        hit = steps[0] if steps else None
+        if hit is not None:
+            # the copies are queued first: they run while the host waits for the comparison
+            self._load(hit, batch, [k for k in keys if k != "type_map"])
+            held = hit.static["type_map"]
+            if not torch.equal(held, batch["type_map"].to(held.device, held.dtype)):
+                rows, blocks = self.tr._type_index_of(batch)
+                hit = next((c for c in steps if c.blocks == blocks), None)
+                if hit is not None:
+                    self._load(hit, batch, keys)
+                    hit.rows.copy_(rows)
+                    steps.remove(hit)
+                    steps.insert(0, hit)
+        if hit is None:
+            hit = self._capture(batch)
+            steps.insert(0, hit)
+        hit.graph.replay()
+        return hit.loss
+
+
+class _Captured(NamedTuple):
+    """One captured step: the graph, its inputs and loss, the element-grouped rows it reads with
+    their (start, count) per element, and what else has to live as long."""
+    graph: object
+    static: dict
+    loss: torch.Tensor
+    rows: torch.Tensor
+    blocks: dict
+    keep: tuple

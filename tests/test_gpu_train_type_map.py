@@ -50,3 +50,27 @@ def test_refilled_type_map(fit_kernel):
             assert (x is None) == (y is None), k
             if x is not None:      # the weight gradients are summed by FP64 atomics
                 assert float((x - y).abs().max()) <= 1e-10 * max(1e-3, float(y.abs().max())), k
+
+
+def test_graphed_step_follows_the_type_map():
+    """Captured steps on batches of one shape with other orders and counts of the elements: every
+    update from the first weights (SGD, rate 1) is minus an eager step's gradient of that batch."""
+    make, data = batches()
+    model = make()
+    tr = train.GraphedTrainer(train.FusedTrainer(model), torch.optim.SGD(model.parameters(), lr=1.0))
+    first = {k: model.param(k).detach().clone() for k in model.names}
+    for k in (0, 1, 2, 0, 2, 1, 1, 0):
+        tr.step(data[k])                       # a capture makes warm-up updates too
+        with torch.no_grad():
+            for name in model.names:
+                model.param(name).copy_(first[name])
+        fresh = make()
+        want = train.FusedTrainer(fresh).loss_and_backward(data[k])[0]
+        assert float(tr.step(data[k])) == pytest.approx(want, rel=1e-12), k
+        with torch.no_grad():
+            for name in model.names:
+                y = fresh.param(name).grad
+                y = torch.zeros_like(first[name]) if y is None else y
+                x = first[name] - model.param(name)
+                assert float((x - y).abs().max()) <= 1e-10 * max(1e-3, float(y.abs().max())), (k, name)
+                model.param(name).copy_(first[name])

@@ -225,13 +225,16 @@ class GraphedNepTrainer:
         g = torch.cuda.CUDAGraph()
         self.opt.zero_grad(set_to_none=True)
         with torch.cuda.graph(g, stream=side):   # the warm-up's workspaces are reused
-            loss = self.loss(static, tindex)
+            # part of the graph: a later batch of this shape may order its elements differently
+            tindex_g = self.model.type_index(static["type_map"])
+            loss = self.loss(static, tindex_g)
             loss.backward()
             self.opt.step()
-        # the graph reads the one-hot type index and the module caches' tensors (image index,
-        # row of ones) by address, so they live as long as the graph does
+        # the graph reads the module caches' tensors (image index, row of ones) by address, so they
+        # live as long as the graph does
         counts = tuple(int(c) for c in static["num_atom"].tolist())
-        keep = (tindex, nep_ops.cached_image_index(counts, tindex.device), splitk.cached_ones())
+        keep = (tindex, tindex_g, nep_ops.cached_image_index(counts, tindex.device),
+                splitk.cached_ones())
         return g, static, loss, keep
 
     def step(self, batch) -> torch.Tensor:

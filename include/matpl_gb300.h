@@ -31,10 +31,10 @@ typedef enum {
     MATPL_ERR_UNSUPPORTED = 5   /* model shape outside the compiled kernels */
 } matpl_status;
 
-/* Codes a kernel writes to err_dev (0 = fine). */
+/* Codes a kernel writes to err_dev (0 = fine; of several, the largest stays). */
 #define MATPL_KERR_NEIGHBOR_OVERFLOW 1   /* a type block exceeds m (NeighConst.f90:75-78) */
 #define MATPL_KERR_BAD_TYPE 2            /* atom type index outside [0, ntypes) */
-#define MATPL_KERR_TIMEOUT 3             /* a bounded tensor-core completion wait gave up */
+#define MATPL_KERR_TIMEOUT 3             /* a bounded wait inside a kernel gave up: outputs invalid */
 #define MATPL_KERR_TABLE_RANGE 6         /* compressed model: s outside the table's grid */
 
 /* Compute forms.  MIXED*: FP32 data, embedding and fitting GEMMs on the tensor cores

@@ -28,7 +28,7 @@ env_stats_kernel(int batch, int natoms, int nslots, int ntypes, const int32_t *_
         const int b = (int)(ba / natoms), a = (int)(ba - (long long)b * natoms);
         const int t = type_map[a];
         if (t < 0 || t >= ntypes) {
-            if (lane == 0) atomicOr(err, MATPL_KERR_BAD_TYPE);
+            if (lane == 0) atomicMax(err, MATPL_KERR_BAD_TYPE);
             continue;
         }
         double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};

@@ -77,7 +77,7 @@ __device__ __forceinline__ void cmp_forward(const T *__restrict__ tab, int k, T 
                           : __fadd_rn((float)P.csmax, __fmul_rn(__fmul_rn(fi, (float)P.cdx), 10.f));
     const T f2 = s - (T)xk;
     if (idx < 0 || idx >= P.crows) {
-        if (P.err) atomicOr(P.err, MATPL_KERR_TABLE_RANGE);
+        if (P.err) atomicMax(P.err, MATPL_KERR_TABLE_RANGE);
         idx = idx < 0 ? 0 : P.crows - 1;
     }
     const T *c = tab + ((long long)k * P.crows + idx) * E * P.cnc;

@@ -75,14 +75,14 @@ lmp_neighbors(int inum, int nall, const int *__restrict__ ilist, Lists lists,
     for (long long ii = gw; ii < inum; ii += nw) {
         const int i = ilist[ii];
         if (i < 0 || i >= inum) {  // rows are indexed by i (pair_matpl.cpp:589)
-            if (lane == 0) atomicOr(err, MATPL_KERR_BAD_COUNT);
+            if (lane == 0) atomicMax(err, MATPL_KERR_BAD_COUNT);
             continue;
         }
         const int til = type[i] - 1;
         const int ti = (til >= 0 && til < ntypes_lmp) ? type_to_model[til] : -1;
         if (lane == 0) {
             type_map[ii] = ti;
-            if (ti < 0 || ti >= nt) atomicOr(err, MATPL_KERR_BAD_TYPE);
+            if (ti < 0 || ti >= nt) atomicMax(err, MATPL_KERR_BAD_TYPE);
         }
         const double xi = x[3 * i], yi = x[3 * i + 1], zi = x[3 * i + 2];
         int cnt[16];
@@ -108,11 +108,11 @@ lmp_neighbors(int inum, int nall, const int *__restrict__ ilist, Lists lists,
                     rsq = da(da(dm(dx, dx), dm(dy, dy)), dm(dz, dz));
                     keep = ubits(rsq) <= rc2_bits;
                     if (keep && (tj < 0 || tj >= nt)) {
-                        atomicOr(err, MATPL_KERR_BAD_TYPE);
+                        atomicMax(err, MATPL_KERR_BAD_TYPE);
                         keep = false;
                     }
                 } else {
-                    atomicOr(err, MATPL_KERR_BAD_COUNT);
+                    atomicMax(err, MATPL_KERR_BAD_COUNT);
                 }
             }
             if (keep && ubits(rsq) < local_min) local_min = ubits(rsq);
@@ -158,7 +158,7 @@ lmp_neighbors(int inum, int nall, const int *__restrict__ ilist, Lists lists,
             local_min = v < local_min ? v : local_min;
         }
         if (lane == 0) {
-            if (over) atomicOr(err, MATPL_KERR_NEIGHBOR_OVERFLOW);
+            if (over) atomicMax(err, MATPL_KERR_NEIGHBOR_OVERFLOW);
             if (local_min < ubits(kNoPair)) atomicMin(min_rsq, local_min);
         }
     }

@@ -336,7 +336,7 @@ nep_eval_kernel(EvalArgs A, long long atoms_per_run) {
         }
         if (ti < 0 || ti >= L.ntypes) {
             if (lane == 0) {
-                atomicOr(A.err, MATPL_KERR_BAD_TYPE);
+                atomicMax(A.err, MATPL_KERR_BAD_TYPE);
                 if (!A.feats) reinterpret_cast<T *>(A.Ei)[i] = T(0);
             }
             if (!A.feats) {
@@ -358,9 +358,9 @@ nep_eval_kernel(EvalArgs A, long long atoms_per_run) {
             int tj = -1;
             if (j >= 0 && j < A.natoms) {
                 tj = (int)A.type_map[j];
-                if (tj < 0 || tj >= L.ntypes) { atomicOr(A.err, MATPL_KERR_BAD_TYPE); tj = -1; }
+                if (tj < 0 || tj >= L.ntypes) { atomicMax(A.err, MATPL_KERR_BAD_TYPE); tj = -1; }
             } else if (j >= A.natoms) {
-                atomicOr(A.err, MATPL_KERR_BAD_COUNT);
+                atomicMax(A.err, MATPL_KERR_BAD_COUNT);
             }
             return tj;
         };
@@ -677,7 +677,7 @@ nep_eval_kernel(EvalArgs A, long long atoms_per_run) {
         __syncwarp();
     }
     if (!A.feats) flush_energy(A, frame, e_frame, lane);
-    if (!in_turn && lane == 0) atomicOr(A.err, MATPL_KERR_TIMEOUT);
+    if (!in_turn && lane == 0) atomicMax(A.err, MATPL_KERR_TIMEOUT);
 }
 
 __global__ void nep_frame_start(const long long *__restrict__ num_atom, int nframes,
@@ -690,7 +690,7 @@ __global__ void nep_frame_start(const long long *__restrict__ num_atom, int nfra
             a += num_atom[f] > 0 ? num_atom[f] : 0;
         }
         start[nframes] = a;
-        if (a != natoms) atomicOr(err, MATPL_KERR_BAD_COUNT);
+        if (a != natoms) atomicMax(err, MATPL_KERR_BAD_COUNT);
     }
 }
 

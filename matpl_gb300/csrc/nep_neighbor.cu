@@ -200,7 +200,7 @@ nepnb_setup(const long long *__restrict__ num_atom, const double *__restrict__ b
             sum += chunk;
         }
         bad |= sum != natoms;
-        if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(err, MATPL_KERR_BAD_COUNT);
+        if (__any_sync(0xffffffffu, bad) && lane == 0) atomicMax(err, MATPL_KERR_BAD_COUNT);
     }
     __syncthreads();
     for (int f = warp; f < nframes; f += nwarps) {
@@ -231,7 +231,7 @@ nepnb_setup(const long long *__restrict__ num_atom, const double *__restrict__ b
         const int rep = (int)num_cell[3 * f + k];
         if (lane < 3) {
             F.rep[k] = rep;
-            if (rep < 1) atomicOr(err, MATPL_KERR_BAD_BOX);
+            if (rep < 1) atomicMax(err, MATPL_KERR_BAD_BOX);
         }
         const bool single = __all_sync(0xffffffffu, rep == 1);
         // cell geometry of the original cell: columns of box_orig are the lattice vectors; lane k
@@ -481,7 +481,7 @@ __device__ __forceinline__ void count_types(const SearchArgs &A, const WarpLists
             if (in_r) atomicAdd(&W.tcount[t2], 1);
             if (in_a) atomicAdd(&W.tcount[A.ntypes + t2], 1);
         } else {
-            atomicOr(A.err, MATPL_KERR_BAD_TYPE);
+            atomicMax(A.err, MATPL_KERR_BAD_TYPE);
         }
     }
 }
@@ -629,7 +629,7 @@ __global__ void __launch_bounds__(128, 6) nepnb_search(SearchArgs A, int warps_p
         if (A.skin && F.mode != 0) {   // the skin list is built for cell-list frames only
             if (lane == 0) {
                 A.skin_cnt[n1] = 0;
-                atomicOr(A.err, MATPL_KERR_BAD_BOX);
+                atomicMax(A.err, MATPL_KERR_BAD_BOX);
             }
             continue;
         }
@@ -848,7 +848,7 @@ __global__ void __launch_bounds__(128, 6) nepnb_search(SearchArgs A, int warps_p
         if (A.skin) {
             if (lane == 0) {
                 A.skin_cnt[n1] = min(cr, A.max_r);
-                if (cr > A.max_r) atomicOr(A.err, MATPL_KERR_NEIGHBOR_OVERFLOW);
+                if (cr > A.max_r) atomicMax(A.err, MATPL_KERR_NEIGHBOR_OVERFLOW);
             }
             continue;
         }
@@ -856,7 +856,7 @@ __global__ void __launch_bounds__(128, 6) nepnb_search(SearchArgs A, int warps_p
         if (lane == 0) {
             A.NN_r[n1] = cr;
             A.NN_a[n1] = ca;
-            if (cr > A.max_r || ca > A.max_a) atomicOr(A.err, MATPL_KERR_NEIGHBOR_OVERFLOW);
+            if (cr > A.max_r || ca > A.max_a) atomicMax(A.err, MATPL_KERR_NEIGHBOR_OVERFLOW);
         }
     }
 }
@@ -1014,7 +1014,7 @@ nepnb_skin_filter(const NepFrame *__restrict__ fr, int nframes, long long natoms
                     const float zf = H[6] * f0 + H[7] * f1 + H[8] * f2;
                     pass = xf * xf + yf * yf + zf * zf < pre2;
                 } else {
-                    atomicOr(err, MATPL_KERR_BAD_COUNT);
+                    atomicMax(err, MATPL_KERR_BAD_COUNT);
                 }
             }
             const unsigned b = __ballot_sync(0xffffffffu, pass);
@@ -1049,7 +1049,7 @@ nepnb_skin_filter(const NepFrame *__restrict__ fr, int nframes, long long natoms
         if (lane == 0) {
             NN_r[n1] = cr;
             NN_a[n1] = ca;
-            if (cr > max_r || ca > max_a) atomicOr(err, MATPL_KERR_NEIGHBOR_OVERFLOW);
+            if (cr > max_r || ca > max_a) atomicMax(err, MATPL_KERR_NEIGHBOR_OVERFLOW);
         }
     }
 }
@@ -1090,7 +1090,7 @@ nepnb_skin_filter_compact(long long natoms, const int *__restrict__ skin,
                     in_r = r2 < rc2_r;
                     in_a = r2 < rc2_a;
                 } else {
-                    atomicOr(err, MATPL_KERR_BAD_COUNT);
+                    atomicMax(err, MATPL_KERR_BAD_COUNT);
                 }
             }
             const unsigned br = __ballot_sync(0xffffffffu, in_r);
@@ -1113,7 +1113,7 @@ nepnb_skin_filter_compact(long long natoms, const int *__restrict__ skin,
         if (lane == 0) {
             NN_r[n1] = cr;
             NN_a[n1] = ca;
-            if (cr > max_r || ca > max_a) atomicOr(err, MATPL_KERR_NEIGHBOR_OVERFLOW);
+            if (cr > max_r || ca > max_a) atomicMax(err, MATPL_KERR_NEIGHBOR_OVERFLOW);
         }
     }
 }

@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(32 * kFeatWarps, sizeof(T) == 4 && NM <= 5 ? 8
     for (long long i = gw; i < A.natoms; i += nw) {
         const int ti = (int)A.type[i];
         if (ti < 0 || ti >= T_) {
-            if (lane == 0) atomicOr(A.err, MATPL_KERR_BAD_TYPE);
+            if (lane == 0) atomicMax(A.err, MATPL_KERR_BAD_TYPE);
             if (MODE != kBwd && lane < n_) static_cast<T *>(A.q)[i * A.ldQ + lane] = T(0);
             if (MODE == kBwd && A.grad_d12) zero_slots<T>(A, i, 0, lane);
             continue;
@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(32 * kFeatWarps, sizeof(T) == 4 && NM <= 5 ? 8
             const long long ps = i * A.nn + slot;
             const long long j = slot < A.nn ? A.NL[ps] : -1;
             const bool ok = j >= 0 && j < A.natoms;
-            if (j >= A.natoms) atomicOr(A.err, MATPL_KERR_BAD_COUNT);
+            if (j >= A.natoms) atomicMax(A.err, MATPL_KERR_BAD_COUNT);
             if (!__any_sync(0xffffffffu, ok)) {
                 if (MODE == kBwd && A.grad_d12) zero_slots<T>(A, i, base, lane);
                 break;
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(32 * kFeatWarps, sizeof(T) == 4 && NM <= 5 ? 8
             if (ok) {
                 tj = (int)A.type[j];
                 if (tj < 0 || tj >= T_) {
-                    atomicOr(A.err, MATPL_KERR_BAD_TYPE);
+                    atomicMax(A.err, MATPL_KERR_BAD_TYPE);
                     tj = -1;
                 }
             }
@@ -441,7 +441,7 @@ __global__ void __launch_bounds__(32 * kFeatWarps, sizeof(T) == 4 && NM <= 5 ? 5
     for (long long i = gw; i < A.natoms; i += nw) {
         const int ti = (int)A.type[i];
         if (ti < 0 || ti >= T_) {
-            if (lane == 0) atomicOr(A.err, MATPL_KERR_BAD_TYPE);
+            if (lane == 0) atomicMax(A.err, MATPL_KERR_BAD_TYPE);
             if (MODE != kBwd)
                 for (int e = lane; e < n_ * (A.l3 + four + five); e += 32)
                     static_cast<T *>(A.q)[i * A.ldQ + e] = T(0);
@@ -458,12 +458,12 @@ __global__ void __launch_bounds__(32 * kFeatWarps, sizeof(T) == 4 && NM <= 5 ? 5
             const long long ps = i * A.nn + slot;
             const long long j = slot < A.nn ? A.NL[ps] : -1;
             bool ok = j >= 0 && j < A.natoms;
-            if (j >= A.natoms) atomicOr(A.err, MATPL_KERR_BAD_COUNT);
+            if (j >= A.natoms) atomicMax(A.err, MATPL_KERR_BAD_COUNT);
             if (!__any_sync(0xffffffffu, ok)) break;
             nvalid = base + 32;
             int tj = ok ? (int)A.type[j] : -1;
             if (ok && (tj < 0 || tj >= T_)) {
-                atomicOr(A.err, MATPL_KERR_BAD_TYPE);
+                atomicMax(A.err, MATPL_KERR_BAD_TYPE);
                 ok = false;
             }
             T f[KM], df[KM], g[NM], gp[NM], ux, uy, uz, ri;
@@ -781,7 +781,7 @@ nep_cgrad_kernel(int part, int natoms, int ntypes, int nmax, int K,
         int ta = -1;
         if (a < natoms) {
             const long long v = type_map[a];
-            if (v < 0 || v >= ntypes) atomicOr(err, MATPL_KERR_BAD_TYPE);
+            if (v < 0 || v >= ntypes) atomicMax(err, MATPL_KERR_BAD_TYPE);
             else ta = (int)v;
         }
         tsh[threadIdx.x] = ta;
@@ -880,7 +880,7 @@ nep_force_virial_kernel(int natoms, int nn, int nimages, const long long *__rest
         if (i >= natoms) break;
         const long long b = image_of[i];
         if (b < 0 || b >= nimages) {
-            if (lane == 0) atomicOr(err, MATPL_KERR_BAD_COUNT);
+            if (lane == 0) atomicMax(err, MATPL_KERR_BAD_COUNT);
             continue;
         }
         if (b != cur) {                 // a frame boundary inside the warp's atoms
@@ -901,7 +901,7 @@ nep_force_virial_kernel(int natoms, int nn, int nimages, const long long *__rest
             for (int c = 0; c < 3; ++c) f[c] = e0 * (x[c] / r) + dE[4 * q + 1 + c];
             const long long j = NL[q];
             if (j >= natoms) {
-                atomicOr(err, MATPL_KERR_BAD_COUNT);
+                atomicMax(err, MATPL_KERR_BAD_COUNT);
             } else if (j >= 0) {
 #pragma unroll
                 for (int c = 0; c < 3; ++c) atomicAdd(force + 3 * j + c, f[c]);
@@ -966,7 +966,7 @@ nep_force_virial_grad_kernel(int natoms, int nn, int nimages, const long long *_
 #pragma unroll
                 for (int a = 0; a < 3; ++a) u[a] = -gF[3 * i + a];
                 if (j >= natoms) {
-                    atomicOr(err, MATPL_KERR_BAD_COUNT);
+                    atomicMax(err, MATPL_KERR_BAD_COUNT);
                 } else if (j >= 0) {
 #pragma unroll
                     for (int a = 0; a < 3; ++a) u[a] += gF[3 * j + a];
@@ -975,7 +975,7 @@ nep_force_virial_grad_kernel(int natoms, int nn, int nimages, const long long *_
             if (gV) {
                 const long long b = image_of[i];
                 if (b < 0 || b >= nimages) {
-                    atomicOr(err, MATPL_KERR_BAD_COUNT);
+                    atomicMax(err, MATPL_KERR_BAD_COUNT);
                 } else {
 #pragma unroll
                     for (int a = 0; a < 3; ++a)

@@ -51,7 +51,7 @@ nep_zbl_kernel(long long natoms, int nn, int nimages, const long long *__restric
          i += nw) {
         const long long ti = type_map[i];
         if (ti < 0 || ti >= ntypes) {
-            if (lane == 0) atomicOr(err, MATPL_KERR_BAD_TYPE);
+            if (lane == 0) atomicMax(err, MATPL_KERR_BAD_TYPE);
             continue;
         }
         double e_sum = 0.0, v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
@@ -64,12 +64,12 @@ nep_zbl_kernel(long long natoms, int nn, int nimages, const long long *__restric
             const T r = (T)Ri[4 * q];
             if (!(r > T(0) && r <= zb)) continue;
             if (j >= natoms) {
-                atomicOr(err, MATPL_KERR_BAD_COUNT);
+                atomicMax(err, MATPL_KERR_BAD_COUNT);
                 continue;
             }
             const long long tj = type_map[j];
             if (tj < 0 || tj >= ntypes) {
-                atomicOr(err, MATPL_KERR_BAD_TYPE);
+                atomicMax(err, MATPL_KERR_BAD_TYPE);
                 continue;
             }
             any = true;
@@ -117,7 +117,7 @@ nep_zbl_kernel(long long natoms, int nn, int nimages, const long long *__restric
             for (int a = 0; a < 3; ++a) atomicAdd(force + 3 * i + a, fi[a]);
             const long long b = image_of[i];
             if (b < 0 || b >= nimages) {
-                atomicOr(err, MATPL_KERR_BAD_COUNT);
+                atomicMax(err, MATPL_KERR_BAD_COUNT);
             } else {
                 if (Etot) atomicAdd(Etot + b, e_sum);
 #pragma unroll

@@ -383,12 +383,19 @@ class NEP(torch.nn.Module):
                 nep_ops.nep_zbl(self.cfg.zbl, self.cfg.atom_type, i64(NL_angular),
                                 f64(Ri_angular), tm, counts, out["Ei"], out["Etot"], out["Force"],
                                 out["Virial"])
-        if self.check_errors:
-            code = int(self.err.item())
-            if code:
-                self.err.zero_()
-                raise _lib.MatplError(f"matpl_nep_eval kernel error code {code}")
+        self._check()
         return out
+
+    def _check(self):
+        from . import _lib
+        code = int(self.err.item()) if self.check_errors else 0
+        if code:
+            self.err.zero_()
+            what = {_lib.KERR_BAD_TYPE: "atom type outside the model",
+                    _lib.KERR_BAD_COUNT: "num_atom or a list index does not fit the atoms",
+                    _lib.KERR_TIMEOUT: "a wait between warps gave up; the outputs are invalid"}
+            raise _lib.MatplError(f"matpl_nep_eval kernel error code {code} "
+                                  f"({what.get(code, 'unknown')})")
 
     def _evaluate_compact(self, NN_r, NL_r, Ri_r, NN_a, NL_a, Ri_a, na, tm, ws, stream, out,
                           descriptor_only):
@@ -417,11 +424,7 @@ class NEP(torch.nn.Module):
                                          ptr(out["Ei"]), ptr(out["Etot"]), ptr(out["Force"]),
                                          ptr(out["Virial"]), ptr(ws), ws.numel(), stream),
               "matpl_nep_eval_compact")
-        if self.check_errors:
-            code = int(self.err.item())
-            if code:
-                self.err.zero_()
-                raise _lib.MatplError(f"matpl_nep_eval kernel error code {code}")
+        self._check()
         return out
 
     def descriptor(self, NN_radial, NL_radial, Ri_radial, NN_angular, NL_angular, Ri_angular,

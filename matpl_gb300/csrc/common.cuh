@@ -46,6 +46,16 @@ int require_current_device(const void *p, const char *what);
         if (matpl_dev_rc_ != MATPL_OK) return matpl_dev_rc_;                    \
     } while (0)
 
+// Lets `kernel` take `bytes` of dynamic shared memory on the current device.  The limit belongs to
+// the kernel and so to every host thread that launches it, and what a call needs depends on its
+// sizes: the limit is only ever raised, or one thread would lower it between another's request
+// and launch.
+cudaError_t allow_smem(const void *kernel, size_t bytes);
+template <typename K>
+cudaError_t allow_smem(K *kernel, size_t bytes) {
+    return allow_smem(reinterpret_cast<const void *>(kernel), bytes);
+}
+
 // Optional per-kernel timing (matpl_profile_begin / matpl_profile_collect): when enabled,
 // every launch site records a CUDA event pair on its own stream.
 bool profiling_enabled();

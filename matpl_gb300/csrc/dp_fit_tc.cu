@@ -555,7 +555,7 @@ int launch_fit_tc(bool fast, const float *A, const int32_t *type_map, const floa
     const long long cap = 2LL * device_sms();            // two resident CTAs per SM
     const int grid = (int)(ntiles < cap ? ntiles : cap);
     auto k = fast ? dp_fit_tc<true> : dp_fit_tc<false>;
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FIT_SMEM);
+    allow_smem(k, FIT_SMEM);
     ProfScope ps("dp_fit_tc", s);
     k<<<grid, FT, FIT_SMEM, s>>>(A, order, type_start, params, tiles, Ei, dA, err, batch, natoms,
                                  ntypes);

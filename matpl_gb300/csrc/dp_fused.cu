@@ -547,9 +547,8 @@ template <typename T, int R>
 int launch_fit(const T *A, const int32_t *type_map, const T *params, T *Ei, T *dA,
                const EvalParams &P, cudaStream_t s) {
     const size_t smem = sizeof(T) * (size_t)R * (NA + DIN + 4 * F);
-    if (cudaFuncSetAttribute(dp_fit<T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem) != cudaSuccess)
-        return check_launch("cudaFuncSetAttribute(dp_fit)");
+    if (allow_smem(dp_fit<T, R>, smem) != cudaSuccess)
+        return check_launch("shared memory of dp_fit");
     const long long ntiles = ((long long)P.batch * P.natoms + R - 1) / R;
     const int grid = (int)std::min<long long>(ntiles, (long long)device_sms() * 16);
     ProfScope ps("dp_fit", s);
@@ -864,8 +863,8 @@ int launch_eval(int mode, const matpl_dp_model *M, const EvalParams &P,
     // no GEMM); the mixed forms still run the fitting nets on the tensor cores
     const bool simt_embed = mode == MATPL_F32 || mode == MATPL_F64 || P.ctab != nullptr;
     if (simt_embed) {
-        cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_f);
-        cudaFuncSetAttribute(kb, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b);
+        allow_smem(kf, smem_f);
+        allow_smem(kb, smem_b);
         ProfScope ps("dp_embed_fwd", s);
         kf<<<gridw, nwarps * 32, smem_f, s>>>(list_neigh, idr, type_map, params, davg, dstd, pad, A, P);
     } else {

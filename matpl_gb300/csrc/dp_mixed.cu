@@ -986,13 +986,13 @@ int launch_mixed_embed(bool backward, const int32_t *list_neigh, const int32_t *
     const int grid = (int)std::min<long long>(ngroups, (long long)device_sms() * per_sm);
     if (!backward) {
         auto k = dp_embed_fwd_tc<SPLIT, FAST>;
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_smem(k, smem);
         ProfScope ps("dp_embed_fwd_tc", s);
         k<<<grid, TM, smem, s>>>(list_neigh, idr, type_map, params, wtiles, davg, dstd,
                                  pad_or_dA, A_or_force, err, P);
     } else {
         auto k = dp_embed_bwd_tc<SPLIT, FAST>;
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_smem(k, smem);
         ProfScope ps("dp_embed_bwd_tc", s);
         k<<<grid, TM, smem, s>>>(list_neigh, idr, type_map, params, wtiles, davg, dstd,
                                  pad_or_dA, A_or_force, atom_vir, err, P);

@@ -939,8 +939,7 @@ int launch_pad(bool backward, const matpl_dp_model *md, int batch, int natoms, i
     const long long nblk = (long long)sms * (16 / G);
     const int chunk = (int)(((long long)P.rows + nblk - 1) / nblk);
     const int grid = (P.rows + chunk - 1) / chunk;
-    cudaFuncSetAttribute(dp_pad_reduce<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)(sper * G));
+    allow_smem(dp_pad_reduce<T>, sper * G);
     {
         ProfScope ps("dp_pad_reduce", s);
         dp_pad_reduce<T><<<grid, 128 * G, sper * G, s>>>(tm, n_empty, (const T *)in, P, chunk,
@@ -988,7 +987,7 @@ int launch(bool backward, const matpl_dp_model *md, int batch, int natoms, int n
         while (warps > 1 && needf(warps) > 110 * 1024) --warps;
         const size_t smem = needf(warps);
         MATPL_REQUIRE(smem <= 220 * 1024, MATPL_ERR_UNSUPPORTED, "too many types for shared memory");
-        cudaFuncSetAttribute(dp_dual_fwd<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_smem(dp_dual_fwd<T>, smem);
         long long grid = (total + warps - 1) / warps;
         if (grid > (long long)sms * 8) grid = (long long)sms * 8;
         ProfScope ps("dp_dual_fwd", s);
@@ -1005,7 +1004,7 @@ int launch(bool backward, const matpl_dp_model *md, int batch, int natoms, int n
     while (warps > 1 && need(warps) > 220 * 1024) --warps;
     const size_t smem = need(warps);
     MATPL_REQUIRE(smem <= 220 * 1024, MATPL_ERR_UNSUPPORTED, "too many types for shared memory");
-    cudaFuncSetAttribute(dp_dual_bwd<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(dp_dual_bwd<T>, smem);
     long long grid = (total + warps - 1) / warps;
     if (grid > (long long)sms * 4) grid = (long long)sms * 4;
     cudaMemsetAsync(out0, 0, wbytes, s);

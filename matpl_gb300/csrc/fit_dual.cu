@@ -564,9 +564,8 @@ int run(long long nrows, const void *fit_params, const void *D, const void *Dd, 
     const long long cap = (long long)device_sms() * 2;
     if (g1 > cap) g1 = cap;
     const size_t smem = sizeof(T) * (size_t)kRowsSmem;
-    if (cudaFuncSetAttribute(fit_dual_rows<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem) != cudaSuccess)
-        return check_launch("cudaFuncSetAttribute(fit_dual_rows)");
+    if (allow_smem(fit_dual_rows<T>, smem) != cudaSuccess)
+        return check_launch("shared memory of fit_dual_rows");
     {
         ProfScope ps("dp_fit_dual", s);
         fit_dual_rows<T><<<(int)g1, 256, smem, s>>>(R);
@@ -578,9 +577,8 @@ int run(long long nrows, const void *fit_params, const void *D, const void *Dd, 
     MATPL_REQUIRE(chunks < (1LL << 31), MATPL_ERR_INVALID, "too many rows");
     constexpr int SUB = kSub<T>;
     const size_t smem_w = 2 * sizeof(T) * (size_t)(2 * SUB * (kKT + 1) + 2 * SUB * (kUT + 1));
-    if (cudaFuncSetAttribute(fit_dual_wgrad<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem_w) != cudaSuccess)
-        return check_launch("cudaFuncSetAttribute(fit_dual_wgrad)");
+    if (allow_smem(fit_dual_wgrad<T>, smem_w) != cudaSuccess)
+        return check_launch("shared memory of fit_dual_wgrad");
     {
         ProfScope ps("dp_fit_dual_wgrad", s);
         fit_dual_wgrad<T><<<dim3((unsigned)chunks, 10), 256, smem_w, s>>>(W);

@@ -680,14 +680,12 @@ static int neighbor_build(int batch, int natoms, int ntypes, int m_neigh, double
     const int S = ntypes * m_neigh;
     const size_t smem = (size_t)kWarps * (S * 4 * (out_dtype == MATPL_F64 ? 8 : 4) + nb_ints(S) * 4 + S);
     if (out_dtype == MATPL_F64) {
-        cudaFuncSetAttribute(nb_search<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
+        allow_smem(nb_search<double>, smem);
         nb_search<double><<<grid_for(na, kWarps), kWarps * 32, smem, s>>>(
             img, wpos, wpos32, type_map, cell_of, cell_start, cell_atoms, list_neigh, (double *)image_dr,
             num_neigh, err_dev, P);
     } else {
-        cudaFuncSetAttribute(nb_search<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
+        allow_smem(nb_search<float>, smem);
         nb_search<float><<<grid_for(na, kWarps), kWarps * 32, smem, s>>>(
             img, wpos, wpos32, type_map, cell_of, cell_start, cell_atoms, list_neigh, (float *)image_dr,
             num_neigh, err_dev, P);

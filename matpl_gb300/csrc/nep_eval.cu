@@ -836,9 +836,8 @@ int launch_eval(const EvalArgs &A0, cudaStream_t s) {
     if (nruns < sms * rpb) rpb = (int)std::max<long long>(1, (nruns + sms - 1) / sms);
     const int wpb = rpb << A.pair;
     const size_t smem = A.pair ? smem_pair : smem_of(wpb, A.warp_bytes);
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
-        return check_launch("cudaFuncSetAttribute(nep_eval)");
+    if (allow_smem(kern, smem) != cudaSuccess)
+        return check_launch("shared memory of nep_eval");
     const int grid = (int)((nruns + rpb - 1) / rpb);
     {
         ProfScope ps(A.feats ? "nep_descriptor" : "nep_eval", s);

@@ -1207,15 +1207,13 @@ int run(int nframes, long long natoms, const long long *num_atom, const long lon
     const int grid = blocks_for(natoms, wpb, device_sms() * 64);
     if (count_only) {
         if (typed) {
-            cudaFuncSetAttribute(nepnb_search<true, true>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            allow_smem(nepnb_search<true, true>, smem);
             nepnb_search<true, true><<<grid, 32 * wpb, smem, s>>>(A, wpb);
         } else {
             nepnb_search<true, false><<<grid, 32 * wpb, smem, s>>>(A, wpb);
         }
     } else {
-        cudaFuncSetAttribute(nepnb_search<false, false>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_smem(nepnb_search<false, false>, smem);
         nepnb_search<false, false><<<grid, 32 * wpb, smem, s>>>(A, wpb);
     }
     return check_launch(count_only ? "matpl_nep_maxneigh" : "matpl_nep_neighbor");
@@ -1275,8 +1273,7 @@ int run_skin_update(int nframes, long long natoms, const long long *num_atom, co
     while (wpb > 1 && per_warp * wpb > 96 * 1024) wpb >>= 1;
     const size_t smem = align_up(per_warp * wpb, 16);
     const int grid = blocks_for(natoms, wpb, device_sms() * 64);
-    cudaFuncSetAttribute(nepnb_search<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem);
+    allow_smem(nepnb_search<false, false>, smem);
     nepnb_search<false, false><<<grid, 32 * wpb, smem, s>>>(A, wpb);
     nepnb_gate_clear<<<1, 1, 0, s>>>(gate, nbuild);
     return check_launch("matpl_nep_skin_update");

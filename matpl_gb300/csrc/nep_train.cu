@@ -711,8 +711,7 @@ template <typename T, int MODE, int NM, int KM>
 int launch_mb(const FeatArgs &A, cudaStream_t s) {
     const size_t smem = sizeof(MbSmem<T, MODE, NM, KM>) * kFeatWarps + table_bytes<T>(A);
     auto k = nepmb_op<T, MODE, NM, KM>;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess) {
+    if (allow_smem(k, smem) != cudaSuccess) {
         set_error("matpl_nep_feat: shared-memory attribute rejected");
         return MATPL_ERR_CUDA;
     }
@@ -724,8 +723,7 @@ template <typename T, int MODE, int NM, int KM>
 int launch_2b(const FeatArgs &A, cudaStream_t s) {
     const size_t smem = A.dc ? table_bytes<T>(A) + sizeof(T) * kFeatWarps * A.ntypes * A.nbase : 0;
     auto k = nep2b_op<T, MODE, NM, KM>;
-    if (smem && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-                    cudaSuccess) {
+    if (smem && allow_smem(k, smem) != cudaSuccess) {
         set_error("matpl_nep_feat: shared-memory attribute rejected");
         return MATPL_ERR_CUDA;
     }

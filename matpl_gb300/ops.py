@@ -216,7 +216,8 @@ def workspace(device: torch.device, nbytes: int, tag: str) -> torch.Tensor:
 def stream_workspaces(stream: int):
     """The scratch buffers held now for one stream, for a graph captured on it to keep alive
     (streams come from a pool, so a later capture on the same one may replace them)."""
-    return tuple(buf for (_, st, _), buf in _ws_cache.items() if st == stream)
+    held = list(_ws_cache.items())         # other threads add theirs meanwhile
+    return tuple(buf for (_, st, _), buf in held if st == stream)
 
 
 @_lib.on_device

@@ -300,21 +300,25 @@ nb_search(const NbImage *__restrict__ img, const double *__restrict__ wpos,
 #pragma unroll
         for (int q = 0; q < 9; ++q) Lf[q] = im.Lf[q];
         const float thr2 = im.thr2;
-        const int nimg1 = 2 * im.nper[2] + 1, nimg2 = 2 * im.nper[1] + 1;
-        const int nimg = im.iflag ? (2 * im.nper[0] + 1) * nimg2 * nimg1 : 1;
+        const unsigned nimg1 = 2u * im.nper[2] + 1u, nimg2 = 2u * im.nper[1] + 1u;
+        const int nimg = im.iflag ? (int)((2u * im.nper[0] + 1u) * nimg2 * nimg1) : 1;
 
         // ---- phase A: enumerate candidates (flattened over cell ranges / images), FP32 filter
         int ncand = 0;
         bool cap_hit = false;
         if (im.iflag) {
-            long long T = (long long)P.natoms * nimg;
-            if (T > 0x7fffffffLL) {           // keys would overflow int32: no candidates
+            // candidate c = (j, i1, i2, i3) in mixed radix, advanced by 32 per pass without
+            // divisions.  A cell vector so short that a radix or the number of candidates leaves
+            // int32 is refused: the walk and its keys hold for positive radices only.
+            auto radix = [&](int k) { return (int)(2u * (unsigned)im.nper[k] + 1u); };
+            const int n1 = radix(0), n2 = radix(1), n3 = radix(2);
+            const long long most = 0x7fffffffLL;
+            long long T = P.natoms;
+            if (!(n1 > 0 && n2 > 0 && n3 > 0 && (T *= n1) <= most && (T *= n2) <= most &&
+                  (T *= n3) <= most)) {
                 if (lane == 0) atomicMax(err, MATPL_KERR_BAD_BOX);
                 T = 0;
             }
-            // candidate c = (j, i1, i2, i3) in mixed radix, advanced by 32 per pass without
-            // divisions
-            const int n3 = nimg1, n2 = nimg2, n1 = 2 * im.nper[0] + 1;
             const int s3 = 32 % n3, s2 = 32 / n3 % n2, s1 = 32 / n3 / n2 % n1, sj = 32 / n3 / n2 / n1;
             int i3 = lane % n3, i2 = lane / n3 % n2, i1 = lane / n3 / n2 % n1, j = lane / n3 / n2 / n1;
             for (long long c0 = 0; c0 < T; c0 += 32) {

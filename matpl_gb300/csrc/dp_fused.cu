@@ -218,8 +218,9 @@ __device__ __forceinline__ void stage_weights(const T *__restrict__ src, T *dst,
 }
 
 // --------------------------------------------------------------------------- dp_embed_fwd
-// SPLIT: the block's warps share one atom, each taking every kWarps-th run of 32 slots, and warp 0 adds
-// their sums in order (FP64 only: in FP32 a caller's FP64 totals would show the regrouping).
+// SPLIT (see the launch): the block's warps share one atom, each taking every kWarps-th run of 32 slots,
+// and warp 0 adds their sums in order (FP64 only: in FP32 a caller's FP64 totals would show the
+// regrouping).
 template <typename T, bool WS, bool CMP, bool SPLIT>
 __global__ void __launch_bounds__(kWarps * 32)
 dp_embed_fwd(const int32_t *__restrict__ list_neigh, const T *__restrict__ idr,
@@ -832,12 +833,6 @@ int launch_eval(int mode, const matpl_dp_model *M, const EvalParams &P,
         dp_pad<T><<<(nnet + 3) / 4, 128, 0, s>>>(params, davg, dstd, pad, P.ntypes, P);
     }
 
-    // A small batch runs one atom per block, so that its atoms reach every SM before any SM takes a
-    // second: FP64 issues two lanes a clock per SM, and 108 atoms in four-warp blocks of four atoms
-    // kept 27 SMs busy (forward + backward 1.5 ms, 0.97 ms in one-warp blocks).  In FP64 the block's
-    // four warps then share the atom: one warp fills less than half of the pipe (0.97 -> 0.33 ms).
-    // Above 16 atoms per SM both shapes fill the chip and the four-atom block stages the nets a
-    // quarter as often.
     const size_t wbytes = sizeof(T) * (size_t)nnet * EmbOff::SIZE;
     const bool ws_ok = wbytes <= 128 * 1024 && P.ctab == nullptr;   // tables: no net weights
     const size_t wpart = ws_ok ? wbytes : 0;
@@ -845,11 +840,26 @@ int launch_eval(int mode, const matpl_dp_model *M, const EvalParams &P,
         return wpart + sizeof(T) * w * (backward ? 2 * E * 32 + NA : 32 * (E + 1 + 4)) +
                sizeof(int) * w * P.nslots;
     };
-    const bool small = total < 16LL * device_sms();
-    const bool split = small && sizeof(T) == 8 && smem_of(kWarps, true) <= 220 * 1024;
-    const int nwarps = small && !split ? 1 : kWarps, atoms = small ? 1 : kWarps;
+    // Four atoms a block, one per warp; or one atom a block, shared by its four warps, which small FP64
+    // batches take: the pipe issues two lanes a clock per SM, so what counts is how many atoms the
+    // fullest SM gets, and a block of four fills one SM while others idle (forward + backward of 108
+    // atoms of one element: 676 us in blocks of four, 329 shared).  A shared atom costs up to a
+    // quarter more of its SM (at 45 pairs two of the four warps have none; every block stages the nets
+    // of all type pairs), twice as much where only one such block fits, and three blocks of four are
+    // placed as four on some SMs: the line compares the two forms' fullest SM.  Two elements, us,
+    // blocks of four / shared: 600 atoms 712 / 728, 768 1301 / 1080, 1,216 1290 / 1450, 1,824 2600 /
+    // 2300, 2,400 2546 / 2963; three elements (one block): 152 740 / 371, 304 742 / 743, 1,216 1468 /
+    // 2890; four (nets read from memory): 456 2059 / 1259, 912 2725 / 2470, 1,300 3328 / 3738.  FP32
+    // atoms are too cheap to share (2,400 of four elements: 171 in blocks of four, 770 in one-atom blocks).
+    const size_t need = smem_of(kWarps, true), limit = 220 * 1024;
+    const long long sms = device_sms();
+    const long long alone = (total + sms - 1) / sms, four = (total + 4 * sms - 1) / (4 * sms);
+    const bool staged = ws_ok || P.ctab != nullptr;
+    const bool split = sizeof(T) == 8 && need <= limit && (staged || four <= 2) &&
+                       (2 * need <= limit ? 5 : 8) * alone < 16 * (four == 3 ? 4 : four);
+    const int nwarps = need <= limit ? kWarps : 1, atoms = split ? 1 : nwarps;
     const int gridw = (int)std::max<long long>(
-        1, std::min<long long>((total + atoms - 1) / atoms, (long long)device_sms() * 8 * (kWarps / nwarps)));
+        1, std::min<long long>((total + atoms - 1) / atoms, sms * 8 * (kWarps / nwarps)));
     const size_t smem_f = smem_of(nwarps, false), smem_b = smem_of(nwarps, true);
     constexpr bool D = sizeof(T) == 8;
     auto kf = P.ctab ? (split ? dp_embed_fwd<T, false, true, D> : dp_embed_fwd<T, false, true, false>)
@@ -878,7 +888,6 @@ int launch_eval(int mode, const matpl_dp_model *M, const EvalParams &P,
         // the widest tile that still gives every SM one: at 108 atoms (FP64) one-atom tiles
         // take 48 us where four 32-atom tiles took over 300
         constexpr int RB = sizeof(T) == 8 ? 8 : 16;
-        const long long sms = device_sms();
         if (total >= RB * sms) st = launch_fit<T, RB>(A, type_map, params, Ei, dA, P, s);
         else if (total >= 4 * sms) st = launch_fit<T, 4>(A, type_map, params, Ei, dA, P, s);
         else st = launch_fit<T, 1>(A, type_map, params, Ei, dA, P, s);

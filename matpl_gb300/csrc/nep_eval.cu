@@ -68,8 +68,7 @@ struct EvalArgs {
     int o_stash_g, o_stash_b, o_s, o_dEds, o_fin, o_dq, o_dpre;
     int o_rj, o_rv, o_rgp, o_aj, o_av, o_ag, o_agp;
     int rpb;                 // runs per block (further warps only help to stage the parameters)
-    int pair;                // 1: two warps per run
-    int o_vir;               // pair: the run's virial sums, [runs of the block][9][32]
+    int o_vir;               // two warps per run: the run's virial sums, [runs of the block][9][32]
 };
 
 // f64 -> f32, round to nearest even, with integer instructions: the FP64 pipe of this part
@@ -191,8 +190,8 @@ constexpr bool can_pair() { return sizeof(T) == 4 && NRM <= 5; }
 // they take its atoms alternately, and only the force pass (about an eighth of the time), which
 // reads and extends the run's virial sums, is handed from one to the other through a pair of
 // mbarriers.  The sums are the ones a single warp forms, in the same order.
-template <typename T, int NRM, int KRM, int NAM, int KAM, bool CL, bool EX>
-__global__ void __launch_bounds__((can_pair<T, NRM>() ? 2 : 1) * kRunsPerBlock * 32)
+template <typename T, int NRM, int KRM, int NAM, int KAM, bool CL, bool EX, bool PAIR>
+__global__ void __launch_bounds__((PAIR ? 2 : 1) * kRunsPerBlock * 32)
 nep_eval_kernel(EvalArgs A, long long atoms_per_run) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const NepLayout &L = A.L;
@@ -204,7 +203,8 @@ nep_eval_kernel(EvalArgs A, long long atoms_per_run) {
     if (threadIdx.x < 24) c3s[threadIdx.x] = C3<T>(threadIdx.x);
     // turn[run][w]: warp w of the run may start its next force pass
     __shared__ __align__(8) uint64_t turn[kRunsPerBlock][2];
-    const int pair = can_pair<T, NRM>() ? A.pair : 0, run = pair ? wib >> 1 : wib, wg = pair ? wib & 1 : 0;
+    constexpr int pair = PAIR ? 1 : 0;
+    const int run = wib >> pair, wg = wib & pair;
     if (pair && threadIdx.x < 2 * kRunsPerBlock) tc::mbar_init(&turn[threadIdx.x >> 1][threadIdx.x & 1], 1);
     // parameters: c2, c3, q_scaler as packed; per element W0 rows padded to Hp, b0, W1, b1
     {
@@ -779,7 +779,6 @@ template <typename T, int NRM, int KRM, int NAM, int KAM, bool CL, bool EX>
 int launch_eval(const EvalArgs &A0, cudaStream_t s) {
     EvalArgs A = A0;
     const NepLayout &L = A.L;
-    auto kern = nep_eval_kernel<T, NRM, KRM, NAM, KAM, CL, EX>;
     // per-warp scratch, 16-byte aligned pieces
     int off = 0;
     auto take = [&](size_t bytes) {
@@ -833,14 +832,19 @@ int launch_eval(const EvalArgs &A0, cudaStream_t s) {
     // 0.49 -> 0.32 ms)
     A.o_vir = (int)smem_of(2 * rpb, A.warp_bytes);
     const size_t smem_pair = A.o_vir + rpb * 9 * 32 * t;
-    A.pair = can_pair<T, NRM>() && blocks == 1 && apr > 1 && !A.feats && smem_pair <= limit + 4 * 1024;
+    const bool pair = can_pair<T, NRM>() && blocks == 1 && apr > 1 && !A.feats && smem_pair <= limit + 4 * 1024;
     // small batches: fewer runs per block, so that every SM gets one.  The block keeps its warps: each
     // stages all parameters, and 32 threads take up to 95 us for that (100 atoms of four elements,
     // FP32, 100 hidden units: 42 us in 13 blocks of 8 runs, 137 us in 100 one-warp blocks).
     if (nruns < sms * rpb) rpb = (int)std::max<long long>(1, (nruns + sms - 1) / sms);
     A.rpb = rpb;
-    const int wpb = rpb << A.pair, threads = 32 * std::max(wpb, kRunsPerBlock);
-    const size_t smem = A.pair ? smem_pair : smem_of(wpb, A.warp_bytes);
+    // a kernel of its own: with the hand-off compiled in, single-warp runs took 74 us where they now take
+    // 71 (8,000 atoms, lists of 72 / 28)
+    constexpr bool CP = can_pair<T, NRM>();
+    auto kern = pair ? nep_eval_kernel<T, NRM, KRM, NAM, KAM, CL, EX, CP>
+                     : nep_eval_kernel<T, NRM, KRM, NAM, KAM, CL, EX, false>;
+    const int wpb = pair ? 2 * rpb : rpb, threads = 32 * std::max(wpb, kRunsPerBlock);
+    const size_t smem = pair ? smem_pair : smem_of(wpb, A.warp_bytes);
     if (allow_smem(kern, smem) != cudaSuccess)
         return check_launch("shared memory of nep_eval");
     const int grid = (int)((nruns + rpb - 1) / rpb);

@@ -112,10 +112,22 @@ __device__ __forceinline__ void flush_tables(const T *tab, int E, const FeatArgs
 }
 
 // ---------------------------------------------------------------- radial (calculateNepFeat)
+// Blocks an SM that the registers have to leave room for.  The large form (n up to 8) takes 152 registers
+// in FP32 and 197 in FP64 unless it is told, half the warps it had in its earlier shape: backward
+// of 15,000 atoms, one type of n 5 / K 13, 36 + 36 pairs: radial 129 us so, 80 before; angular 611 (255
+// registers), 472 before.  With the bounds here the three passes of 10,000 such atoms take 724 us
+// (880 without, 814 before).
+template <typename T, int NM>
+constexpr int radial_blocks() { return NM > 5 ? (sizeof(T) == 8 ? 4 : 6) : sizeof(T) == 8 ? 1 : 8; }
+template <typename T, int MODE, int NM>
+constexpr int angular_blocks() {
+    return sizeof(T) == 8 ? (MODE == kFwd && NM > 5 ? 5 : 1) : NM <= 5 ? 5 : MODE == kBwd2 ? 4 : 3;
+}
+
 // Bound by issue: the sums over pairs of one type (W) take as long as basis and features.  Empty slots
 // are written here, so no caller clears grad_d12.
 template <typename T, int MODE, int NM, int KM>
-__global__ void __launch_bounds__(32 * kFeatWarps, sizeof(T) == 4 && NM <= 5 ? 8 : 1) nep2b_op(FeatArgs A) {
+__global__ void __launch_bounds__(32 * kFeatWarps, radial_blocks<T, NM>()) nep2b_op(FeatArgs A) {
     __shared__ T s_st[kFeatWarps][32][KM + 1];
     __shared__ __align__(16) int s_tj[kFeatWarps][32];
     extern __shared__ __align__(16) unsigned char mb_raw[];
@@ -416,7 +428,7 @@ __device__ __forceinline__ void harm_d(int m, T ux, T uy, T uz, T ri, T &b, T &b
 // c-gradient: backward 167 -> 108 us, second backward 209 -> 162; 100,000: 786 -> 508, 1119 -> 791.  Five blocks an SM
 // in FP32 (102 registers): with 128 the backward takes 117 us.
 template <typename T, int MODE, int NM, int KM>
-__global__ void __launch_bounds__(32 * kFeatWarps, sizeof(T) == 4 && NM <= 5 ? 5 : 1) nepmb_op(FeatArgs A) {
+__global__ void __launch_bounds__(32 * kFeatWarps, angular_blocks<T, MODE, NM>()) nepmb_op(FeatArgs A) {
     extern __shared__ __align__(16) unsigned char mb_raw[];
     using Sm = MbSmem<T, MODE, NM, KM>;
     constexpr int NP = Sm::NP;
@@ -692,14 +704,18 @@ __global__ void __launch_bounds__(32 * kFeatWarps, sizeof(T) == 4 && NM <= 5 ? 5
     if (want_c && A.dc) flush_tables<T>(tabs, E, A);
 }
 
-// Blocks: enough for every atom's warp, but where each leaves a table behind, one wave of them.
-template <typename K>
+// Blocks: enough for every atom's warp, but where each leaves a table behind, one wave of them in FP32
+// (5,000 atoms, n 5, K 13: 398 us for first and second backward with forward, 421 in two waves) and
+// up to four in FP64, whose blocks run long enough for the last of a single wave to show (2,000 such
+// atoms: 3152 us in one wave, 2952 in four).
+template <typename T, typename K>
 int feat_blocks(const FeatArgs &A, K k, size_t smem) {
     const long long need = (A.natoms + kFeatWarps - 1) / kFeatWarps;
     int per_sm = 32;
     if (A.dc && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 32 * kFeatWarps, smem) != cudaSuccess)
         per_sm = 1;
-    return (int)std::max<long long>(1, std::min<long long>(need, (long long)device_sms() * std::max(per_sm, 1)));
+    const int waves = A.dc && sizeof(T) == 8 ? 4 : 1;
+    return (int)std::max<long long>(1, std::min<long long>(need, (long long)device_sms() * waves * std::max(per_sm, 1)));
 }
 
 template <typename T>
@@ -715,7 +731,7 @@ int launch_mb(const FeatArgs &A, cudaStream_t s) {
         set_error("matpl_nep_feat: shared-memory attribute rejected");
         return MATPL_ERR_CUDA;
     }
-    k<<<feat_blocks(A, k, smem), 32 * kFeatWarps, smem, s>>>(A);
+    k<<<feat_blocks<T>(A, k, smem), 32 * kFeatWarps, smem, s>>>(A);
     return check_launch("matpl_nep_feat");
 }
 
@@ -727,7 +743,7 @@ int launch_2b(const FeatArgs &A, cudaStream_t s) {
         set_error("matpl_nep_feat: shared-memory attribute rejected");
         return MATPL_ERR_CUDA;
     }
-    k<<<feat_blocks(A, k, smem), 32 * kFeatWarps, smem, s>>>(A);
+    k<<<feat_blocks<T>(A, k, smem), 32 * kFeatWarps, smem, s>>>(A);
     return check_launch("matpl_nep_feat");
 }
 

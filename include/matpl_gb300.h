@@ -471,6 +471,11 @@ int matpl_nep_eval_compact(int dtype, const matpl_nep_model *model, int nframes,
                            double *Etot, void *force, double *virial, void *workspace,
                            size_t workspace_bytes, void *stream);
 
+/* matpl_bytes_differ: *answer = 1 where the two device arrays differ in a byte, else 0.  answer is
+ *   device or pinned host memory (there it can be read once the stream has passed the call).
+ */
+int matpl_bytes_differ(const void *a, const void *b, size_t bytes, int32_t *answer, void *stream);
+
 /* ------------------------------------------------------------------------------------
  * Data-path statistics.  Replaces the per-image calc_stat + smooth of
  * src/pre_data/dpuni_data_loader.py:422-563 (davg / dstd of calculate_davg_dstd, :377-420).

@@ -63,10 +63,43 @@ env_stats_kernel(int batch, int natoms, int nslots, int ntypes, const int32_t *_
     }
 }
 
+// Bound: latency.  One block: a type map is some kilobytes (16,000 int32: four loads a thread).
+__global__ void __launch_bounds__(1024)
+bytes_differ_kernel(const unsigned char *__restrict__ a, const unsigned char *__restrict__ b,
+                    size_t n, int32_t *answer) {
+    const uintptr_t at = (uintptr_t)a | (uintptr_t)b;
+    size_t done = 0;
+    bool d = false;
+    if ((at & 15u) == 0) {
+        const uint4 *x = reinterpret_cast<const uint4 *>(a), *y = reinterpret_cast<const uint4 *>(b);
+        for (size_t q = threadIdx.x; q < n / 16; q += blockDim.x) {
+            const uint4 u = x[q], v = y[q];
+            d |= ((u.x ^ v.x) | (u.y ^ v.y) | (u.z ^ v.z) | (u.w ^ v.w)) != 0u;
+        }
+        done = n / 16 * 16;
+    } else if ((at & 3u) == 0) {
+        const unsigned *x = reinterpret_cast<const unsigned *>(a), *y = reinterpret_cast<const unsigned *>(b);
+        for (size_t q = threadIdx.x; q < n / 4; q += blockDim.x) d |= x[q] != y[q];
+        done = n / 4 * 4;
+    }
+    for (size_t q = done + threadIdx.x; q < n; q += blockDim.x) d |= a[q] != b[q];
+    const int any = __syncthreads_or(d);
+    if (threadIdx.x == 0) *answer = any != 0;
+}
+
 }  // namespace
 }  // namespace matpl
 
 using namespace matpl;
+
+extern "C" int matpl_bytes_differ(const void *a, const void *b, size_t bytes, int32_t *answer,
+                                  void *stream) {
+    MATPL_REQUIRE(answer && (bytes == 0 || (a && b)), MATPL_ERR_INVALID, "null pointer argument");
+    MATPL_REQUIRE_ON_DEVICE(a, "matpl_bytes_differ");
+    bytes_differ_kernel<<<1, 1024, 0, as_stream(stream)>>>(
+        static_cast<const unsigned char *>(a), static_cast<const unsigned char *>(b), bytes, answer);
+    return check_launch("matpl_bytes_differ");
+}
 
 extern "C" int matpl_env_stats(int batch, int natoms, int nslots, int ntypes,
                                const int32_t *type_map, const int32_t *list_neigh,

@@ -15,6 +15,7 @@ traffic).  Parameters use the reference's state-dict names; ``pack_params`` lays
 ``csrc/dp_layout.cuh`` expects.
 """
 import ctypes
+import threading
 from typing import Dict, List, Optional
 
 import torch
@@ -120,22 +121,46 @@ class LastMap:
     """What a type map on the device leads to (finding its atoms by element costs a host read and
     several launches), kept until another map comes.  Neither a tensor's address nor its version says
     that it holds the same values (inference tensors, ``.data``, a graph's replay), so a copy of the
-    map is kept and compared: one host read per call.  An entry belongs to the stream it was made
+    map is kept and compared at every call: one launch that answers in pinned host memory, readable
+    after the next synchronisation with the stream.  An entry belongs to the stream it was made
     on: no other stream reads its tensors before they are written or after they are freed."""
 
     def __init__(self):
         self._entry = None
+        self._answers = {}                        # thread -> its pinned word
 
-    def get(self, tmap: torch.Tensor, key, make):
+    def __reduce__(self):                         # copied and saved models start without one
+        return LastMap, ()
+
+    def ask(self, tmap: torch.Tensor, key):
+        """Queues the comparison of ``tmap`` with the kept map; ``get`` takes what it returns."""
         from .ops import _stream
         key = (_stream(tmap.device), key)
         e = self._entry
-        if e is not None and e[0] == key and e[1].shape == tmap.shape and \
-                e[1].dtype == tmap.dtype and e[1].device == tmap.device and torch.equal(e[1], tmap):
-            return e[2]
+        if e is None or e[0] != key or e[1].shape != tmap.shape or e[1].dtype != tmap.dtype or \
+                e[1].device != tmap.device or not tmap.is_contiguous():
+            return key, None, None
+        me = threading.get_ident()
+        word = self._answers.get(me)
+        if word is None:
+            if len(self._answers) >= 64:
+                self._answers = {}
+            word = self._answers[me] = torch.empty(1, dtype=torch.int32, pin_memory=True)
+        differ(e[1], tmap, word)
+        return key, e, word
+
+    def get(self, tmap: torch.Tensor, make, asked, synced: bool = False):
+        """The kept value, or ``make(tmap)`` where the map is another one.  ``synced``: the stream
+        has been synchronised since ``ask``."""
+        key, e, word = asked
+        if e is not None:
+            if not synced:
+                torch.cuda.current_stream(tmap.device).synchronize()
+            if word.item() == 0:
+                return e[2]
         with torch.inference_mode(False):         # the entry serves calls in every mode
             value = make(tmap)
-            self._entry = (key, tmap.detach().clone(), value)
+            self._entry = (key, tmap.detach().clone(memory_format=torch.contiguous_format), value)
         return value
 
     def last(self, tmap: torch.Tensor, key):
@@ -144,6 +169,15 @@ class LastMap:
         if e is None or e[0][1] != key or e[1].shape != tmap.shape:
             raise _lib.MatplError("make one call with this type map before capturing it in a graph")
         return e[2]
+
+
+@_lib.on_device
+def differ(a: torch.Tensor, b: torch.Tensor, answer: torch.Tensor):
+    """Queues the comparison of two contiguous device tensors of one size; ``answer`` (pinned host int32)
+    is 1 where a byte differs once the stream has passed it."""
+    from .ops import _stream
+    check(_lib.load().matpl_bytes_differ(ptr(a), ptr(b), a.numel() * a.element_size(), ptr(answer),
+                                         _stream(a.device)), "matpl_bytes_differ")
 
 
 class DP(torch.nn.Module):
@@ -208,24 +242,24 @@ class DP(torch.nn.Module):
             m.ctab_rows, m.ctab_order, m.ctab_dx, m.ctab_smin, m.ctab_smax = self._ctab
         return m
 
-    def _grouped_perm(self, tmap: torch.Tensor, present: List[int]) -> torch.Tensor:
+    def _grouped_perm(self, tmap: torch.Tensor, present: List[int], asked=None,
+                      synced: bool = False) -> torch.Tensor:
         """Atoms of ``tmap`` (the caller's type map) grouped by element, on the model's device."""
         def grouped(m):
             return [torch.nonzero(m == t).flatten() for t in present]
         if not tmap.is_cuda:
             return torch.cat(grouped(tmap)).to(self.packed.device)
-        key = (self.packed.device, tuple(present))
-        if torch.cuda.is_current_stream_capturing():
+        if asked is None:
             # a graph reads the map at every replay: the element counts are those of the last call,
             # the order is found in the graph (a stable sort puts an element's atoms first)
-            counts = self._order.last(tmap, key)[1]
+            counts = self._order.last(tmap, tuple(present))[1]
             return torch.cat([torch.sort((tmap != t).to(torch.int32), stable=True)[1][:n]
                               for t, n in zip(present, counts)])
 
         def make(m):
             parts = grouped(m)
             return torch.cat(parts), [q.numel() for q in parts]
-        return self._order.get(tmap, key, make)[0]
+        return self._order.get(tmap, make, asked, synced)[0]
 
     @_lib.on_device
     def evaluate(self, list_neigh: torch.Tensor, Imagetype_map: torch.Tensor, present: List[int],
@@ -235,6 +269,11 @@ class DP(torch.nn.Module):
 
         ``num_neigh`` [B,N,ntypes] int32 (from ``find_neighbore(..., occupied_only=True)``)
         gives the type blocks' lengths; the list's slots past them are then never read."""
+        out = self._launch(list_neigh, Imagetype_map, present, ImageDR, nghost, out, num_neigh)
+        self._check()
+        return out
+
+    def _launch(self, list_neigh, Imagetype_map, present, ImageDR, nghost=0, out=None, num_neigh=None):
         if not (list_neigh.is_cuda and ImageDR.is_cuda):
             raise _lib.MatplError("DP.evaluate takes CUDA tensors (no CPU fallback)")
         B, N, S = list_neigh.shape
@@ -271,6 +310,11 @@ class DP(torch.nn.Module):
                                              ptr(out["Ei_atom"]), ptr(out["Etot"]),
                                              ptr(out["Force"]), ptr(out["Virial"]), ptr(ws),
                                              ws.numel(), stream), "matpl_dp_eval_occupied")
+        return out
+
+    _launch_on_device = _lib.on_device(_launch)
+
+    def _check(self):
         if self.check_errors:
             code = int(self.err.item())
             if code:
@@ -279,14 +323,23 @@ class DP(torch.nn.Module):
                     raise _lib.MatplError("matpl_dp_eval: a tensor-core completion wait gave up "
                                           "(MATPL_KERR_TIMEOUT); the outputs are invalid")
                 raise _lib.MatplError(f"matpl_dp_eval kernel error code {code}")
-        return out
+
+    def _grouped(self, list_neigh, Imagetype_map, tm, present, ImageDR, nghost):
+        """The evaluation and the element-grouped order; the map's comparison is queued behind the
+        evaluation's kernels, ahead of the read of the error word."""
+        r = self._launch_on_device(list_neigh, tm, present, ImageDR, nghost)
+        asked = None
+        if Imagetype_map.is_cuda and not torch.cuda.is_current_stream_capturing():
+            asked = self._order.ask(Imagetype_map, tuple(present))
+        self._check()
+        synced = self.check_errors and Imagetype_map.device == ImageDR.device
+        return r, self._grouped_perm(Imagetype_map, present, asked, synced)
 
     def forward(self, list_neigh, Imagetype_map, atom_type, ImageDR, nghost: int = 0,
                 Egroup_weight=None, divider=None, is_calc_f: Optional[bool] = True):
         present = self.present_types(atom_type)
         tm = Imagetype_map.to(device=ImageDR.device, dtype=torch.int32)
-        r = self.evaluate(list_neigh, tm, present, ImageDR, int(nghost))
-        perm = self._grouped_perm(Imagetype_map, present)
+        r, perm = self._grouped(list_neigh, Imagetype_map, tm, present, ImageDR, int(nghost))
         Ei = r["Ei_atom"][:, perm]
         Etot = r["Etot"].to(self.dtype).unsqueeze(-1)
         Egroup = None

@@ -513,7 +513,7 @@ class FusedTrainer:
                 blocks[ti] = (off, n)
                 off += B * n
             return torch.cat(rows).contiguous(), blocks
-        self._rows, self._blocks = self._order.get(tm32, key, make)
+        self._rows, self._blocks = self._order.get(tm32, make, self._order.ask(tm32, key))
         return self._rows, self._blocks
 
     def _present_types(self, batch):
@@ -631,6 +631,7 @@ class GraphedTrainer:
                  w_f: float = 1.0, w_e: float = 1.0, warmup: int = 3):
         self.tr, self.opt = trainer, optimizer
         self.w_f, self.w_e, self.warmup = w_f, w_e, warmup
+        self._answer = None         # pinned word and event of the type maps' comparison
         self.graphs = {}            # shape key -> captured steps, the last used first
 
     def _keys(self, batch):
@@ -665,16 +666,32 @@ class GraphedTrainer:
             if batch[k].data_ptr() != captured.static[k].data_ptr():
                 captured.static[k].copy_(batch[k], non_blocking=True)
 
+    def _compare(self, a, b):
+        """Queues the comparison of two arrays; the function it returns waits for the answer."""
+        if not (a.is_cuda and a.is_contiguous() and b.is_contiguous()):
+            return lambda: torch.equal(a, b)
+        if self._answer is None:
+            self._answer = torch.empty(1, dtype=torch.int32, pin_memory=True), torch.cuda.Event()
+        word, done = self._answer
+        _dp.differ(a, b, word)
+        done.record(torch.cuda.current_stream(a.device))
+
+        def equal():
+            done.synchronize()
+            return word.item() == 0
+        return equal
+
     def step(self, batch):
         keys = self._keys(batch)
         key = tuple(tuple(batch[k].shape) for k in keys) + (tuple(batch["atom_type"]),)
         steps = self.graphs.setdefault(key, [])
         hit = steps[0] if steps else None
         if hit is not None:
-            # the copies are queued first: they run while the host waits for the comparison
-            self._load(hit, batch, [k for k in keys if k != "type_map"])
             held = hit.static["type_map"]
-            if not torch.equal(held, batch["type_map"].to(held.device, held.dtype)):
+            equal = self._compare(held, batch["type_map"].to(held.device, held.dtype))
+            # these copies run while the host waits for the comparison
+            self._load(hit, batch, [k for k in keys if k != "type_map"])
+            if not equal():
                 rows, blocks = self.tr._type_index_of(batch)
                 hit = next((c for c in steps if c.blocks == blocks), None)
                 if hit is not None:

@@ -282,8 +282,7 @@ class DP(torch.nn.Module):
             else list_neigh.to(torch.int32).contiguous()
         idr = ImageDR if ImageDR.dtype == self.dtype and ImageDR.is_contiguous() \
             else ImageDR.to(self.dtype).contiguous()
-        tm = Imagetype_map if Imagetype_map.dtype == torch.int32 and Imagetype_map.is_cuda \
-            else Imagetype_map.to(device=dev, dtype=torch.int32).contiguous()
+        tm = Imagetype_map.to(device=dev, dtype=torch.int32).contiguous()    # itself where it is one
         if out is None:
             out = {"Ei_atom": torch.empty(B, N, dtype=self.dtype, device=dev),
                    "Etot": torch.empty(B, dtype=torch.float64, device=dev),

@@ -535,7 +535,7 @@ class FusedTrainer:
         idr = batch["ImageDR"]
         idr = idr if idr.dtype == model.dtype and idr.is_contiguous() else idr.to(model.dtype).contiguous()
         tm32 = batch["type_map"]
-        tm32 = tm32 if tm32.dtype == torch.int32 else tm32.to(device=dev, dtype=torch.int32).contiguous()
+        tm32 = tm32.to(device=dev, dtype=torch.int32).contiguous()       # itself where it is one
         present = self._present_types(batch)
         self._present = present
         rows, blocks = self._type_index(tm32, present, B)

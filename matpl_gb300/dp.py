@@ -121,13 +121,13 @@ class LastMap:
     """What a type map on the device leads to (finding its atoms by element costs a host read and
     several launches), kept until another map comes.  Neither a tensor's address nor its version says
     that it holds the same values (inference tensors, ``.data``, a graph's replay), so a copy of the
-    map is kept and compared at every call: one launch that answers in pinned host memory, readable
-    after the next synchronisation with the stream.  An entry belongs to the stream it was made
-    on: no other stream reads its tensors before they are written or after they are freed."""
+    map is kept and compared at every call: one launch that answers in pinned host memory, and an
+    event behind it to wait for.  An entry belongs to the stream it was made on: no other stream
+    reads its tensors before they are written or after they are freed."""
 
     def __init__(self):
         self._entry = None
-        self._answers = {}                        # thread -> its pinned word
+        self._answers = {}                        # thread -> its pinned word and event
 
     def __reduce__(self):                         # copied and saved models start without one
         return LastMap, ()
@@ -140,22 +140,22 @@ class LastMap:
         if e is None or e[0] != key or e[1].shape != tmap.shape or e[1].dtype != tmap.dtype or \
                 e[1].device != tmap.device or not tmap.is_contiguous():
             return key, None, None
-        me = threading.get_ident()
-        word = self._answers.get(me)
-        if word is None:
+        me = (threading.get_ident(), tmap.device)
+        answer = self._answers.get(me)
+        if answer is None:
             if len(self._answers) >= 64:
                 self._answers = {}
-            word = self._answers[me] = torch.empty(1, dtype=torch.int32, pin_memory=True)
-        differ(e[1], tmap, word)
-        return key, e, word
+            answer = self._answers[me] = (torch.empty(1, dtype=torch.int32, pin_memory=True),
+                                          torch.cuda.Event())
+        differ(e[1], tmap, *answer)
+        return key, e, answer
 
-    def get(self, tmap: torch.Tensor, make, asked, synced: bool = False):
-        """The kept value, or ``make(tmap)`` where the map is another one.  ``synced``: the stream
-        has been synchronised since ``ask``."""
-        key, e, word = asked
+    def get(self, tmap: torch.Tensor, make, asked):
+        """The kept value, or ``make(tmap)`` where the map is another one."""
+        key, e, answer = asked
         if e is not None:
-            if not synced:
-                torch.cuda.current_stream(tmap.device).synchronize()
+            word, done = answer
+            done.synchronize()
             if word.item() == 0:
                 return e[2]
         with torch.inference_mode(False):         # the entry serves calls in every mode
@@ -172,12 +172,13 @@ class LastMap:
 
 
 @_lib.on_device
-def differ(a: torch.Tensor, b: torch.Tensor, answer: torch.Tensor):
+def differ(a: torch.Tensor, b: torch.Tensor, answer: torch.Tensor, done: torch.cuda.Event):
     """Queues the comparison of two contiguous device tensors of one size; ``answer`` (pinned host int32)
-    is 1 where a byte differs once the stream has passed it."""
+    is 1 where a byte differs once ``done`` has passed."""
     from .ops import _stream
     check(_lib.load().matpl_bytes_differ(ptr(a), ptr(b), a.numel() * a.element_size(), ptr(answer),
                                          _stream(a.device)), "matpl_bytes_differ")
+    done.record(torch.cuda.current_stream(a.device))
 
 
 class DP(torch.nn.Module):
@@ -242,8 +243,7 @@ class DP(torch.nn.Module):
             m.ctab_rows, m.ctab_order, m.ctab_dx, m.ctab_smin, m.ctab_smax = self._ctab
         return m
 
-    def _grouped_perm(self, tmap: torch.Tensor, present: List[int], asked=None,
-                      synced: bool = False) -> torch.Tensor:
+    def _grouped_perm(self, tmap: torch.Tensor, present: List[int], asked=None) -> torch.Tensor:
         """Atoms of ``tmap`` (the caller's type map) grouped by element, on the model's device."""
         def grouped(m):
             return [torch.nonzero(m == t).flatten() for t in present]
@@ -259,7 +259,7 @@ class DP(torch.nn.Module):
         def make(m):
             parts = grouped(m)
             return torch.cat(parts), [q.numel() for q in parts]
-        return self._order.get(tmap, make, asked, synced)[0]
+        return self._order.get(tmap, make, asked)[0]
 
     @_lib.on_device
     def evaluate(self, list_neigh: torch.Tensor, Imagetype_map: torch.Tensor, present: List[int],
@@ -324,15 +324,19 @@ class DP(torch.nn.Module):
                 raise _lib.MatplError(f"matpl_dp_eval kernel error code {code}")
 
     def _grouped(self, list_neigh, Imagetype_map, tm, present, ImageDR, nghost):
-        """The evaluation and the element-grouped order; the map's comparison is queued behind the
-        evaluation's kernels, ahead of the read of the error word."""
-        r = self._launch_on_device(list_neigh, tm, present, ImageDR, nghost)
+        """The evaluation and the element-grouped order.  With error checks on, the map's comparison is
+        queued behind the evaluation's kernels, where its host time is hidden and the read of the
+        error word waits anyway; without, ahead of them: the host then waits for the comparison
+        while the evaluation runs."""
         asked = None
-        if Imagetype_map.is_cuda and not torch.cuda.is_current_stream_capturing():
+        ask = Imagetype_map.is_cuda and not torch.cuda.is_current_stream_capturing()
+        if ask and not self.check_errors:
+            asked = self._order.ask(Imagetype_map, tuple(present))
+        r = self._launch_on_device(list_neigh, tm, present, ImageDR, nghost)
+        if ask and self.check_errors:
             asked = self._order.ask(Imagetype_map, tuple(present))
         self._check()
-        synced = self.check_errors and Imagetype_map.device == ImageDR.device
-        return r, self._grouped_perm(Imagetype_map, present, asked, synced)
+        return r, self._grouped_perm(Imagetype_map, present, asked)
 
     def forward(self, list_neigh, Imagetype_map, atom_type, ImageDR, nghost: int = 0,
                 Egroup_weight=None, divider=None, is_calc_f: Optional[bool] = True):

@@ -673,8 +673,7 @@ class GraphedTrainer:
         if self._answer is None:
             self._answer = torch.empty(1, dtype=torch.int32, pin_memory=True), torch.cuda.Event()
         word, done = self._answer
-        _dp.differ(a, b, word)
-        done.record(torch.cuda.current_stream(a.device))
+        _dp.differ(a, b, word, done)
 
         def equal():
             done.synchronize()

@@ -164,8 +164,8 @@ __host__ __device__ inline float sqrt_to_f32(float y, double v) {
     return y;
 }
 
-// sqrt(a) correctly rounded, a >= 0, with five FP64 operations instead of the eleven of the
-// library call: an FP32 root and reciprocal root, two Heron steps g += (a - g^2) h with the exact
+// sqrt(a) correctly rounded, a >= 0, with five FP64 operations: an FP32 root and reciprocal root,
+// two Heron steps g += (a - g^2) h with the exact
 // residual of a fused multiply-add, and a test of the last residual: |a - g^2| < g ulp(g)
 // (1 - 2^-20) holds only if the root lies within half an ulp of g, so g is its rounding.  What
 // fails the test (near a rounding boundary, a power of two, a far from 1) takes the library call.

@@ -399,8 +399,8 @@ __device__ __forceinline__ void fit_layer(const T *X, int ldx, int K, const T *_
 // One CTA of eight warps per tile of R atoms: the hidden layers give each thread a column of
 // RG rows, dE/dD (400 columns) gives each warp 50 columns of all rows.  Bound: shared loads and
 // the latency of the weight loads (80 KB per net, from L2).  A tile of 64 atoms whose eight warps
-// each read every weight ran 108 CTAs on 152 SMs at 6,913 atoms: 197 us; 16-atom tiles with a
-// weight load shared by four rows (eight in dE/dD's halves) take 74 us there.
+// each read every weight ran 109 CTAs on 152 SMs at 6,913 atoms: 197 us; 16-atom tiles with a
+// weight load shared by four rows (all sixteen in dE/dD) take 74 us there.
 template <typename T, int R>
 __global__ void __launch_bounds__(256)
 dp_fit(const T *__restrict__ Ain, const int32_t *__restrict__ type_map,

@@ -186,7 +186,7 @@ constexpr bool can_pair() { return sizeof(T) == 4 && NRM <= 5; }
 //
 // Bound: latency.  An atom is ~20 dependent phases, half of the issue slots are empty at 16 warps
 // per SM, and the virial ties a run's atoms together: its per-lane sums run over the atoms in order.
-// Where shared memory leaves room for one 8-run block per SM, two warps share a run (`pair`):
+// Where shared memory leaves room for one 8-run block per SM, two warps share a run (PAIR):
 // they take its atoms alternately, and only the force pass (about an eighth of the time), which
 // reads and extends the run's virial sums, is handed from one to the other through a pair of
 // mbarriers.  The sums are the ones a single warp forms, in the same order.
@@ -828,7 +828,7 @@ int launch_eval(const EvalArgs &A0, cudaStream_t s) {
     const long long apr = (A.natoms + runs - 1) / runs;
     const long long nruns = (A.natoms + apr - 1) / apr;
     // two warps per run where a block of them fits and the runs alone leave an SM 8 warps
-    // (100,000 atoms, lists of 80 / 32: 1.08 -> 0.75 ms; 50,000 atoms, compact lists of 104 / 48:
+    // (100,000 atoms, lists of 80 / 32: 1.08 -> 0.73 ms; 50,000 atoms, compact lists of 104 / 48:
     // 0.49 -> 0.32 ms)
     A.o_vir = (int)smem_of(2 * rpb, A.warp_bytes);
     const size_t smem_pair = A.o_vir + rpb * 9 * 32 * t;

@@ -596,7 +596,7 @@ __device__ __forceinline__ void dequeue32(int *queue, int &qn, int lane) {
 // COUNT: only count neighbors (calculate_maxneigh); TYPED: counts per neighbor element.
 // Bound by the FP64 pipe (70 % active) and issue.  The cell-ordered FP32 positions are read in runs
 // (no index, no gather), the exact test skips the orthorhombic zeros, and the root takes five FP64
-// operations: 575 -> 454 us for 100,000 atoms in one frame, and 62 -> 30 us for 6 x 72 replicated
+// operations: 575 -> 452 us for 100,000 atoms in one frame, and 62 -> 30 us for 6 x 72 replicated
 // atoms (FP32 test ahead of the exact one, one warp per block so that every SM has some).  Six blocks
 // an SM: seven and eight spill, 459 and 458 us.
 template <bool COUNT, bool TYPED>

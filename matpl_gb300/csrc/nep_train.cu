@@ -351,7 +351,7 @@ __device__ __forceinline__ T sbar_dot(const T *c3, int m, const T *sv, const T *
 }
 
 // per warp shared memory of the angular operator; the tangents (sd, sbd, gb, bb, fb) exist in BWD2
-// only and pass 2's f_k take the place of pass 1's b_m: 4.6 KB a warp in BWD, 9.7 in BWD2 (FP32)
+// only and pass 2's f_k take the place of pass 1's b_m: 5.4 KB a warp in BWD, 10.1 in BWD2 (FP32, n 5)
 template <typename T, int MODE, int NM, int KM>
 struct alignas(16) MbSmem {
     static constexpr int NP = (NM + 3) / 4 * 4, D = MODE == kBwd2 ? 1 : 0, G = MODE == kFwd ? 0 : 1;
@@ -425,8 +425,9 @@ __device__ __forceinline__ void harm_d(int m, T ux, T uy, T uz, T ri, T &b, T &b
 // Bound by issue and shared loads (FP64: by the FP64 pipe).  Pass 1 has lanes over m with all n in
 // registers, so a pair's b_m is read once instead of once per n; the c-terms walk the pairs of one type
 // instead of testing every pair for every entry.  20,000 atoms, four types, 22 pairs each, FP32, with the
-// c-gradient: backward 167 -> 108 us, second backward 209 -> 162; 100,000: 786 -> 508, 1119 -> 791.  Five blocks an SM
-// in FP32 (102 registers): with 128 the backward takes 117 us.
+// c-gradient: backward 167 -> 108 us, second backward 209 -> 162; 100,000: 786 -> 508, 1119 -> 791.  Five
+// blocks an SM in FP32 (96 registers): with 128 the backward takes 117 us.  (Shared memory leaves the
+// second backward of four types four: 41 KB a block and 11 of tables.)
 template <typename T, int MODE, int NM, int KM>
 __global__ void __launch_bounds__(32 * kFeatWarps, angular_blocks<T, MODE, NM>()) nepmb_op(FeatArgs A) {
     extern __shared__ __align__(16) unsigned char mb_raw[];

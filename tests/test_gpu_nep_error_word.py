@@ -49,3 +49,17 @@ def test_descriptor_operators():
     with pytest.raises(_lib.MatplError, match="error 5"):
         nep_ops.calculateNepFeat(prm["c_param_2"].to(DEV), ra, la, bad, ra.new_empty(0), 6.0, 0)
 
+
+def test_bad_type_inside_a_shared_run():
+    """Two warps share a run of atoms: a bad type alone is reported, not a hand-off that gave up."""
+    cfg = NP.NepConfig(atom_type=[3, 14])
+    fr = NP.frames_from_structures([structures.random_packed(2433, 0.05, [3, 14], [0.5, 0.5], seed=2)], 6.0)
+    tm = t(np.arange(2433) % 2, torch.int64)
+    na = t(fr.num_atom.reshape(-1, 1), torch.int64)
+    a, b, la, lb, ra, rb = ops.calculate_neighbor(na, tm, torch.arange(2, device=DEV), t(fr.box), t(fr.box_orig),
+                                                  t(fr.num_cell, torch.int64), t(fr.position), 6.0, 4.0,
+                                                  112, 60, True)
+    tm[1200] = 7
+    m = NP.NEP(cfg, NP.init_params(cfg, 3, energy_shift=-3.0), "float32", device=DEV, check_errors=False)
+    r = m.evaluate(a, la, ra, b, lb, rb, na, tm)
+    assert int(m.err.item()) == _lib.KERR_BAD_TYPE and float(r["Ei"][1200]) == 0.0

@@ -843,13 +843,13 @@ int launch_eval(int mode, const matpl_dp_model *M, const EvalParams &P,
     // Four atoms a block, one per warp; or one atom a block, shared by its four warps, which small FP64
     // batches take: the pipe issues two lanes a clock per SM, so what counts is how many atoms the
     // fullest SM gets, and a block of four fills one SM while others idle (forward + backward of 108
-    // atoms of one element: 676 us in blocks of four, 329 shared).  A shared atom costs up to a
+    // atoms of one element: 680 us in blocks of four, 329 shared).  A shared atom costs up to a
     // quarter more of its SM (at 45 pairs two of the four warps have none; every block stages the nets
     // of all type pairs), twice as much where only one such block fits, and three blocks of four are
-    // placed as four on some SMs: the line compares the two forms' fullest SM.  Two elements, us,
-    // blocks of four / shared: 600 atoms 712 / 728, 768 1301 / 1080, 1,216 1290 / 1450, 1,824 2600 /
-    // 2300, 2,400 2546 / 2963; three elements (one block): 152 740 / 371, 304 742 / 743, 1,216 1468 /
-    // 2890; four (nets read from memory): 456 2059 / 1259, 912 2725 / 2470, 1,300 3328 / 3738.  FP32
+    // placed as four on some SMs: the line compares the two forms' fullest SM.  us in blocks of four /
+    // shared, two elements: 600 atoms 712 / 729, 768 1281 / 1077, 1,216 1302 / 1462, 1,824 2529 / 2230,
+    // 2,400 2551 / 2962; three (one shared block fits): 152 744 / 368, 304 740 / 733, 1,216 1470 /
+    // 2893; four (nets read from memory): 456 2032 / 1230, 912 2666 / 2410, 1,300 3311 / 3553.  FP32
     // atoms are too cheap to share (2,400 of four elements: 171 in blocks of four, 770 in one-atom blocks).
     const size_t need = smem_of(kWarps, true), limit = 220 * 1024;
     const long long sms = device_sms();

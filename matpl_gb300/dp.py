@@ -176,6 +176,7 @@ def differ(a: torch.Tensor, b: torch.Tensor, answer: torch.Tensor, done: torch.c
     """Queues the comparison of two contiguous device tensors of one size; ``answer`` (pinned host int32)
     is 1 where a byte differs once ``done`` has passed."""
     from .ops import _stream
+    done.synchronize()             # an earlier comparison that nobody waited for writes the same word
     check(_lib.load().matpl_bytes_differ(ptr(a), ptr(b), a.numel() * a.element_size(), ptr(answer),
                                          _stream(a.device)), "matpl_bytes_differ")
     done.record(torch.cuda.current_stream(a.device))

@@ -224,6 +224,10 @@ class DP(torch.nn.Module):
             self._ctab = (int(tab.shape[1]), int(compress["order"]), float(compress["dx"]),
                           float(compress["sij_min"]), float(compress["sij_max"]))
 
+    def __setstate__(self, state):
+        super().__setstate__(state)
+        self.__dict__.setdefault("_order", LastMap())      # models pickled before it existed
+
     # dp_dp.py:145-165
     def present_types(self, atom_type) -> List[int]:
         at = [int(a) for a in (atom_type.tolist() if isinstance(atom_type, torch.Tensor) else atom_type)]

@@ -127,7 +127,7 @@ class LastMap:
 
     def __init__(self):
         self._entry = None
-        self._answers = {}                        # thread -> its pinned word and event
+        self._answers = {}                        # (thread, device) -> its pinned word and event
 
     def __reduce__(self):                         # copied and saved models start without one
         return LastMap, ()

@@ -696,8 +696,7 @@ class GraphedTrainer:
                 if hit is not None:
                     self._load(hit, batch, keys)
                     hit.rows.copy_(rows)
-                    steps.remove(hit)
-                    steps.insert(0, hit)
+                    steps[:] = [hit] + [c for c in steps if c is not hit]
         if hit is None:
             hit = self._capture(batch)
             steps.insert(0, hit)
